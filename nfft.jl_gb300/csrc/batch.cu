@@ -7,7 +7,9 @@
 //             plans' FFTs, gather (persistent warps over all plans' nodes);
 //   adjoint:  grid zero-fill, value sort, spreading (persistent CTAs taking
 //             tasks of all plans from one atomic counter), the plans' FFTs,
-//             crop+apodize.
+//             crop+apodize;
+//   D = 2:    gather and spreading run one warp per task over the plans'
+//             concatenated task lists (warp2.cuh), without the value sort.
 // The plans' FFTs run concurrently on forked streams: the fused pruned FFT
 // (with its own pad / crop, reading the image pointer from the per-call
 // table) for power-of-two grids, cuFFT for the others.
@@ -17,6 +19,7 @@
 // mode and spreading variant; their tiles, grids and node sets may differ.
 #include "interp_body.cuh"
 #include "spread_body.cuh"
+#include "warp2.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -40,7 +43,9 @@ struct nfft_batch {
   void* d_items = nullptr;        // BatchItem<T>[n]
   int64_t* d_base = nullptr;      // 5 prefix arrays of n+1: pairs, nodes, tasks, image, grid
   void** d_ptrs = nullptr;        // per call: input/output pointer of each plan
-  int* d_counter = nullptr;       // persistent spreading task counter
+  int* d_counter = nullptr;       // persistent spreading task counter (D = 3)
+  int4* d_tasks = nullptr;        // D = 2: every plan's tasks, {tile, first node, end node, plan}
+  size_t gather_smem = 0;         // D = 2: shared memory of the tiled gather (0: the direct gather)
   // pinned ring of per-call pointer tables: a slot is refilled only after the
   // copy that last read it has run (its event), so the copy never stalls the host
   static constexpr int kSlots = 8;
@@ -64,7 +69,9 @@ template <typename T> struct BatchItem {
   Geom<T> G;
   Nodes<T> Nd;
   const int4* tasks;
-  int pitch;
+  const int32_t* tile_start;
+  int task_chunk;
+  int pitch;   // D = 2: of the warp2 tiles, else of the spreading tile
   T* grid;
   typename Cplx<T>::type* fsorted;
   int N[3];
@@ -230,11 +237,104 @@ __global__ void __launch_bounds__(OwnedCfg<D, L>::THREADS) batch_spread_kernel(c
   }
 }
 
+// D = 2: the plans' tasks in one list, with the plan in .w.  A single plan
+// cuts its hot tiles into short tasks to fill the GPU; a batch fills it anyway
+// and joins the pieces of a tile up to `most` nodes again (fewer tiles
+// loaded and flushed): 32 plans of 9.3e6 nodes in all 1.30 / 1.23 / 1.20 / 1.21 ms
+// forward + adjoint with 128 / 256 / 512 / 1024, 6 plans of 2e5 nodes 119 / 125 /
+// 129 / 129 us, so 512 from 2^21 nodes on and 128 below.
+// `keep` (first pass, out = null): 1 for the first piece of each joined task;
+// second pass: the kept tasks at their scanned places.
+template <typename T>
+__global__ void __launch_bounds__(256) batch_tasks_kernel(const BatchItem<T>* __restrict__ items, const int64_t* base,
+                                                          int n, int64_t total, int most, int32_t* __restrict__ keep,
+                                                          const int32_t* __restrict__ place, int4* __restrict__ out) {
+  for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < total; q += int64_t(gridDim.x) * blockDim.x) {
+    const int pi = find_plan(base, n, q);
+    const BatchItem<T>& it = items[pi];
+    int4 t = it.tasks[q - __ldg(base + pi)];
+    const int group = max(1, most / it.task_chunk) * it.task_chunk;
+    const bool first = (t.y - __ldg(it.tile_start + t.x)) % group == 0;
+    if (!out) {
+      keep[q] = first;
+    } else if (first) {
+      t.z = min(t.y + group, __ldg(it.tile_start + t.x + 1));
+      t.w = pi;
+      out[place[q]] = t;
+    }
+  }
+}
+
+template <int L, typename T, bool TABLE>
+__global__ void __launch_bounds__(32) batch_spread_warp2_kernel(const BatchItem<T>* __restrict__ items,
+                                                                const int4* __restrict__ tasks,
+                                                                void* const* __restrict__ ptrs) {
+  using C = typename Cplx<T>::type;
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  const int4 task = __ldg(tasks + blockIdx.x);
+  const BatchItem<T>& it = items[task.w];
+  const Geom<T> G = it.G;
+  spread_warp2_body<L, T, TABLE>(G, it.Nd, task, static_cast<const C*>(ptrs[2 * task.w]), it.grid, it.pitch, G.coeffs,
+                                 smem_raw);
+}
+
+template <int L, typename T, bool TABLE>
+__global__ void __launch_bounds__(32) batch_gather_warp2_kernel(const BatchItem<T>* __restrict__ items,
+                                                                const int4* __restrict__ tasks,
+                                                                void* const* __restrict__ ptrs) {
+  using C = typename Cplx<T>::type;
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  const int4 task = __ldg(tasks + blockIdx.x);
+  const BatchItem<T>& it = items[task.w];
+  const Geom<T> G = it.G;
+  gather_warp2_body<L, T, TABLE>(G, it.Nd, task, reinterpret_cast<const C*>(it.grid),
+                                 static_cast<C*>(ptrs[2 * task.w + 1]), it.pitch, G.coeffs, smem_raw);
+}
+
 int grid_for_items(int64_t work, int per_block) {
   int64_t b = (work + per_block - 1) / per_block;
   const int64_t cap = 152 * 16;
   if (b > cap) b = cap;
   return int(b < 1 ? 1 : b);
+}
+
+// D = 2: builds d_tasks and sets the task total to its length.
+template <typename T> int batch_tasks(nfft_batch* B) {
+  const int64_t total = B->total[B_TASKS];
+  if (total == 0) return NFFT_OK;
+  const auto* items = static_cast<const BatchItem<T>*>(B->d_items);
+  const int64_t* base = B->d_base + B_TASKS * (B->n + 1);
+  const size_t sb = scan_scratch_bytes(total + 1);
+  struct Scratch {
+    char* q = nullptr;
+    ~Scratch() { cudaFree(q); }
+  } tmp;
+  const size_t list = (sizeof(int32_t) * size_t(total + 1) + 255) & ~size_t(255);
+  if (cudaMalloc(&tmp.q, 2 * list + sb) != cudaSuccess) {
+    set_error("allocation of batch tables failed");
+    return NFFT_ERR_ALLOC;
+  }
+  auto* keep = reinterpret_cast<int32_t*>(tmp.q);
+  auto* place = reinterpret_cast<int32_t*>(tmp.q + list);
+  const int grid = grid_for_items(total, 256);
+  const int most = B->total[B_NODES] >= (int64_t(1) << 21) ? 512 : 128;
+  NFFT_CUDA_TRY(cudaMemsetAsync(keep + total, 0, sizeof(int32_t), B->stream));
+  batch_tasks_kernel<T><<<grid, 256, 0, B->stream>>>(items, base, B->n, total, most, keep, nullptr, nullptr);
+  NFFT_LAUNCH_CHECK();
+  if (int rc = exclusive_scan_i32(keep, place, total + 1, tmp.q + 2 * list, sb, B->stream)) return rc;
+  int32_t kept = 0;
+  NFFT_CUDA_TRY(cudaMemcpyAsync(&kept, place + total, sizeof(int32_t), cudaMemcpyDeviceToHost, B->stream));
+  NFFT_CUDA_TRY(cudaStreamSynchronize(B->stream));
+  if (cudaMalloc(&B->d_tasks, sizeof(int4) * size_t(kept)) != cudaSuccess) {
+    B->d_tasks = nullptr;
+    set_error("allocation of batch tables failed");
+    return NFFT_ERR_ALLOC;
+  }
+  batch_tasks_kernel<T><<<grid, 256, 0, B->stream>>>(items, base, B->n, total, most, keep, place, B->d_tasks);
+  NFFT_LAUNCH_CHECK();
+  NFFT_CUDA_TRY(cudaStreamSynchronize(B->stream));
+  B->total[B_TASKS] = kept;
+  return NFFT_OK;
 }
 
 // All plans' grid FFTs, forked over the side streams and joined back into
@@ -282,6 +382,15 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     NFFT_LAUNCH_CHECK();
     int rc = forked_ffts(B, CUFFT_FORWARD);
     if (rc) return rc;
+    if constexpr (D == 2) {
+      if (B->gather_smem > 0) {
+        if (B->total[B_TASKS] == 0) return NFFT_OK;
+        batch_gather_warp2_kernel<L, T, TABLE><<<unsigned(B->total[B_TASKS]), 32, B->gather_smem, B->stream>>>(
+            items, B->d_tasks, B->d_ptrs);
+        NFFT_LAUNCH_CHECK();
+        return NFFT_OK;
+      }
+    }
     batch_gather_kernel<D, L, T, TABLE><<<B->gather_ctas, 256, 0, B->stream>>>(
         items, base + B_NODES * (B->n + 1), B->n, B->total[B_NODES], B->d_ptrs);
     NFFT_LAUNCH_CHECK();
@@ -293,13 +402,21 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     batch_zero_kernel<T><<<grid_for_items(B->total[B_GRID], 256), 256, 0, B->stream>>>(
         items, base + B_GRID * (B->n + 1), B->n, B->total[B_GRID]);
     NFFT_LAUNCH_CHECK();
-    batch_sort_values_kernel<T><<<grid_for_items(B->total[B_NODES], 256), 256, 0, B->stream>>>(
-        items, base + B_NODES * (B->n + 1), B->n, B->total[B_NODES], B->d_ptrs);
-    NFFT_LAUNCH_CHECK();
-    NFFT_CUDA_TRY(cudaMemsetAsync(B->d_counter, 0, sizeof(int), B->stream));
-    batch_spread_kernel<D, L, T, TABLE><<<B->spread_ctas, OwnedCfg<D, L>::THREADS, B->spread_smem, B->stream>>>(
-        items, base + B_TASKS * (B->n + 1), B->n, B->total[B_TASKS], B->d_counter);
-    NFFT_LAUNCH_CHECK();
+    if constexpr (D == 2) {
+      if (B->total[B_TASKS] > 0) {
+        batch_spread_warp2_kernel<L, T, TABLE><<<unsigned(B->total[B_TASKS]), 32, B->spread_smem, B->stream>>>(
+            items, B->d_tasks, B->d_ptrs);
+        NFFT_LAUNCH_CHECK();
+      }
+    } else {
+      batch_sort_values_kernel<T><<<grid_for_items(B->total[B_NODES], 256), 256, 0, B->stream>>>(
+          items, base + B_NODES * (B->n + 1), B->n, B->total[B_NODES], B->d_ptrs);
+      NFFT_LAUNCH_CHECK();
+      NFFT_CUDA_TRY(cudaMemsetAsync(B->d_counter, 0, sizeof(int), B->stream));
+      batch_spread_kernel<D, L, T, TABLE><<<B->spread_ctas, OwnedCfg<D, L>::THREADS, B->spread_smem, B->stream>>>(
+          items, base + B_TASKS * (B->n + 1), B->n, B->total[B_TASKS], B->d_counter);
+      NFFT_LAUNCH_CHECK();
+    }
     int rc = forked_ffts(B, CUFFT_INVERSE);
     if (rc) return rc;
     batch_crop_kernel<T><<<grid_for_items(B->total[B_IMAGE], 256), 256, 0, B->stream>>>(
@@ -307,24 +424,60 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     NFFT_LAUNCH_CHECK();
     return NFFT_OK;
   }
+  // D = 2: the tasks in one list, the tile pitches and the shared memory of
+  // the largest tile; the gather goes through tiles when there are enough
+  // nodes per task on the whole (as for one plan, interp.cu)
+  static int setup2(nfft_batch* B) {
+    using W = Warp2<L, T, TABLE>;
+    constexpr size_t E = 2 * sizeof(T);
+    size_t old_smem = 0, tile = 0;
+    double points = 0;
+    for (nfft_plan* p : B->plans) {
+      old_smem = std::max(old_smem, owned_smem<D, L, T>(p, false));
+      const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
+      tile = std::max(tile, E * size_t(warp2_plan_pitch<L, T, TABLE>(p)) * P1);
+      points += double(p->n_tasks) * P0 * P1;
+    }
+    B->spread_smem = old_smem;
+    if (old_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
+    B->spread_smem = W::SPREAD_STAGE + tile;
+    NFFT_CUDA_TRY(cudaFuncSetAttribute(batch_spread_warp2_kernel<L, T, TABLE>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->spread_smem)));
+    if (double(B->total[B_NODES]) * 256 >= points) {
+      B->gather_smem = W::GATHER_STAGE + tile;
+      NFFT_CUDA_TRY(cudaFuncSetAttribute(batch_gather_warp2_kernel<L, T, TABLE>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->gather_smem)));
+    } else {
+      int dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int64_t want = (B->total[B_NODES] + 63) / 64;
+      B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(sms) * 64)));
+    }
+    return batch_tasks<T>(B);
+  }
   static int setup(nfft_batch* B) {
-    for (nfft_plan* p : B->plans) B->spread_smem = std::max(B->spread_smem, owned_smem<D, L, T>(p, false));
-    if (B->spread_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
-    auto kern = batch_spread_kernel<D, L, T, TABLE>;
-    NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->spread_smem)));
-    int per_sm = 0;
-    NFFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, OwnedCfg<D, L>::THREADS,
-                                                                B->spread_smem));
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int64_t ctas = int64_t(std::max(per_sm, 1)) * sms;
-    B->spread_ctas = int(std::max<int64_t>(1, std::min<int64_t>(ctas, B->total[B_TASKS])));
-    // gather: CTAs of 8 warps, one contiguous node chunk each (8 nodes per warp
-    // and CTA at least), at most 64 CTAs per SM
-    const int64_t want = (B->total[B_NODES] + 63) / 64;
-    B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(sms) * 64)));
-    return NFFT_OK;
+    if constexpr (D == 2) {
+      return setup2(B);
+    } else {
+      for (nfft_plan* p : B->plans) B->spread_smem = std::max(B->spread_smem, owned_smem<D, L, T>(p, false));
+      if (B->spread_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
+      auto kern = batch_spread_kernel<D, L, T, TABLE>;
+      NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->spread_smem)));
+      int per_sm = 0;
+      NFFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, OwnedCfg<D, L>::THREADS,
+                                                                  B->spread_smem));
+      int dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      int64_t ctas = int64_t(std::max(per_sm, 1)) * sms;
+      B->spread_ctas = int(std::max<int64_t>(1, std::min<int64_t>(ctas, B->total[B_TASKS])));
+      // gather: CTAs of 8 warps, one contiguous node chunk each (8 nodes per warp
+      // and CTA at least), at most 64 CTAs per SM
+      const int64_t want = (B->total[B_NODES] + 63) / 64;
+      B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(sms) * 64)));
+      return NFFT_OK;
+    }
   }
 };
 
@@ -347,6 +500,21 @@ int run(nfft_batch* B, int what) {
   return B->table ? dispatch<double, true>(B, what) : dispatch<double, false>(B, what);
 }
 
+template <typename T, bool TABLE> int batch_pitch2_t(const nfft_plan* p) {
+  switch (p->m) {
+    case 2: return warp2_plan_pitch<4, T, TABLE>(p);
+    case 3: return warp2_plan_pitch<6, T, TABLE>(p);
+    case 4: return warp2_plan_pitch<8, T, TABLE>(p);
+    case 5: return warp2_plan_pitch<10, T, TABLE>(p);
+    case 6: return warp2_plan_pitch<12, T, TABLE>(p);
+    case 7: return warp2_plan_pitch<14, T, TABLE>(p);
+    default: return warp2_plan_pitch<16, T, TABLE>(p);
+  }
+}
+template <typename T> int batch_pitch2(const nfft_plan* p, bool table) {
+  return table ? batch_pitch2_t<T, true>(p) : batch_pitch2_t<T, false>(p);
+}
+
 template <typename T> int fill_items(nfft_batch* B) {
   std::vector<BatchItem<T>> items(B->n);
   std::vector<int64_t> base(5 * (B->n + 1), 0);
@@ -356,7 +524,9 @@ template <typename T> int fill_items(nfft_batch* B) {
     it.G = make_geom<T>(p);
     it.Nd = make_nodes<T>(p);
     it.tasks = p->tasks;
-    it.pitch = p->spread_pitch;
+    it.tile_start = p->tile_start;
+    it.task_chunk = p->task_chunk;
+    it.pitch = p->D == 2 ? batch_pitch2<T>(p, B->table) : p->spread_pitch;
     it.grid = static_cast<T*>(p->grid);
     it.fsorted = static_cast<typename Cplx<T>::type*>(p->fsorted);
     const T* inv = static_cast<const T*>(p->inv);
@@ -394,6 +564,7 @@ extern "C" int nfft_batch_destroy(nfft_batch* B) {
   cudaFree(B->d_base);
   cudaFree(B->d_ptrs);
   cudaFree(B->d_counter);
+  cudaFree(B->d_tasks);
   for (int i = 0; i < nfft_batch::kSlots; ++i)
     if (B->ring_ev[i]) cudaEventDestroy(B->ring_ev[i]);
   cudaFreeHost(B->h_ring);

@@ -11,6 +11,7 @@
 // plane are 32-bit; the plane offset is 64-bit.
 #include "interp_body.cuh"
 #include "tile3.cuh"
+#include "warp2.cuh"
 
 namespace nfft {
 namespace {
@@ -494,6 +495,41 @@ int interp_tile3(const nfft_plan* cp, const Geom<float>& G, const Nodes<float>& 
   return -1;
 }
 
+// D = 2: one warp per task (warp2.cuh); blockIdx.y: column of a multi-column launch.
+template <int L, typename T, bool TABLE>
+__global__ void __launch_bounds__(32) gather_warp2_kernel(Geom<T> G, Nodes<T> Nd, const int4* __restrict__ tasks,
+                                                          const typename Cplx<T>::type* __restrict__ g,
+                                                          typename Cplx<T>::type* __restrict__ fhat, int pitch,
+                                                          int64_t gcol, int64_t fcol,
+                                                          const __grid_constant__ WinPoly<L, T, TABLE> wp) {
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  gather_warp2_body<L, T, TABLE>(G, Nd, __ldg(tasks + blockIdx.x), g + blockIdx.y * gcol, fhat + blockIdx.y * fcol,
+                                 pitch, wp.c, smem_raw);
+}
+
+// -1: not applicable (no task list, tile too large, or too few nodes per
+// task to pay for bringing their tile into shared memory).
+template <int L, typename T, bool TABLE>
+int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* g,
+                        typename Cplx<T>::type* fhat, int ncols, int64_t gcol, int64_t fcol) {
+  using W = Warp2<L, T, TABLE>;
+  if (!p->tasks || p->n_tasks == 0) return -1;
+  const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
+  if (p->M * 256 < p->n_tasks * int64_t(P0) * P1) return -1;
+  const int pitch = warp2_plan_pitch<L, T, TABLE>(p);
+  const size_t smem = W::GATHER_STAGE + 2 * sizeof(T) * size_t(pitch) * P1;
+  if (smem > 227 * 1024) return -1;
+  WinPoly<L, T, TABLE> wp{};
+  if constexpr (!TABLE)
+    for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  auto kern = gather_warp2_kernel<L, T, TABLE>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), 32, smem, p->stream>>>(G, Nd, p->tasks, g, fhat, pitch, gcol,
+                                                                            fcol, wp);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
 // ncols columns in one launch (blockIdx.y): grids g + c gcol, values fhat + c fcol.
 template <int D, int L, typename T>
 int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int64_t gcol, int64_t fcol) {
@@ -511,6 +547,11 @@ int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int6
   if (blocks > cap) blocks = cap;
   const C* gp = static_cast<const C*>(g);
   C* fp = static_cast<C*>(fhat);
+  if constexpr (D == 2) {
+    const int rc = p->wtab ? gather_warp2_launch<L, T, true>(p, G, Nd, gp, fp, ncols, gcol, fcol)
+                           : gather_warp2_launch<L, T, false>(p, G, Nd, gp, fp, ncols, gcol, fcol);
+    if (rc != -1) return rc;
+  }
   if (ncols > 1) {
     const dim3 grid{unsigned(blocks), unsigned(ncols), 1u};
     if (p->wtab)

@@ -142,6 +142,8 @@ struct nfft_plan {
   // spreading tasks: (home tile, first node, end node, 0), hot tiles split
   int64_t n_tasks = 0;
   int4* tasks = nullptr;
+  int task_chunk = 1024;           // most nodes of a task
+  int64_t task_columns = 1;        // columns that every launch over the tasks covers (directional plans)
   int spread_pitch = 0;            // shared-memory row pitch of the padded spreading tile
   int spread_layout = 1;           // D = 3 spreading kernel: 1 = 8 warps owning slices, 2 = 16 warps owning
                                    // (slice group, row parity)

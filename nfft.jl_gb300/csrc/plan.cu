@@ -769,12 +769,24 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
   if (p->prm.blocking) {
     // hot tiles are split into chunks of at most `chunk` nodes (each chunk is
     // one spreading task and flushes its padded tile once);
-    // NFFT_GB300_TASK_CHUNK overrides the default 1024
+    // NFFT_GB300_TASK_CHUNK overrides the default.  D = 2 tasks run on one
+    // warp each (warp2.cuh), ~60 cycles a node, so 1024 nodes of a hot tile
+    // take 30 us on their own, longer than a whole small transform; large
+    // sets fill the GPU anyway and prefer fewer flushes.  Forward + adjoint of
+    // a radial 128^2 image, us with 64 / 128 / 256 / 512 nodes per task:
+    // 4,000 nodes 42 / 44 / 44 / 44, 20,000 nodes 42 / 48 / 58 / 79, 200,000
+    // nodes 58 / 63 / 67 / 85, 800,000 nodes 115 / 116 / 121 / 143; 64 slices of
+    // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
     int chunk = 1024;
+    if (D == 2 && !p->prm.compensated) {
+      const int64_t work = M * p->task_columns;
+      chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
+    }
     if (const char* e = getenv("NFFT_GB300_TASK_CHUNK")) {
       const int c = atoi(e);
       if (c >= 32 && c <= (1 << 20)) chunk = c;
     }
+    p->task_chunk = chunk;
     rc = launch_build_tasks(p, chunk);
     if (rc) return rc;
     p->fsorted = node_buffer(p, P::NB_FSORTED, 2 * rs * size_t(M));

@@ -23,9 +23,38 @@
 // The lock of the reference becomes the L2 atomics of the flush.
 #include "spread_body.cuh"
 #include "spread_tile3.cuh"
+#include "warp2.cuh"
 
 namespace nfft {
 namespace {
+
+// D = 2, uncompensated: one warp per task (warp2.cuh); blockIdx.y: column of a multi-column launch.
+template <int L, typename T, bool TABLE>
+__global__ void __launch_bounds__(32) spread_warp2_kernel(Geom<T> G, Nodes<T> Nd, const int4* __restrict__ tasks,
+                                                          const typename Cplx<T>::type* __restrict__ fhat,
+                                                          T* __restrict__ g, int pitch, int64_t fcol, int64_t gcol,
+                                                          const __grid_constant__ WinPoly<L, T, TABLE> wp) {
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  spread_warp2_body<L, T, TABLE>(G, Nd, __ldg(tasks + blockIdx.x), fhat + blockIdx.y * fcol, g + blockIdx.y * gcol,
+                                 pitch, wp.c, smem_raw);
+}
+
+template <int L, typename T, bool TABLE>
+int spread_warp2_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* fhat, T* g,
+                        int ncols, int64_t fcol, int64_t gcol_t) {
+  using W = Warp2<L, T, TABLE>;
+  const int pitch = warp2_plan_pitch<L, T, TABLE>(p);
+  const size_t smem = W::SPREAD_STAGE + 2 * sizeof(T) * size_t(pitch) * size_t(p->bs[1] + L - 1);
+  WinPoly<L, T, TABLE> wp{};
+  if constexpr (!TABLE)
+    for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  auto kern = spread_warp2_kernel<L, T, TABLE>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), 32, smem, p->stream>>>(G, Nd, p->tasks, fhat, g, pitch, fcol,
+                                                                            gcol_t, wp);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
 
 // fHat in bin-sorted order (node4[i].w = input index), for coalesced staging.
 // blockIdx.y: column of a multi-column launch (input fhat + y fcol, output out + y M)
@@ -182,10 +211,15 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
       set_error("padded spreading tile (%zu bytes) does not fit in shared memory; use a smaller blockSize", smem);
       return NFFT_ERR_UNSUPPORTED;
     }
-    auto kern = comp ? (p->wtab ? spread_owned_kernel<D, L, T, true, true> : spread_owned_kernel<D, L, T, false, true>)
-                     : (p->wtab ? spread_owned_kernel<D, L, T, true, false> : spread_owned_kernel<D, L, T, false, false>);
+    if constexpr (D == 2) {
+      if (!comp)
+        return p->wtab ? spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
+                       : spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+    }
+    auto kern = p->wtab ? spread_owned_kernel<D, L, T, true, true> : spread_owned_kernel<D, L, T, false, true>;
     int threads = OwnedCfg<D, L>::THREADS;
     if constexpr (D == 3) {
+      if (!comp) kern = p->wtab ? spread_owned_kernel<D, L, T, true, false> : spread_owned_kernel<D, L, T, false, false>;
       if (!comp && p->spread_layout == 2) {  // 16 warps: slice group x row parity
         kern = p->wtab ? spread_owned_kernel<D, L, T, true, false, 2> : spread_owned_kernel<D, L, T, false, false, 2>;
         threads = OwnedCfg<D, L, 2>::THREADS;
