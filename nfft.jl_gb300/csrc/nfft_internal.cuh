@@ -147,9 +147,9 @@ struct nfft_plan {
   int spread_pitch = 0;            // shared-memory row pitch of the padded spreading tile
   int spread_layout = 1;           // D = 3 spreading kernel: 1 = 8 warps owning slices, 2 = 16 warps owning
                                    // (slice group, row parity)
-  bool spread_tile3 = true;        // 3-D FP32 m = 4: shape-specialised spreading kernel (spread_tile3.cuh)
+  bool spread_tile3 = true;        // 3-D FP32: shape-specialised spreading kernels (spread_plane3.cuh, spread_tile3.cuh)
   bool spread_tma = true;          // its bulk tensor reduction flush for tiles that do not wrap
-  bool gather_tma = true;          // 3-D FP32 m = 4 gather from tiles loaded by bulk tensor copies
+  bool gather_tma = true;          // 3-D FP32 gather from tiles loaded by bulk tensor copies
   // tensor maps of the grids the tiled kernels moved tiles of (the plan's two
   // grids), with their grid and tile shape; replaced least recently made first
   CUtensorMap tmap[2] = {};
@@ -170,7 +170,7 @@ struct nfft_plan {
   bool spread_zero_copy = true;    // table spreader: clear the tile by a bulk copy of zero_tile
   void* zero_tile = nullptr;       // 128 KB of zeros
   bool fft_staged = true;          // FP32 line FFTs: tile staged by cp.async, in-place four-step
-  bool spread_rec = true;          // 3-D FP32 table spreader: one-step staging with per-warp records
+  bool spread_rec = true;          // 3-D FP32: the plane-owner spreader (spread_plane3.cuh)
   int gather_pf = 4;               // TMA gather: L2 prefetch of the tile gather_pf x (SM count) tasks ahead (0: off)        // set while the spreading target is known to be zero
   int gather_pitch = 0;            // shared-memory row pitch of the staged gather tile
   bool gather_tiled = false;       // gather from shared-memory tiles (else straight from L1/L2)
@@ -227,6 +227,13 @@ int launch_pad_apodize(const nfft_plan* p, const void* f, void* g);
 int launch_crop_apodize(const nfft_plan* p, const void* g, void* f);
 int launch_real_to_complex(const nfft_plan* p, const void* in, void* out, int64_t n);
 int launch_real_part(const nfft_plan* p, const void* in, void* out, int64_t n);
+// gather3.cu: -1 = not applicable
+int launch_gather_plane3(const nfft_plan* p, const void* g, void* fhat);
+// spread3.cu: -1 = not applicable
+int launch_spread_plane3(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fcol, int64_t gcol_t);
+// spread.cu: the plan's buffer of zeros that clears spreading tiles (null: not available)
+constexpr size_t kZeroTileBytes = 128 * 1024;
+const float4* zero_tile_for(nfft_plan* p);
 // interp.cu
 int launch_interp(const nfft_plan* p, const void* g, int g_real, void* fhat, int fhat_real);
 // ncols columns in one launch: grids g + c gcol, node values fhat + c fcol (complex elements)

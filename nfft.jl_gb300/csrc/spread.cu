@@ -99,55 +99,6 @@ int tile3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, con
   return NFFT_OK;
 }
 
-// The one-step staging kernel for table windows: values fhat + c fcol in the
-// caller's order, read through the bin-sorted nodes' input indices.
-template <int BX, int BY, int BZ>
-int tile3_rec_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fhat, float* gp,
-                     int ncols, int64_t fcol, int64_t gcol_t) {
-  using TC = Tile3<BX, BY, BZ>;
-  using TR = Tile3Rec<BX, BY, BZ>;
-  const CUtensorMap* map = (ncols == 1 && p->spread_tma) ? tile3_map<BX, BY, BZ>(p, gp) : nullptr;
-  CUtensorMap none{};
-  // a zeroed buffer of the largest padded tile, copied into shared memory to
-  // clear each CTA's tile (allocated once per plan)
-  static_assert(TC::NACC * 8 <= 128 * 1024, "zero tile buffer");
-  if (!p->zero_tile && p->spread_zero_copy) {
-    if (cudaMalloc(&p->zero_tile, 128 * 1024) != cudaSuccess ||
-        cudaMemsetAsync(p->zero_tile, 0, 128 * 1024, p->stream) != cudaSuccess) {
-      cudaFree(p->zero_tile);
-      p->zero_tile = nullptr;
-      p->spread_zero_copy = false;  // plain stores clear the tile
-      cudaGetLastError();
-    }
-  }
-  WinCoeffs8 wc{};
-  if (!p->wtab)
-    for (int q = 0; q < 8 * 9; ++q) wc.c[q] = float(p->coeffs_host[q]);
-  auto kr = p->wtab ? spread_tile3_rec_kernel<BX, BY, BZ, true> : spread_tile3_rec_kernel<BX, BY, BZ, false>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TR::SMEM)));
-  kr<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), TC::THREADS, TR::SMEM, p->stream>>>(
-      map ? *map : none, map ? 1 : 0, G, Nd, p->tasks, fhat, gp, ncols > 1 ? fcol : 0, gcol_t,
-      p->spread_zero_copy ? static_cast<const float4*>(p->zero_tile) : nullptr, p->dflag + 1, wc);
-  NFFT_LAUNCH_CHECK();
-  return NFFT_OK;
-}
-
-// The one-step kernel when the plan's tiles have a shape-specialised form
-// (no value sort); -1 = not applicable.
-int spread_tile3_user(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fhat, float* gp,
-                      int ncols, int64_t fcol, int64_t gcol_t) {
-  if (!p->spread_tile3 || !p->spread_rec || (!p->wtab && !p->frac4) || p->D != 3 || p->m != 4 ||
-      p->prm.compensated ||
-      p->spread_layout != 1 || p->bs[2] != 8)
-    return -1;
-  const int64_t bx = p->bs[0], by = p->bs[1];
-  if (bx == 16 && by == 8) return tile3_rec_launch<16, 8, 8>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-  if (bx == 16 && by == 16) return tile3_rec_launch<16, 16, 8>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-  if (bx == 32 && by == 8) return tile3_rec_launch<32, 8, 8>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-  if (bx == 8 && by == 8) return tile3_rec_launch<8, 8, 8>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-  return -1;
-}
-
 // The shape-specialised 3-D kernel when the plan's tiles have one of its
 // shapes (FP32, m = 4, uncompensated, 8-warp layout); -1 = not applicable.
 int spread_tile3(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fs, float* gp, int ncols,
@@ -225,8 +176,8 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
         threads = OwnedCfg<D, L, 2>::THREADS;
       }
     }
-    if constexpr (D == 3 && L == 8 && sizeof(T) == 4) {  // values read in the caller's order
-      const int rc = spread_tile3_user(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+    if constexpr (D == 3 && sizeof(T) == 4 && L <= 12) {  // values read in the caller's order
+      const int rc = launch_spread_plane3(p, fhat, g, ncols, fcol, gcol_t);
       if (rc != -1) return rc;
     }
     NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -272,6 +223,21 @@ int spread_dispatch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t 
 #undef NFFT_SPREAD_ARGS
 
 }  // namespace
+
+// A zeroed buffer as large as the largest padded tile, copied into shared
+// memory to clear each CTA's tile (allocated once per plan).
+const float4* zero_tile_for(nfft_plan* p) {
+  if (!p->zero_tile && p->spread_zero_copy) {
+    if (cudaMalloc(&p->zero_tile, kZeroTileBytes) != cudaSuccess ||
+        cudaMemsetAsync(p->zero_tile, 0, kZeroTileBytes, p->stream) != cudaSuccess) {
+      cudaFree(p->zero_tile);
+      p->zero_tile = nullptr;
+      p->spread_zero_copy = false;  // plain stores clear the tile
+      cudaGetLastError();
+    }
+  }
+  return p->spread_zero_copy ? static_cast<const float4*>(p->zero_tile) : nullptr;
+}
 
 // Row pitch (in accumulator elements) of the padded tile: the smallest pitch
 // >= the padded row length for which every shared-memory access phase of a

@@ -1,13 +1,15 @@
-// Fixed 3-D tile shapes (m = 4) shared by the shape-specialised spreading
-// (spread_tile3.cuh) and gather (interp.cu) kernels: the tile padded by the
-// window, laid out in shared memory as a TMA box of the grid, and the host
-// side that encodes the grid's tensor map.
+// Fixed 3-D tile shapes shared by the shape-specialised spreading
+// (spread_tile3.cuh, spread_plane3.cuh) and gather (interp.cu,
+// gather_plane3.cuh) kernels: the tile padded by the window, laid out in
+// shared memory as a TMA box of the grid, and the host side that encodes the
+// grid's tensor map.
 //
 // The padded tile of a tile with origin (o0, o1, o2) covers grid x from
-// o0 - m (even: one leading column outside the window, so that the box starts
-// on a 16-byte boundary) and grid y, z from o - m + 1; its rows have a
-// constant pitch (>= the padded width, = 8 mod 16 complex values, so the two
-// row pairs a half-warp touches fall in distinct banks).  A tile whose box
+// o0 - m (m even: one leading column outside the window, so that the box
+// starts on a 16-byte boundary) or o0 - m + 1 (m odd) and grid y, z from
+// o - m + 1; its rows have a constant pitch (>= the padded width, = 2m mod 16
+// complex values, so that consecutive taps of an x-y plane, taken row after
+// row, fall in distinct banks).  A tile whose box
 // lies inside the grid moves between grid and shared memory with one bulk
 // tensor copy; a tile whose box wraps around the grid is moved per point.
 #pragma once
@@ -21,10 +23,12 @@
 namespace nfft {
 namespace {
 
-template <int BX, int BY, int BZ> struct Tile3 {
-  static constexpr int L = 8;
-  static constexpr int P0 = BX + L;                      // columns, from grid x o0 - m
-  static constexpr int PITCH = P0 + ((8 - P0 % 16) + 16) % 16;  // >= P0, = 8 mod 16: conflict-free row pairs
+template <int BX, int BY, int BZ, int L_ = 8> struct Tile3 {
+  static constexpr int L = L_;
+  static constexpr int LEAD = (L / 2) % 2 == 0 ? 1 : 0;  // columns before the window of the first point
+  static constexpr int XOFF = L / 2 - 1 + LEAD;          // the tile starts at grid x o0 - XOFF (even)
+  static constexpr int P0 = BX + L;                      // columns
+  static constexpr int PITCH = P0 + ((L - P0 % 16) + 16) % 16;  // >= P0, = L mod 16: conflict-free rows
   static constexpr int P1 = BY + L - 1;
   static constexpr int P2 = BZ + L - 1;
   static constexpr int PLANE = PITCH * P1;
@@ -61,10 +65,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned addr, unsigned parity
 
 // The grid region of a tile's padded box lies inside the grid (no wrap):
 // the box is added with one bulk tensor reduction.
-template <int BX, int BY, int BZ>
+template <int BX, int BY, int BZ, int L = 8>
 __device__ __forceinline__ bool tile3_interior(const Geom<float>& G, int o0, int o1, int o2) {
-  using TC = Tile3<BX, BY, BZ>;
-  const int x = o0 - 4, y = o1 - 3, z = o2 - 3;
+  using TC = Tile3<BX, BY, BZ, L>;
+  const int x = o0 - TC::XOFF, y = o1 - (L / 2 - 1), z = o2 - (L / 2 - 1);
   return x >= 0 && y >= 0 && z >= 0 && x + TC::PITCH <= G.Nt[0] && y + TC::P1 <= G.Nt[1] && z + TC::P2 <= G.Nt[2];
 }
 
@@ -96,12 +100,12 @@ EncodeTiledFn encode_tiled() {
 }
 
 // Tensor map of the FP32 grid g (2 Ntilde[0] floats x Ntilde[1] x Ntilde[2])
-// with the padded-tile box of Tile3<BX, BY, BZ>, cached on the plan per grid
+// with the padded-tile box of Tile3<BX, BY, BZ, L>, cached on the plan per grid
 // and shape (two entries: the plan's forward and adjoint grids).  Null when it
 // cannot be made (no driver entry point, grid not 16-byte aligned, box larger
 // than the grid): the kernels then move tiles point by point.
-template <int BX, int BY, int BZ> const CUtensorMap* tile3_map(nfft_plan* p, void* g) {
-  using TC = Tile3<BX, BY, BZ>;
+template <int BX, int BY, int BZ, int L = 8> const CUtensorMap* tile3_map(nfft_plan* p, void* g) {
+  using TC = Tile3<BX, BY, BZ, L>;
   const int64_t key = (int64_t(BX) << 20) | (int64_t(BY) << 10) | BZ;
   for (int i = 0; i < 2; ++i)
     if (p->tmap_grid[i] == g && p->tmap_key[i] == key) return &p->tmap[i];

@@ -196,7 +196,7 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
   for (int s = 0; s < W::NSTEP; ++s) {
     const int t = lane + 32 * s;
     act[s] = W::TAPS % 32 == 0 || t < W::TAPS;
-    const int tt = act[s] ? t : 0;
+    const int tt = act[s] ? t : W::TAPS - 1;
     iy[s] = tt / L;
     ix[s] = tt - iy[s] * L;
     lofs[s] = iy[s] * pitch + ix[s];
@@ -334,7 +334,7 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
   for (int s = 0; s < W::NSTEP; ++s) {
     const int t = lane + 32 * s;
     act[s] = W::TAPS % 32 == 0 || t < W::TAPS;
-    const int tt = act[s] ? t : 0;
+    const int tt = act[s] ? t : W::TAPS - 1;
     iy[s] = tt / L;
     ix[s] = tt - iy[s] * L;
     lofs[s] = iy[s] * pitch + ix[s];
@@ -366,11 +366,12 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
         T sr = T(0), si = T(0);
 #pragma unroll
         for (int q = 0; q < W::NSTEP; ++q) {
-          const C v = p[lofs[q]];
-          T w = row[ix[q]] * row[L + iy[q]];
-          if (!act[q]) w = T(0);
-          sr = fma(w, v.x, sr);
-          si = fma(w, v.y, si);
+          const T w = row[ix[q]] * row[L + iy[q]];
+          if (act[q]) {  // (idle lanes of the last step make no request)
+            const C v = p[lofs[q]];
+            sr = fma(w, v.x, sr);
+            si = fma(w, v.y, si);
+          }
         }
         ar[k] = sr;
         ai[k] = si;
