@@ -1,17 +1,21 @@
 // Gather interpolation (convolve!): fHat[j] = sum over the (2m)^D window taps
 // of prod_d phi_d * g[tap], src/convolution.jl:229-344 (blocked) and :56-99.
 //
-// Warp per node (D >= 2) or 32/G nodes per warp (D = 1), nodes visited in
-// bin-sorted order; for D >= 2 each CTA takes a contiguous chunk of the
-// sorted nodes, so the nodes an SM visits close in time read overlapping grid
+// D = 1: one thread per node (line1.cuh); D = 2: one warp per task from
+// tiles in shared memory (warp2.cuh); D = 3, FP32: tiled (below, gather3.cu).
+// Otherwise a warp per node, nodes visited in bin-sorted order; each CTA takes
+// a contiguous chunk of the sorted nodes, so the nodes an SM visits close in time read overlapping grid
 // neighbourhoods through L1, and a warp issues all of a node's grid loads
 // before its sums (memory-level parallelism).  Window values come from the stored window
 // tensor (TENSOR / FULL / LINEAR) or from the fitted polynomial evaluated with
 // its coefficients held in registers (POLYNOMIAL).  Grid offsets within a
 // plane are 32-bit; the plane offset is 64-bit.
 #include "interp_body.cuh"
+#include "line1.cuh"
 #include "tile3.cuh"
 #include "warp2.cuh"
+
+#include <algorithm>
 
 namespace nfft {
 namespace {
@@ -33,71 +37,21 @@ __global__ void __launch_bounds__(kInterpThreads) interp_kernel(Geom<T> G, Nodes
                                                                  const typename Cplx<T>::type* __restrict__ g,
                                                                  typename Cplx<T>::type* __restrict__ fhat,
                                                                  int64_t gcol = 0, int64_t fcol = 0) {
-  using C = typename Cplx<T>::type;
-  using LN = Lanes<D, L>;
+  static_assert(D >= 2, "D = 1: line1.cuh");
   if constexpr (COLS) {  // column of a multi-column launch
     g += blockIdx.y * gcol;
     fhat += blockIdx.y * fcol;
   }
   const int lane = threadIdx.x & 31;
-  const int64_t warp_global = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int64_t warps_total = int64_t(gridDim.x) * (blockDim.x >> 5);
-  const int m = G.m;
-  const bool small = G.small_grid;
-
-  if constexpr (D == 1) {
-    // 32/G1 nodes per warp, lane -> (node slot, tap ix)
-    const int slot = lane / LN::G1, ix = lane % LN::G1;
-    const bool act = ix < L;
-    T c[LN::DEG];
-    if constexpr (!TABLE) {
-#pragma unroll
-      for (int q = 0; q < LN::DEG; ++q) c[q] = act ? __ldg(G.coeffs + ix * LN::DEG + q) : T(0);
-    }
-    for (int64_t base = warp_global * LN::NPW; base < Nd.M; base += warps_total * LN::NPW) {
-      const int64_t i = base + slot;
-      T ar = T(0), ai = T(0);
-      int4 nd = make_int4(0, 0, 0, 0);
-      if (i < Nd.M) nd = __ldg(Nd.node4 + i);
-      if (i < Nd.M && act) {
-        T w;
-        if constexpr (TABLE) {
-          w = __ldg(Nd.wtab + i * L + ix);
-        } else {
-          const T t = __ldg(Nd.frac4 + 4 * i) - T(0.5);
-          w = c[LN::DEG - 1];
-#pragma unroll
-          for (int q = LN::DEG - 2; q >= 0; --q) w = fma(w, t, c[q]);
-        }
-        const int gx = small ? wrap_any(nd.x + G.sh[0] - m + 1 + ix, G.Nt[0])
-                             : wrap_once(nd.x + G.sh[0] - m + 1 + ix, G.Nt[0]);
-        const C v = __ldg(g + gx);
-        ar = w * v.x;
-        ai = w * v.y;
-      }
-#pragma unroll
-      for (int o = LN::G1 / 2; o > 0; o >>= 1) {
-        ar += __shfl_xor_sync(0xFFFFFFFFu, ar, o);
-        ai += __shfl_xor_sync(0xFFFFFFFFu, ai, o);
-      }
-      if (ix == 0 && i < Nd.M) {
-        C r;
-        r.x = ar;
-        r.y = ai;
-        fhat[nd.w] = r;
-      }
-    }
-  } else {
-    PolyRegs<D, L, T> P;
-    if constexpr (!TABLE) P.load(G.coeffs, lane);
-    // each CTA takes a contiguous chunk of the bin-sorted nodes: nodes a CTA
-    // visits close in time share their grid neighbourhood in L1
-    const int64_t chunk = (Nd.M + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = int64_t(blockIdx.x) * chunk;
-    const int64_t hi = lo + chunk < Nd.M ? lo + chunk : Nd.M;
-    for (int64_t i = lo + (threadIdx.x >> 5); i < hi; i += blockDim.x >> 5)
-      interp_node<D, L, T, TABLE>(G, Nd, P, i, lane, g, fhat);
-  }
+  PolyRegs<D, L, T> P;
+  if constexpr (!TABLE) P.load(G.coeffs, lane);
+  // each CTA takes a contiguous chunk of the bin-sorted nodes: nodes a CTA
+  // visits close in time share their grid neighbourhood in L1
+  const int64_t chunk = (Nd.M + gridDim.x - 1) / gridDim.x;
+  const int64_t lo = int64_t(blockIdx.x) * chunk;
+  const int64_t hi = lo + chunk < Nd.M ? lo + chunk : Nd.M;
+  for (int64_t i = lo + (threadIdx.x >> 5); i < hi; i += blockDim.x >> 5)
+    interp_node<D, L, T, TABLE>(G, Nd, P, i, lane, g, fhat);
 }
 
 // Tile-staged gather: one CTA per spreading task (home tile or chunk of a hot
@@ -127,7 +81,6 @@ __global__ void __launch_bounds__(kInterpThreads) interp_tile_kernel(Geom<T> G, 
   const int plane = pitch * P1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int m1 = G.m - 1;
-  const bool small = G.small_grid;
   // stage the padded tile with asynchronous copies (cp.async): every row
   // copy is issued before the single wait, so a warp keeps all of its rows'
   // loads in flight instead of one load-store round trip per row
@@ -152,100 +105,59 @@ __global__ void __launch_bounds__(kInterpThreads) interp_tile_kernel(Geom<T> G, 
     cp_async_wait_all();
   }
   __syncthreads();
-  if constexpr (D == 1) {
-    const int slot = lane / LN::G1, ix = lane % LN::G1;
-    const bool act = ix < L;
-    T c[LN::DEG];
-    if constexpr (!TABLE) {
+  PolyRegs<D, L, T> P;
+  if constexpr (!TABLE) P.load(G.coeffs, lane);
+  const int ix = lane % L, ry = lane / L;
+  const bool xact = ry < LN::RY;
+  for (int i = task.y + warp; i < task.z; i += nwarps) {
+    const int4 nd = __ldg(Nd.node4 + i);
+    T W[LN::NW];
+    node_weights<D, L, T, TABLE>(Nd, P, i, lane, W);
+    const T wx = wsel<D, L>(W, ix);
+    const int px = nd.x - o0 + ix, py = nd.y - o1;
+    int row[LN::NSTEP];
+    T wxy[LN::NSTEP];
 #pragma unroll
-      for (int q = 0; q < LN::DEG; ++q) c[q] = act ? __ldg(G.coeffs + ix * LN::DEG + q) : T(0);
+    for (int s = 0; s < LN::NSTEP; ++s) {
+      const int iy = s * LN::RY + ry;
+      const bool ok = xact && iy < L;
+      const int iyc = ok ? iy : 0;
+      const T wy = wsel<D, L>(W, L + iyc);  // every lane shuffles
+      row[s] = (py + iyc) * pitch + px;
+      wxy[s] = ok ? wx * wy : T(0);
     }
-    for (int b = task.y + warp * LN::NPW; b < task.z; b += nwarps * LN::NPW) {
-      const int i = b + slot;
-      T ar = T(0), ai = T(0);
-      int4 nd = make_int4(0, 0, 0, 0);
-      if (i < task.z) nd = __ldg(Nd.node4 + i);
-      if (i < task.z && act) {
-        T w;
-        if constexpr (TABLE) {
-          w = __ldg(Nd.wtab + int64_t(i) * L + ix);
-        } else {
-          const T tt = __ldg(Nd.frac4 + 4 * int64_t(i)) - T(0.5);
-          w = c[LN::DEG - 1];
-#pragma unroll
-          for (int q = LN::DEG - 2; q >= 0; --q) w = fma(w, tt, c[q]);
-        }
-        const C v = tile[nd.x - o0 + ix];
-        ar = w * v.x;
-        ai = w * v.y;
-      }
-#pragma unroll
-      for (int o = LN::G1 / 2; o > 0; o >>= 1) {
-        ar += __shfl_xor_sync(0xFFFFFFFFu, ar, o);
-        ai += __shfl_xor_sync(0xFFFFFFFFu, ai, o);
-      }
-      if (ix == 0 && i < task.z) {
-        C r;
-        r.x = ar;
-        r.y = ai;
-        fhat[nd.w] = r;
-      }
-    }
-  } else {
-    PolyRegs<D, L, T> P;
-    if constexpr (!TABLE) P.load(G.coeffs, lane);
-    const int ix = lane % L, ry = lane / L;
-    const bool xact = ry < LN::RY;
-    for (int i = task.y + warp; i < task.z; i += nwarps) {
-      const int4 nd = __ldg(Nd.node4 + i);
-      T W[LN::NW];
-      node_weights<D, L, T, TABLE>(Nd, P, i, lane, W);
-      const T wx = wsel<D, L>(W, ix);
-      const int px = nd.x - o0 + ix, py = nd.y - o1;
-      int row[LN::NSTEP];
-      T wxy[LN::NSTEP];
+    T ar = T(0), ai = T(0);
+    if constexpr (D == 2) {
 #pragma unroll
       for (int s = 0; s < LN::NSTEP; ++s) {
-        const int iy = s * LN::RY + ry;
-        const bool ok = xact && iy < L;
-        const int iyc = ok ? iy : 0;
-        const T wy = wsel<D, L>(W, L + iyc);  // every lane shuffles
-        row[s] = (py + iyc) * pitch + px;
-        wxy[s] = ok ? wx * wy : T(0);
+        const C v = tile[row[s]];
+        ar = fma(wxy[s], v.x, ar);
+        ai = fma(wxy[s], v.y, ai);
       }
-      T ar = T(0), ai = T(0);
-      if constexpr (D == 2) {
+    } else {
+      const C* pl = tile + (nd.z - o2) * plane;
+#pragma unroll
+      for (int iz = 0; iz < L; ++iz) {
+        const T wz = wsel<D, L>(W, 2 * L + iz);
 #pragma unroll
         for (int s = 0; s < LN::NSTEP; ++s) {
-          const C v = tile[row[s]];
-          ar = fma(wxy[s], v.x, ar);
-          ai = fma(wxy[s], v.y, ai);
-        }
-      } else {
-        const C* pl = tile + (nd.z - o2) * plane;
-#pragma unroll
-        for (int iz = 0; iz < L; ++iz) {
-          const T wz = wsel<D, L>(W, 2 * L + iz);
-#pragma unroll
-          for (int s = 0; s < LN::NSTEP; ++s) {
-            const C v = pl[iz * plane + row[s]];
-            const T w = wxy[s] * wz;
-            ar = fma(w, v.x, ar);
-            ai = fma(w, v.y, ai);
-          }
+          const C v = pl[iz * plane + row[s]];
+          const T w = wxy[s] * wz;
+          ar = fma(w, v.x, ar);
+          ai = fma(w, v.y, ai);
         }
       }
+    }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        ar += __shfl_xor_sync(0xFFFFFFFFu, ar, o);
-        ai += __shfl_xor_sync(0xFFFFFFFFu, ai, o);
-      }
-      if (lane == 0) {
-        C r;
-        r.x = ar;
-        r.y = ai;
-        fhat[nd.w] = r;
-      }
+    for (int o = 16; o > 0; o >>= 1) {
+      ar += __shfl_xor_sync(0xFFFFFFFFu, ar, o);
+      ai += __shfl_xor_sync(0xFFFFFFFFu, ai, o);
+    }
+    if (lane == 0) {
+      C r;
+      r.x = ar;
+      r.y = ai;
+      fhat[nd.w] = r;
     }
   }
 }
@@ -530,6 +442,35 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   return NFFT_OK;
 }
 
+// D = 1 (line1.cuh).  A tile row of 1024 points is 8 KB: with fewer than 16 nodes per
+// task the nodes read the grid themselves.
+template <int L, typename T, bool TABLE>
+int gather_line_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* g,
+                       typename Cplx<T>::type* fhat, int ncols, int64_t gcol, int64_t fcol) {
+  LinePoly<L, T, TABLE> wp{};
+  if constexpr (!TABLE)
+    for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  const size_t smem = 2 * sizeof(T) * size_t(p->bs[0] + L - 1);
+  if (p->tasks && p->n_tasks > 0 && p->M >= 16 * p->n_tasks && smem <= 227 * 1024) {
+    auto kern = gather_line_kernel<L, T, TABLE, true>;
+    NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    // phases of the scattered stores: about 32 MB of output each from 64 MB on
+    // (2^24 nodes, 134 MB: 478 us in one phase, 291 in four; forward + adjoint
+    // 1356 / 1245 / 1233 / 1298 us with 1 / 2 / 4 / 8, 2^23 nodes 639 / 624 / 615 / 649)
+    const int64_t out = int64_t(2 * sizeof(T)) * p->M;
+    int64_t phases = out >= (int64_t(64) << 20) ? (out + (int64_t(32) << 20) - 1) / (int64_t(32) << 20) : 1;
+    phases = std::max<int64_t>(1, std::min<int64_t>(phases, p->M / (p->n_tasks * 64)));
+    kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols), unsigned(phases)), kLineThreads, smem, p->stream>>>(
+        G, Nd, p->tasks, g, fhat, gcol, fcol, wp);
+  } else {
+    const unsigned blocks = unsigned((p->M + kLineThreads - 1) / kLineThreads);
+    gather_line_kernel<L, T, TABLE, false><<<dim3(blocks, unsigned(ncols)), kLineThreads, 0, p->stream>>>(
+        G, Nd, nullptr, g, fhat, gcol, fcol, wp);
+  }
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
 // ncols columns in one launch (blockIdx.y): grids g + c gcol, values fhat + c fcol.
 template <int D, int L, typename T>
 int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int64_t gcol, int64_t fcol) {
@@ -537,52 +478,59 @@ int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int6
   Nodes<T> Nd = make_nodes<T>(p);
   if (Nd.M == 0) return NFFT_OK;
   using C = typename Cplx<T>::type;
-  const int64_t per_block = (kInterpThreads / 32) * (D == 1 ? Lanes<D, L>::NPW : 1);
-  int64_t blocks = (Nd.M + per_block - 1) / per_block;
-  int dev = 0, sms = 1;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-                                                cudaSuccess || sms < 1)
-    sms = 1;
-  const int64_t cap = (int64_t(sms) * 64 + ncols - 1) / ncols;
-  if (blocks > cap) blocks = cap;
   const C* gp = static_cast<const C*>(g);
   C* fp = static_cast<C*>(fhat);
-  if constexpr (D == 2) {
-    const int rc = p->wtab ? gather_warp2_launch<L, T, true>(p, G, Nd, gp, fp, ncols, gcol, fcol)
-                           : gather_warp2_launch<L, T, false>(p, G, Nd, gp, fp, ncols, gcol, fcol);
-    if (rc != -1) return rc;
-  }
-  if (ncols > 1) {
-    const dim3 grid{unsigned(blocks), unsigned(ncols), 1u};
-    if (p->wtab)
-      interp_kernel<D, L, T, true, true><<<grid, kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp, gcol, fcol);
-    else
-      interp_kernel<D, L, T, false, true><<<grid, kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp, gcol, fcol);
-    NFFT_LAUNCH_CHECK();
-    return NFFT_OK;
-  }
-  if constexpr (D == 3 && sizeof(T) == 4) {
-    const int rc = L == 8 ? interp_tile3(p, G, Nd, gp, fp) : launch_gather_plane3(p, g, fhat);
-    if (rc != -1) return rc;
-  }
-  if (p->tasks && p->gather_tiled) {
-    const int P1 = D >= 2 ? int(p->bs[1]) + L - 1 : 1;
-    const int P2 = D == 3 ? int(p->bs[2]) + L - 1 : 1;
-    const size_t smem = sizeof(C) * size_t(p->gather_pitch) * P1 * P2;
-    if (smem <= 227 * 1024 && p->n_tasks > 0) {
-      auto kern = p->wtab ? interp_tile_kernel<D, L, T, true> : interp_tile_kernel<D, L, T, false>;
-      NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-      kern<<<unsigned(p->n_tasks), kInterpThreads, smem, p->stream>>>(G, Nd, p->tasks, gp, fp, p->gather_pitch);
+  if constexpr (D == 1) {
+    // FP32 TENSOR plans: as in the spreader (spread.cu), Horner instead of the table's rows
+    return p->wtab && !(sizeof(T) == 4 && G.mode == WIN_POLY)
+               ? gather_line_launch<L, T, true>(p, G, Nd, gp, fp, ncols, gcol, fcol)
+               : gather_line_launch<L, T, false>(p, G, Nd, gp, fp, ncols, gcol, fcol);
+  } else {
+    const int64_t per_block = kInterpThreads / 32;
+    int64_t blocks = (Nd.M + per_block - 1) / per_block;
+    int dev = 0, sms = 1;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
+                                                  cudaSuccess || sms < 1)
+      sms = 1;
+    const int64_t cap = (int64_t(sms) * 64 + ncols - 1) / ncols;
+    if (blocks > cap) blocks = cap;
+    if constexpr (D == 2) {
+      const int rc = p->wtab ? gather_warp2_launch<L, T, true>(p, G, Nd, gp, fp, ncols, gcol, fcol)
+                             : gather_warp2_launch<L, T, false>(p, G, Nd, gp, fp, ncols, gcol, fcol);
+      if (rc != -1) return rc;
+    }
+    if (ncols > 1) {
+      const dim3 grid{unsigned(blocks), unsigned(ncols), 1u};
+      if (p->wtab)
+        interp_kernel<D, L, T, true, true><<<grid, kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp, gcol, fcol);
+      else
+        interp_kernel<D, L, T, false, true><<<grid, kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp, gcol, fcol);
       NFFT_LAUNCH_CHECK();
       return NFFT_OK;
     }
+    if constexpr (D == 3 && sizeof(T) == 4) {
+      const int rc = L == 8 ? interp_tile3(p, G, Nd, gp, fp) : launch_gather_plane3(p, g, fhat);
+      if (rc != -1) return rc;
+    }
+    if (p->tasks && p->gather_tiled) {
+      const int P1 = D >= 2 ? int(p->bs[1]) + L - 1 : 1;
+      const int P2 = D == 3 ? int(p->bs[2]) + L - 1 : 1;
+      const size_t smem = sizeof(C) * size_t(p->gather_pitch) * P1 * P2;
+      if (smem <= 227 * 1024 && p->n_tasks > 0) {
+        auto kern = p->wtab ? interp_tile_kernel<D, L, T, true> : interp_tile_kernel<D, L, T, false>;
+        NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        kern<<<unsigned(p->n_tasks), kInterpThreads, smem, p->stream>>>(G, Nd, p->tasks, gp, fp, p->gather_pitch);
+        NFFT_LAUNCH_CHECK();
+        return NFFT_OK;
+      }
+    }
+    if (p->wtab)
+      interp_kernel<D, L, T, true><<<unsigned(blocks), kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp);
+    else
+      interp_kernel<D, L, T, false><<<unsigned(blocks), kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp);
+    NFFT_LAUNCH_CHECK();
+    return NFFT_OK;
   }
-  if (p->wtab)
-    interp_kernel<D, L, T, true><<<unsigned(blocks), kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp);
-  else
-    interp_kernel<D, L, T, false><<<unsigned(blocks), kInterpThreads, 0, p->stream>>>(G, Nd, gp, fp);
-  NFFT_LAUNCH_CHECK();
-  return NFFT_OK;
 }
 
 #define NFFT_INTERP_ARGS p, g, fhat, ncols, gcol, fcol

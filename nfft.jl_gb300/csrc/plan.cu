@@ -777,7 +777,9 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     // 4,000 nodes 42 / 44 / 44 / 44, 20,000 nodes 42 / 48 / 58 / 79, 200,000
     // nodes 58 / 63 / 67 / 85, 800,000 nodes 115 / 116 / 121 / 143; 64 slices of
     // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
-    int chunk = 1024;
+    // D = 1: 2048, so that tiles of about 1024 nodes are not cut into a task
+    // of 1024 and one of a few (line1.cuh takes a task in equal batches).
+    int chunk = D == 1 ? 2048 : 1024;
     if (D == 2 && !p->prm.compensated) {
       const int64_t work = M * p->task_columns;
       chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;

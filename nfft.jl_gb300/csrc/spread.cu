@@ -22,6 +22,7 @@
 //     (red.global.add.v2), wrapping periodically; all-zero points are skipped.
 // The lock of the reference becomes the L2 atomics of the flush.
 #include "spread_body.cuh"
+#include "line1.cuh"
 #include "spread_tile3.cuh"
 #include "warp2.cuh"
 
@@ -37,6 +38,22 @@ __global__ void __launch_bounds__(32) spread_warp2_kernel(Geom<T> G, Nodes<T> Nd
   extern __shared__ __align__(32) unsigned char smem_raw[];
   spread_warp2_body<L, T, TABLE>(G, Nd, __ldg(tasks + blockIdx.x), fhat + blockIdx.y * fcol, g + blockIdx.y * gcol,
                                  pitch, wp.c, smem_raw);
+}
+
+template <int L, typename T, bool TABLE, bool KAHAN>
+int spread_line_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* fhat, T* g,
+                       int ncols, int64_t fcol, int64_t gcol_t) {
+  const size_t smem = Line1<L, T, KAHAN>::smem(int(p->bs[0]));
+  if (smem > 227 * 1024) return -1;
+  LinePoly<L, T, TABLE> wp{};
+  if constexpr (!TABLE)
+    for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  auto kern = spread_line_kernel<L, T, TABLE, KAHAN>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), kLineThreads, smem, p->stream>>>(G, Nd, p->tasks, fhat, g, fcol,
+                                                                                      gcol_t, wp);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
 }
 
 template <int L, typename T, bool TABLE>
@@ -132,6 +149,23 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
     return NFFT_ERR_UNSUPPORTED;
   }
   if constexpr (D == 1) {
+    // the sorting spreader, up to 1024 cells (the counts and their scan outgrow
+    // the CTA) and from 3 nodes per 2 cells of the occupied tiles on: its sort
+    // and scan cost the same for few nodes (forward + adjoint, us, against the
+    // per-node kernels below: 0.5 nodes per cell 173 / 162, 1.2 nodes 50 / 49, 2
+    // nodes 1233 / 1540 compensated, 30 nodes 180 / 222, 1500 nodes 243 / 448)
+    if (p->bs[0] <= kLineMaxTile && 2 * p->M >= 3 * p->n_tasks * p->bs[0]) {
+      // FP32 TENSOR plans: Horner (2m multiply-adds a value) gives the table's own
+      // values for less than reading them; FP64 units are too few for that
+      const bool table = p->wtab && !(sizeof(T) == 4 && G.mode == WIN_POLY);
+      const int rc =
+          p->prm.compensated
+              ? (table ? spread_line_launch<L, T, true, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
+                       : spread_line_launch<L, T, false, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t))
+              : (table ? spread_line_launch<L, T, true, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
+                       : spread_line_launch<L, T, false, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t));
+      if (rc != -1) return rc;
+    }
     if (p->prm.compensated) {
       const size_t smem = ((sizeof(typename Acc<T, true>::type) * size_t(p->bs[0] + L - 1) + 31) & ~size_t(31)) +
                           sizeof(T) * size_t(2 * 32 * L + L * (L + 1));
