@@ -119,18 +119,18 @@ template <int S, int R, typename C> __device__ __forceinline__ void dft(C (&v)[R
 // butterfly j of line w loads positions j + r N/R, twiddles by
 // (j mod NS) r / (NS R) turns, transforms, and stores at
 // (j div NS) NS R + (j mod NS) + r NS.
-template <typename T, int S, int N, int W, int R, int NS>
+template <typename T, int S, int N, int W, int NT, int R, int NS>
 __device__ __forceinline__ void fft_pass(Cx<T>* buf, const Cx<T>* __restrict__ tw) {
   using C = Cx<T>;
   constexpr int NB = N / R;
   constexpr int TOT = NB * W;
-  constexpr int BPT = (TOT + kFftThreads - 1) / kFftThreads;
+  constexpr int BPT = (TOT + NT - 1) / NT;
   constexpr int P = W + 1;
   C v[BPT][R];
 #pragma unroll
   for (int b = 0; b < BPT; ++b) {
-    const int t = threadIdx.x + b * kFftThreads;
-    if (TOT % kFftThreads == 0 || t < TOT) {
+    const int t = threadIdx.x + b * NT;
+    if (TOT % NT == 0 || t < TOT) {
       const int w = t % W, j = t / W;
 #pragma unroll
       for (int r = 0; r < R; ++r) v[b][r] = buf[(j + r * NB) * P + w];
@@ -139,8 +139,8 @@ __device__ __forceinline__ void fft_pass(Cx<T>* buf, const Cx<T>* __restrict__ t
   __syncthreads();
 #pragma unroll
   for (int b = 0; b < BPT; ++b) {
-    const int t = threadIdx.x + b * kFftThreads;
-    if (TOT % kFftThreads == 0 || t < TOT) {
+    const int t = threadIdx.x + b * NT;
+    if (TOT % NT == 0 || t < TOT) {
       const int w = t % W, j = t / W;
       const int k = j & (NS - 1);
       if constexpr (NS > 1) {
@@ -161,13 +161,13 @@ __device__ __forceinline__ void fft_pass(Cx<T>* buf, const Cx<T>* __restrict__ t
   __syncthreads();
 }
 
-template <typename T, int S, int N, int W, int NS = 1>
+template <typename T, int S, int N, int W, int NT, int NS = 1>
 __device__ __forceinline__ void fft_lines(Cx<T>* buf, const Cx<T>* __restrict__ tw) {
   if constexpr (NS < N) {
     constexpr int REM = N / NS;
     constexpr int R = REM % 8 == 0 ? 8 : REM;
-    fft_pass<T, S, N, W, R, NS>(buf, tw);
-    fft_lines<T, S, N, W, NS * R>(buf, tw);
+    fft_pass<T, S, N, W, NT, R, NS>(buf, tw);
+    fft_lines<T, S, N, W, NT, NS * R>(buf, tw);
   }
 }
 
@@ -189,11 +189,11 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 #define NFFT_TOE_PREFETCH 1
 #endif
 
-// Move the W x n tile elements q = threadIdx.x + i * kFftThreads through
+// Move the W x n tile elements q = threadIdx.x + i * NT through
 // registers in batches of up to 8: every load of a batch is issued before
 // its stores, so a thread keeps a batch of global (or shared) loads in flight
 // instead of one load-store round trip per element.
-template <typename C, int ITEMS, typename Load, typename Store>
+template <typename C, int ITEMS, int NT, typename Load, typename Store>
 __device__ __forceinline__ void staged_copy(Load ld, Store st) {
   constexpr int CH = ITEMS < 8 ? ITEMS : 8;
   static_assert(ITEMS % CH == 0, "tile items per thread");
@@ -201,9 +201,9 @@ __device__ __forceinline__ void staged_copy(Load ld, Store st) {
   for (int c0 = 0; c0 < ITEMS; c0 += CH) {
     C v[CH];
 #pragma unroll
-    for (int i = 0; i < CH; ++i) v[i] = ld(int(threadIdx.x) + (c0 + i) * kFftThreads);
+    for (int i = 0; i < CH; ++i) v[i] = ld(int(threadIdx.x) + (c0 + i) * NT);
 #pragma unroll
-    for (int i = 0; i < CH; ++i) st(int(threadIdx.x) + (c0 + i) * kFftThreads, v[i]);
+    for (int i = 0; i < CH; ++i) st(int(threadIdx.x) + (c0 + i) * NT, v[i]);
   }
 }
 
@@ -226,8 +226,8 @@ template <typename T> struct Inv3 {
 };
 
 // forward X: image rows -> deconvolved, zero-padded, transformed grid rows
-template <typename T, int NX, int W>
-__global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, true>()) fft_x_pad_kernel(FftGeom G, Inv3<T> inv, const Cx<T>* __restrict__ f,
+template <typename T, int NX, int W, int NT = kFftThreads>
+__global__ void __launch_bounds__(NT, NT < kFftThreads ? 1 : fft_min_blocks<T, NX, true>()) fft_x_pad_kernel(FftGeom G, Inv3<T> inv, const Cx<T>* __restrict__ f,
                                                                 Cx<T>* __restrict__ g, const Cx<T>* __restrict__ tw, void* const* slot) {
   using C = Cx<T>;
   if (slot) f = static_cast<const C*>(slot[0]);  // image pointer read from device memory
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, true>()) ff
   const int64_t rows = int64_t(G.N[1]) * G.N[2];
   const int64_t r0 = int64_t(blockIdx.x) * W;
   const int N0 = G.N[0], h0 = G.N[0] / 2;
-  constexpr int ITEMS = NX * W / kFftThreads;
+  constexpr int ITEMS = NX * W / NT;
   // per row: the y / z deconvolution factor and the grid row offset
   __shared__ T s_row[W];
   __shared__ int64_t s_goff[W];
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, true>()) ff
   // raw image values land asynchronously; padding positions are zeroed
 #pragma unroll 4
   for (int i = 0; i < ITEMS; ++i) {
-    const int q = int(threadIdx.x) + i * kFftThreads;
+    const int q = int(threadIdx.x) + i * NT;
     const int pos = q % NX, w = q / NX;
     const int nx = wrap_once(pos + h0, NX);
     if (r0 + w < rows && nx < N0) {
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, true>()) ff
   // deconvolution factors (each thread scales the elements it copied)
 #pragma unroll 4
   for (int i = 0; i < ITEMS; ++i) {
-    const int q = int(threadIdx.x) + i * kFftThreads;
+    const int q = int(threadIdx.x) + i * NT;
     const int pos = q % NX, w = q / NX;
     const int nx = wrap_once(pos + h0, NX);
     if (nx < N0) {
@@ -287,16 +287,16 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, true>()) ff
     }
   }
   __syncthreads();
-  fft_lines<T, -1, NX, W>(buf, tw);
-  staged_copy<C, ITEMS>([&](int q) { return buf[(q % NX) * P + q / NX]; },
+  fft_lines<T, -1, NX, W, NT>(buf, tw);
+  staged_copy<C, ITEMS, NT>([&](int q) { return buf[(q % NX) * P + q / NX]; },
                         [&](int q, C v) {
                           if (r0 + q / NX < rows) g[s_goff[q / NX] + q % NX] = v;
                         });
 }
 
 // adjoint X': grid rows of the image -> transformed, cropped, deconvolved image rows
-template <typename T, int NX, int W>
-__global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, false>()) fft_x_crop_kernel(FftGeom G, Inv3<T> inv, const Cx<T>* __restrict__ g,
+template <typename T, int NX, int W, int NT = kFftThreads>
+__global__ void __launch_bounds__(NT, NT < kFftThreads ? 1 : fft_min_blocks<T, NX, false>()) fft_x_crop_kernel(FftGeom G, Inv3<T> inv, const Cx<T>* __restrict__ g,
                                                                  Cx<T>* __restrict__ f, const Cx<T>* __restrict__ tw, void* const* slot) {
   if (slot) f = static_cast<Cx<T>*>(slot[0]);  // image pointer read from device memory
   using C = Cx<T>;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, false>()) f
   const int64_t rows = int64_t(G.N[1]) * G.N[2];
   const int64_t r0 = int64_t(blockIdx.x) * W;
   const int N0 = G.N[0], h0 = G.N[0] / 2;
-  constexpr int ITEMS = NX * W / kFftThreads;
+  constexpr int ITEMS = NX * W / NT;
   __shared__ T s_row[W];
   __shared__ int64_t s_goff[W];
   if (threadIdx.x < W) {
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, false>()) f
   __syncthreads();
 #pragma unroll 4
   for (int i = 0; i < ITEMS; ++i) {
-    const int q = int(threadIdx.x) + i * kFftThreads;
+    const int q = int(threadIdx.x) + i * NT;
     const int pos = q % NX, w = q / NX;
     if (r0 + w < rows) {
       cp_async_elem(buf + pos * P + w, g + s_goff[w] + pos);
@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NX, false>()) f
   }
   cp_async_wait_all();
   __syncthreads();
-  fft_lines<T, 1, NX, W>(buf, tw);
-  staged_copy<C, ITEMS>([&](int q) { return buf[(q % NX) * P + q / NX]; },
+  fft_lines<T, 1, NX, W, NT>(buf, tw);
+  staged_copy<C, ITEMS, NT>([&](int q) { return buf[(q % NX) * P + q / NX]; },
                         [&](int q, C v) {
                           const int pos = q % NX, w = q / NX;
                           const int nx = wrap_once(pos + h0, NX);
@@ -366,8 +366,8 @@ struct LineGeom {
   int outer_N, outer_Nt;
 };
 
-template <typename T, int NL, int W, bool FWD>
-__global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, FWD>()) fft_lines_kernel(LineGeom L, Cx<T>* __restrict__ g,
+template <typename T, int NL, int W, bool FWD, int NT = kFftThreads>
+__global__ void __launch_bounds__(NT, NT < kFftThreads ? 1 : fft_min_blocks<T, NL, FWD>()) fft_lines_kernel(LineGeom L, Cx<T>* __restrict__ g,
                                                                 const Cx<T>* __restrict__ tw) {
   using C = Cx<T>;
   extern __shared__ __align__(16) unsigned char fft_smem[];
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, FWD>()) fft
   const int head = L.n_img - L.n_img / 2;   // image positions [0, head) and [NL - n_img/2, NL)
   const int tail0 = NL - L.n_img / 2;
   // thread -> fixed column w, positions p0, p0 + PS, ...
-  constexpr int PS = kFftThreads / W;
+  constexpr int PS = NT / W;
   const int w = threadIdx.x % W, p0 = threadIdx.x / W;
   const C* src = base + w + int64_t(p0) * L.stride;
   const int64_t step = int64_t(PS) * L.stride;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, FWD>()) fft
   }
   cp_async_wait_all();
   __syncthreads();
-  fft_lines<T, FWD ? -1 : 1, NL, W>(buf, tw);
+  fft_lines<T, FWD ? -1 : 1, NL, W, NT>(buf, tw);
   C* dst = base + w + int64_t(p0) * L.stride;
 #pragma unroll 4
   for (int pos = p0; pos < NL; pos += PS, dst += step)
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, false>()) f
   }
   cp_async_wait_all();
   __syncthreads();
-  fft_lines<T, -1, NL, W>(buf, tw);
+  fft_lines<T, -1, NL, W, kFftThreads>(buf, tw);
   const C* lsrc = lam + off + w + int64_t(p0) * L.stride;
 #pragma unroll 4
   for (int pos = p0; pos < NL; pos += PS, lsrc += step) {
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, false>()) f
     buf[pos * P + w] = c_mul(buf[pos * P + w], l);
   }
   __syncthreads();
-  fft_lines<T, 1, NL, W>(buf, tw);
+  fft_lines<T, 1, NL, W, kFftThreads>(buf, tw);
   C* dst = base + w + int64_t(p0) * L.stride;
 #pragma unroll 4
   for (int pos = p0; pos < NL; pos += PS, dst += step)
@@ -465,8 +465,19 @@ __global__ void __launch_bounds__(kFftThreads, fft_min_blocks<T, NL, false>()) f
 #endif
 template <typename T> constexpr int lines_per_cta() { return sizeof(T) == 4 ? NFFT_FFT_W32 : NFFT_FFT_W64; }
 
-template <int NL, typename T> size_t fft_smem_bytes() {
-  return size_t(NL) * (lines_per_cta<T>() + 1) * sizeof(Cx<T>);
+// Small transforms: with W lines per CTA as above a 256^2 image makes 16 to 32
+// CTAs.  When they would not reach half of the SMs, a CTA takes fewer lines
+// (and proportionally fewer threads): x rows one by one (FP64; the FP64 units
+// are what bounds them) or in pairs, y / z lines at least a 32-byte sector of
+// columns together.  128^2 FP64 image: x passes 20 -> 12, y passes 18 -> 10 us,
+// forward + adjoint 113 -> 81 us; 256^2 FP32 image: x 12 -> 10, y 6.6 -> 6.0 us.
+// From 128 CTAs on the full width is the faster one (64^3 FP64 grid, 4000 nodes:
+// 147 us, 152 with the x rows one by one).
+template <typename T> constexpr int small_x_lines() { return sizeof(T) == 4 ? 2 : 1; }
+template <typename T> constexpr int small_y_lines() { return sizeof(T) == 4 ? 4 : 2; }
+
+template <int NL, typename T> size_t fft_smem_bytes(int W = lines_per_cta<T>()) {
+  return size_t(NL) * (W + 1) * sizeof(Cx<T>);
 }
 
 
@@ -658,13 +669,12 @@ __global__ void zmask_kernel(const int32_t* __restrict__ tstart, int nt0, int nt
 // reads only those (the spreading wrote nothing else into the zeroed grid)
 // and skips blocks with none: their lines are zero, and so is their
 // transform, which the zeroed grid already holds.  MASK = 0: no mask.
-template <int NL, bool FWD, int MASK>
-__global__ void __launch_bounds__(256, 3) fft4_lines_staged_kernel(LineGeom L, float2* __restrict__ g,
-                                                                   const float2* __restrict__ tw,
-                                                                   const unsigned long long* __restrict__ zmask) {
+template <int NL, bool FWD, int MASK, int W = kW4>
+__global__ void __launch_bounds__(16 * W, W == kW4 ? 3 : 1) fft4_lines_staged_kernel(
+    LineGeom L, float2* __restrict__ g, const float2* __restrict__ tw, const unsigned long long* __restrict__ zmask) {
   using C = float2;
-  constexpr int R1 = Split4<NL>::R1, R2 = Split4<NL>::R2, W = kW4, S = FWD ? -1 : 1;
-  static_assert(W == 16, "a row of the tile is 8 16-byte chunks");
+  constexpr int R1 = Split4<NL>::R1, R2 = Split4<NL>::R2, S = FWD ? -1 : 1, NT = 16 * W, CH = W / 2;
+  static_assert(W % 2 == 0 && (MASK == 0 || W == 16), "rows of 16-byte chunks; the mask's blocks of 16 columns");
   extern __shared__ __align__(16) unsigned char fft_smem[];
   C* buf = reinterpret_cast<C*>(fft_smem);
   const int tile = blockIdx.x % L.tiles_x;
@@ -675,9 +685,9 @@ __global__ void __launch_bounds__(256, 3) fft4_lines_staged_kernel(LineGeom L, f
   const unsigned long long live = MASK == 2 ? __ldg(zmask + int64_t(o) * L.tiles_x + tile) : ~0ull;
   if (MASK == 2 && live == 0) return;  // nothing of these lines is read (forward) or non-zero (inverse)
   auto used = [&](int pos) { return MASK != 2 || ((live >> (pos >> 3)) & 1ull) != 0; };
-  // stage the tile: NL rows of W complex values (8 chunks of 16 bytes)
-  for (int c = threadIdx.x; c < NL * 8; c += 256) {
-    const int row = c >> 3, part = c & 7;
+  // stage the tile: NL rows of W complex values (CH chunks of 16 bytes)
+  for (int c = threadIdx.x; c < NL * CH; c += NT) {
+    const int row = c / CH, part = c % CH;
     if ((!FWD || row < head || row >= tail0) && (FWD || used(row))) {
       const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(buf + row * W + 2 * part));
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
@@ -688,11 +698,11 @@ __global__ void __launch_bounds__(256, 3) fft4_lines_staged_kernel(LineGeom L, f
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // R1-point DFTs in place: thread (w, n2) owns rows R2 n1 + n2 of column w
-  constexpr int T1 = W * R2, B1 = (T1 + 255) / 256;
+  constexpr int T1 = W * R2, B1 = (T1 + NT - 1) / NT;
 #pragma unroll
   for (int b = 0; b < B1; ++b) {
-    const int task = int(threadIdx.x) + b * 256;
-    if (T1 % 256 == 0 || task < T1) {
+    const int task = int(threadIdx.x) + b * NT;
+    if (T1 % NT == 0 || task < T1) {
       const int w = task % W, n2 = task / W;
       C v[R1];
 #pragma unroll
@@ -710,11 +720,11 @@ __global__ void __launch_bounds__(256, 3) fft4_lines_staged_kernel(LineGeom L, f
   }
   __syncthreads();
   // R2-point DFTs: thread (w, k1) reads rows R2 k1 .. R2 k1 + R2 - 1
-  constexpr int T2 = W * R1, B2 = (T2 + 255) / 256;
+  constexpr int T2 = W * R1, B2 = (T2 + NT - 1) / NT;
 #pragma unroll
   for (int b = 0; b < B2; ++b) {
-    const int task = int(threadIdx.x) + b * 256;
-    if (T2 % 256 == 0 || task < T2) {
+    const int task = int(threadIdx.x) + b * NT;
+    if (T2 % NT == 0 || task < T2) {
       const int w = task % W, k1 = task / W;
       C v[R2];
 #pragma unroll
@@ -731,14 +741,14 @@ __global__ void __launch_bounds__(256, 3) fft4_lines_staged_kernel(LineGeom L, f
 
 // x lines of the image rows: forward pad + deconvolution + FFT (FWD), or
 // backward FFT + crop + deconvolution.
-template <int NX, bool FWD>
-__global__ void __launch_bounds__(256, FWD ? 3 : 2) fft4_x_kernel(FftGeom G, Inv3<float> inv,
+template <int NX, bool FWD, int W = kW4>
+__global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : (FWD ? 3 : 2)) fft4_x_kernel(FftGeom G, Inv3<float> inv,
                                                                   const float2* __restrict__ src,
                                                                   float2* __restrict__ dst,
                                                                   const float2* __restrict__ tw,
                                                                   void* const* slot) {
   using C = float2;
-  constexpr int R1 = Split4<NX>::R1, R2 = Split4<NX>::R2, W = kW4, PR = R1 + 1, PW = R2 * PR, S = FWD ? -1 : 1;
+  constexpr int R1 = Split4<NX>::R1, R2 = Split4<NX>::R2, PR = R1 + 1, PW = R2 * PR, S = FWD ? -1 : 1, NT = 16 * W;
   if (slot) {  // the image pointer is read from device memory (graph replays with new arrays)
     if (FWD) src = static_cast<const float2*>(slot[0]);
     else dst = static_cast<float2*>(slot[0]);
@@ -764,11 +774,11 @@ __global__ void __launch_bounds__(256, FWD ? 3 : 2) fft4_x_kernel(FftGeom G, Inv
     s_goff[threadIdx.x] = goff;
   }
   __syncthreads();
-  constexpr int T1 = W * R2, B1 = (T1 + 255) / 256;
+  constexpr int T1 = W * R2, B1 = (T1 + NT - 1) / NT;
 #pragma unroll
   for (int b = 0; b < B1; ++b) {
-    const int task = int(threadIdx.x) + b * 256;
-    if (T1 % 256 == 0 || task < T1) {
+    const int task = int(threadIdx.x) + b * NT;
+    if (T1 % NT == 0 || task < T1) {
       const int n2 = task % R2, w = task / R2;
       const bool live = r0 + w < rows;
       C v[R1];
@@ -796,11 +806,11 @@ __global__ void __launch_bounds__(256, FWD ? 3 : 2) fft4_x_kernel(FftGeom G, Inv
     }
   }
   __syncthreads();
-  constexpr int T2 = W * R1, B2 = (T2 + 255) / 256;
+  constexpr int T2 = W * R1, B2 = (T2 + NT - 1) / NT;
 #pragma unroll
   for (int b = 0; b < B2; ++b) {
-    const int task = int(threadIdx.x) + b * 256;
-    if (T2 % 256 == 0 || task < T2) {
+    const int task = int(threadIdx.x) + b * NT;
+    if (T2 % NT == 0 || task < T2) {
       const int k1 = task % R1, w = task / R1;
       if (r0 + w < rows) {
         C v[R2];
@@ -958,37 +968,45 @@ template <typename K> int set_smem(K kern, size_t bytes) {
   return NFFT_OK;
 }
 
-template <typename T, int NX> int x_pass_t(nfft_plan* p, const void* src, void* dst, bool fwd, void* const* slot) {
+template <typename T, int NX, int W> int x_pass_w(nfft_plan* p, const void* src, void* dst, bool fwd, void* const* slot) {
   using C = Cx<T>;
+  const unsigned blocks = unsigned((p->N[1] * p->N[2] + W - 1) / W);
   if constexpr (sizeof(T) == 4 && NX <= 512 && NFFT_FFT_FOURSTEP) {
-    const size_t smem = size_t(kW4) * Split4<NX>::R2 * (Split4<NX>::R1 + 1) * sizeof(float2);
-    const unsigned blocks = unsigned((p->N[1] * p->N[2] + kW4 - 1) / kW4);
+    const size_t smem = size_t(W) * Split4<NX>::R2 * (Split4<NX>::R1 + 1) * sizeof(float2);
     const float2* tw = static_cast<const float2*>(p->fft_tw[0]);
-    auto kern = fwd ? fft4_x_kernel<NX, true> : fft4_x_kernel<NX, false>;
+    auto kern = fwd ? fft4_x_kernel<NX, true, W> : fft4_x_kernel<NX, false, W>;
     if (int rc = set_smem(kern, smem)) return rc;
-    kern<<<blocks, 256, smem, p->stream>>>(make_fft_geom(p), make_inv3<float>(p), static_cast<const float2*>(src),
-                                           static_cast<float2*>(dst), tw, slot);
+    kern<<<blocks, 16 * W, smem, p->stream>>>(make_fft_geom(p), make_inv3<float>(p), static_cast<const float2*>(src),
+                                              static_cast<float2*>(dst), tw, slot);
     NFFT_LAUNCH_CHECK();
     return NFFT_OK;
   }
-  constexpr int W = lines_per_cta<T>();
-  const size_t smem = fft_smem_bytes<NX, T>();
-  const int64_t rows = p->N[1] * p->N[2];
-  const unsigned blocks = unsigned((rows + W - 1) / W);
+  constexpr int NT = kFftThreads * W / lines_per_cta<T>();
+  const size_t smem = fft_smem_bytes<NX, T>(W);
   const C* tw = static_cast<const C*>(p->fft_tw[0]);
   if (fwd) {
-    auto kern = fft_x_pad_kernel<T, NX, W>;
+    auto kern = fft_x_pad_kernel<T, NX, W, NT>;
     if (int rc = set_smem(kern, smem)) return rc;
-    kern<<<blocks, kFftThreads, smem, p->stream>>>(make_fft_geom(p), make_inv3<T>(p), static_cast<const C*>(src),
-                                                   static_cast<C*>(dst), tw, slot);
+    kern<<<blocks, NT, smem, p->stream>>>(make_fft_geom(p), make_inv3<T>(p), static_cast<const C*>(src),
+                                          static_cast<C*>(dst), tw, slot);
   } else {
-    auto kern = fft_x_crop_kernel<T, NX, W>;
+    auto kern = fft_x_crop_kernel<T, NX, W, NT>;
     if (int rc = set_smem(kern, smem)) return rc;
-    kern<<<blocks, kFftThreads, smem, p->stream>>>(make_fft_geom(p), make_inv3<T>(p), static_cast<const C*>(src),
-                                                   static_cast<C*>(dst), tw, slot);
+    kern<<<blocks, NT, smem, p->stream>>>(make_fft_geom(p), make_inv3<T>(p), static_cast<const C*>(src),
+                                          static_cast<C*>(dst), tw, slot);
   }
   NFFT_LAUNCH_CHECK();
   return NFFT_OK;
+}
+
+// Whether `lines` lines, W per CTA, leave half of the SMs of the plan's GPU without a CTA.
+bool few_ctas(const nfft_plan* p, int64_t lines, int W) { return 2 * lines <= int64_t(W) * p->sms; }
+
+template <typename T, int NX> int x_pass_t(nfft_plan* p, const void* src, void* dst, bool fwd, void* const* slot) {
+  static_assert(kW4 == lines_per_cta<float>(), "lines per CTA");
+  if (few_ctas(p, p->N[1] * p->N[2], lines_per_cta<T>()))
+    return x_pass_w<T, NX, small_x_lines<T>()>(p, src, dst, fwd, slot);
+  return x_pass_w<T, NX, lines_per_cta<T>()>(p, src, dst, fwd, slot);
 }
 
 // Line geometry of a pass along `axis` (1: y, 2: z) with W lines per CTA.
@@ -1052,6 +1070,23 @@ static const unsigned long long* zmask_for(nfft_plan* p) {
   return static_cast<const unsigned long long*>(p->zmask);
 }
 
+// Stockham line passes with W lines per CTA.
+template <typename T, int NL, int W> int line_pass_w(nfft_plan* p, int axis, bool fwd) {
+  using C = Cx<T>;
+  constexpr int NT = kFftThreads * W / lines_per_cta<T>();
+  const C* tw = static_cast<const C*>(p->fft_tw[axis]);
+  C* g = static_cast<C*>(p->grid);
+  int64_t outer_count;
+  const size_t smem = fft_smem_bytes<NL, T>(W);
+  const LineGeom L = make_line_geom(p, axis, W, &outer_count);
+  const unsigned blocks = unsigned(outer_count * L.tiles_x);
+  auto kern = fwd ? fft_lines_kernel<T, NL, W, true, NT> : fft_lines_kernel<T, NL, W, false, NT>;
+  if (int rc = set_smem(kern, smem)) return rc;
+  kern<<<blocks, NT, smem, p->stream>>>(L, g, tw);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
 template <typename T, int NL> int line_pass_t(nfft_plan* p, int axis, bool fwd) {
   using C = Cx<T>;
   const C* tw = static_cast<const C*>(p->fft_tw[axis]);
@@ -1060,6 +1095,16 @@ template <typename T, int NL> int line_pass_t(nfft_plan* p, int axis, bool fwd) 
   if constexpr (sizeof(T) == 4 && NL <= 512 && NFFT_FFT_FOURSTEP) {
     const LineGeom L = make_line_geom(p, axis, kW4, &outer_count);
     const unsigned blocks4 = unsigned(outer_count * L.tiles_x);
+    constexpr int SW = small_y_lines<T>();
+    if (p->fft_staged && few_ctas(p, outer_count * p->Nt[0], kW4)) {
+      const LineGeom LS = make_line_geom(p, axis, SW, &outer_count);
+      const size_t smem_s = size_t(NL) * SW * sizeof(float2);
+      auto ks = fwd ? fft4_lines_staged_kernel<NL, true, 0, SW> : fft4_lines_staged_kernel<NL, false, 0, SW>;
+      if (int rc = set_smem(ks, smem_s)) return rc;
+      ks<<<unsigned(outer_count * LS.tiles_x), 16 * SW, smem_s, p->stream>>>(LS, g, tw, nullptr);
+      NFFT_LAUNCH_CHECK();
+      return NFFT_OK;
+    }
     if (p->fft_staged) {  // tile staged by cp.async, in-place four-step
       const size_t smem_s = size_t(NL) * kW4 * sizeof(float2);
       const unsigned long long* zm = axis == 2 ? zmask_for(p) : nullptr;
@@ -1078,21 +1123,10 @@ template <typename T, int NL> int line_pass_t(nfft_plan* p, int axis, bool fwd) 
     NFFT_LAUNCH_CHECK();
     return NFFT_OK;
   }
-  constexpr int W = lines_per_cta<T>();
-  const size_t smem = fft_smem_bytes<NL, T>();
-  const LineGeom L = make_line_geom(p, axis, W, &outer_count);
-  const unsigned blocks = unsigned(outer_count * L.tiles_x);
-  if (fwd) {
-    auto kern = fft_lines_kernel<T, NL, W, true>;
-    if (int rc = set_smem(kern, smem)) return rc;
-    kern<<<blocks, kFftThreads, smem, p->stream>>>(L, g, tw);
-  } else {
-    auto kern = fft_lines_kernel<T, NL, W, false>;
-    if (int rc = set_smem(kern, smem)) return rc;
-    kern<<<blocks, kFftThreads, smem, p->stream>>>(L, g, tw);
-  }
-  NFFT_LAUNCH_CHECK();
-  return NFFT_OK;
+  make_line_geom(p, axis, 1, &outer_count);
+  return few_ctas(p, outer_count * p->Nt[0], lines_per_cta<T>())
+             ? line_pass_w<T, NL, small_y_lines<T>()>(p, axis, fwd)
+             : line_pass_w<T, NL, lines_per_cta<T>()>(p, axis, fwd);
 }
 
 // The fused forward FFT x lambda x backward FFT pass along the last axis.

@@ -96,6 +96,7 @@ struct nfft_plan {
   int64_t ntiles[3] = {1, 1, 1};
   int64_t ntiles_total = 1;
   cudaStream_t stream = nullptr;
+  int sms = 1;                // SMs of the plan's GPU
   // FFT of the oversampled grid.  D = 1: one plan.  D >= 2 (pruned): the
   // image occupies a head and a tail range along the last dimension, so the
   // transform runs as batched (D-1)-dimensional FFTs over those slices only

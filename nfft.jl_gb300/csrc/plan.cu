@@ -518,6 +518,12 @@ int nfft_plan_create(nfft_plan** out, int precision, int D, const int64_t* N, in
   p->prm = prm;
   p->m = prm.m;
   p->stream = static_cast<cudaStream_t>(stream);
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || p->sms < 1)
+      p->sms = 1;
+  }
   int64_t total = 1;
   for (int d = 0; d < D; ++d) {
     if (N[d] < 1) {
