@@ -182,7 +182,7 @@ struct nfft_plan {
          NB_KEY2, NB_VAL2, NB_TCOUNT, NB_SCR, NB_TCNT, NB_TOFF, NB_COUNT };
   void* nbuf[NB_COUNT] = {};
   size_t nbuf_cap[NB_COUNT] = {};
-  int* dflag = nullptr;            // device status words: [0] node check, [1] an async copy wait that timed out
+  int* dflag = nullptr;            // device words: [0] node check, [1] an async copy wait that timed out, [2] task count
   size_t scratch_bytes = 0;
 
   // TimingStats: every forward/adjoint records 4 events into a ring slot; the
@@ -205,12 +205,13 @@ namespace nfft {
 int launch_check_nodes(const nfft_plan* p, const void* k, int* flag);
 // the same check on n values of the given precision, without a plan
 int launch_check_node_values(int precision, const void* k, int64_t n, int* flag, cudaStream_t s);
+// flag (optional): set to 1 if a node fails checkNodes
 int launch_reduce_nodes(const nfft_plan* p, const void* k, int32_t* ti_u, void* te_u, uint32_t* key,
-                        int32_t* val, int32_t* tile_count);
+                        int32_t* val, int32_t* tile_count, int* flag = nullptr);
 int launch_build_node_tables(const nfft_plan* p, const int32_t* perm, const int32_t* ti_u, const void* te_u);
 int launch_build_weight_table(const nfft_plan* p);
 int launch_deconv_factors(nfft_plan* p);
-int launch_build_tasks(nfft_plan* p, int chunk);
+int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks);
 // autotune.cu
 int apply_block_size(nfft_plan* p, const int64_t* bs, const void* k, int ny);
 // spread.cu: bank-conflict-free row pitch of a padded spreading tile
@@ -474,9 +475,10 @@ __device__ __forceinline__ T tap_weight(const Geom<T>& G, const T* __restrict__ 
     T x = e + T(G.m - 1 - l);
     T u = (x < T(0) ? -x : x) * G.lut_scale;
     // the LUT holds LUTSize+2 samples; an offset a hair outside [0,1)
-    // (FP32 nodes) must not index past them
+    // (FP32 nodes), or of a node that the check is about to reject (NaN
+    // included), must not index past them
     const T umax = T(G.m) * G.lut_scale;
-    if (u > umax) u = umax;
+    if (!(u <= umax)) u = umax;
     T fi = floor(u);
     int i = int(fi);
     T a = u - fi;

@@ -596,7 +596,7 @@ int nfft_plan_create(nfft_plan** out, int precision, int D, const int64_t* N, in
   const int64_t ninv = p->N[0] + (D > 1 ? p->N[1] : 0) + (D > 2 ? p->N[2] : 0) + 1;
   const int deg = 2 * p->m + 1, L = 2 * p->m;
   if (cudaMalloc(&p->inv, rs * ninv) != cudaSuccess || cudaMalloc(&p->coeffs, rs * deg * L) != cudaSuccess ||
-      cudaMalloc(&p->dflag, 2 * sizeof(int)) != cudaSuccess || cudaMemset(p->dflag, 0, 2 * sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&p->dflag, 4 * sizeof(int)) != cudaSuccess || cudaMemset(p->dflag, 0, 4 * sizeof(int)) != cudaSuccess) {
     set_error("cudaMalloc of plan tables failed");
     return fail(NFFT_ERR_ALLOC);
   }
@@ -724,17 +724,35 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     NFFT_CUDA_TRY(cudaMemcpyAsync(p->k, k, rs * size_t(D * M),
                                   k_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   }
-  // checkNodes
-  int flag = 0;
+  // (the node check runs with the reduction below: its verdict and the task
+  // count are read back together, the only wait of this call)
   NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag, 0, sizeof(int), s));
-  int rc = launch_check_nodes(p, p->k, p->dflag);
-  if (rc) return rc;
-  NFFT_CUDA_TRY(cudaMemcpyAsync(&flag, p->dflag, sizeof(int), cudaMemcpyDeviceToHost, s));
-  NFFT_CUDA_TRY(cudaStreamSynchronize(s));
-  if (flag) {
-    free_nodes(p);
-    set_error("Nodes k need to be within the range [-1/2, 1/2)");
-    return NFFT_ERR_NODE_OUT_OF_RANGE;
+  NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag + 2, 0, sizeof(int), s));
+  int rc = NFFT_OK;
+  int chunk = 0;
+  if (p->prm.blocking) {
+    // hot tiles are split into chunks of at most `chunk` nodes (each chunk is
+    // one spreading task and flushes its padded tile once);
+    // NFFT_GB300_TASK_CHUNK overrides the default.  D = 2 tasks run on one
+    // warp each (warp2.cuh), ~60 cycles a node, so 1024 nodes of a hot tile
+    // take 30 us on their own, longer than a whole small transform; large
+    // sets fill the GPU anyway and prefer fewer flushes.  Forward + adjoint of
+    // a radial 128^2 image, us with 64 / 128 / 256 / 512 nodes per task:
+    // 4,000 nodes 42 / 44 / 44 / 44, 20,000 nodes 42 / 48 / 58 / 79, 200,000
+    // nodes 58 / 63 / 67 / 85, 800,000 nodes 115 / 116 / 121 / 143; 64 slices of
+    // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
+    // D = 1: 2048, so that tiles of about 1024 nodes are not cut into a task
+    // of 1024 and one of a few (line1.cuh takes a task in equal batches).
+    chunk = D == 1 ? 2048 : 1024;
+    if (D == 2 && !p->prm.compensated) {
+      const int64_t work = M * p->task_columns;
+      chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
+    }
+    if (const char* e = getenv("NFFT_GB300_TASK_CHUNK")) {
+      const int c = atoi(e);
+      if (c >= 32 && c <= (1 << 20)) chunk = c;
+    }
+    p->task_chunk = chunk;
   }
   const int64_t nt = p->ntiles_total;
   const int kbits = bits_for(nt);
@@ -754,13 +772,13 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
       return NFFT_ERR_ALLOC;
     }
     NFFT_CUDA_TRY(cudaMemsetAsync(tcount, 0, sizeof(int32_t) * size_t(nt + 1), s));
-    rc = launch_reduce_nodes(p, p->k, ti_u, te_u, key, val, tcount);
+    rc = launch_reduce_nodes(p, p->k, ti_u, te_u, key, val, tcount, p->dflag);
+    if (rc) return rc;
+    rc = launch_tile_lists(p, tcount, chunk, scr, sb, p->dflag + 2);
     if (rc) return rc;
     uint32_t* ko = nullptr;
     int32_t* vo = nullptr;
     rc = radix_sort_pairs(key, val, key2, val2, M, kbits, scr, sb, s, &ko, &vo);
-    if (rc) return rc;
-    rc = exclusive_scan_i32(tcount, p->tile_start, nt + 1, scr, sb, s);
     if (rc) return rc;
     rc = launch_build_node_tables(p, vo, ti_u, te_u);
     if (rc) return rc;
@@ -773,36 +791,21 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
                      sizeof(int4) * size_t(M) + rs * 4 * size_t(M) + (table ? rs * size_t(M * D * L) : 0) +
                      sizeof(int32_t) * size_t(nt + 1);
   if (p->prm.blocking) {
-    // hot tiles are split into chunks of at most `chunk` nodes (each chunk is
-    // one spreading task and flushes its padded tile once);
-    // NFFT_GB300_TASK_CHUNK overrides the default.  D = 2 tasks run on one
-    // warp each (warp2.cuh), ~60 cycles a node, so 1024 nodes of a hot tile
-    // take 30 us on their own, longer than a whole small transform; large
-    // sets fill the GPU anyway and prefer fewer flushes.  Forward + adjoint of
-    // a radial 128^2 image, us with 64 / 128 / 256 / 512 nodes per task:
-    // 4,000 nodes 42 / 44 / 44 / 44, 20,000 nodes 42 / 48 / 58 / 79, 200,000
-    // nodes 58 / 63 / 67 / 85, 800,000 nodes 115 / 116 / 121 / 143; 64 slices of
-    // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
-    // D = 1: 2048, so that tiles of about 1024 nodes are not cut into a task
-    // of 1024 and one of a few (line1.cuh takes a task in equal batches).
-    int chunk = D == 1 ? 2048 : 1024;
-    if (D == 2 && !p->prm.compensated) {
-      const int64_t work = M * p->task_columns;
-      chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
-    }
-    if (const char* e = getenv("NFFT_GB300_TASK_CHUNK")) {
-      const int c = atoi(e);
-      if (c >= 32 && c <= (1 << 20)) chunk = c;
-    }
-    p->task_chunk = chunk;
-    rc = launch_build_tasks(p, chunk);
-    if (rc) return rc;
     p->fsorted = node_buffer(p, P::NB_FSORTED, 2 * rs * size_t(M));
     if (!p->fsorted) return NFFT_ERR_ALLOC;
-    p->scratch_bytes += sizeof(int4) * size_t(p->n_tasks) + 2 * rs * size_t(M);
+    p->scratch_bytes += 2 * rs * size_t(M);
   }
+  int words[3] = {0, 0, 0};
+  NFFT_CUDA_TRY(cudaMemcpyAsync(words, p->dflag, sizeof(words), cudaMemcpyDeviceToHost, s));
   NFFT_CUDA_TRY(cudaStreamSynchronize(s));
   NFFT_CUDA_TRY(cudaGetLastError());
+  if (words[0]) {
+    free_nodes(p);
+    set_error("Nodes k need to be within the range [-1/2, 1/2)");
+    return NFFT_ERR_NODE_OUT_OF_RANGE;
+  }
+  p->n_tasks = words[2];
+  p->scratch_bytes += sizeof(int4) * size_t(p->n_tasks);
   p->has_nodes = true;
   p->nodes_version += 1;
   p->timing[0] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -23,7 +23,7 @@ template <typename T>
 __global__ void reduce_nodes_kernel(const T* __restrict__ k, int D, int64_t M, int Nt0, int Nt1, int Nt2, int bs0,
                                     int bs1, int bs2, int nt0, int nt1, int32_t* __restrict__ ti,
                                     T* __restrict__ te, uint32_t* __restrict__ key, int32_t* __restrict__ val,
-                                    int32_t* __restrict__ tile_count) {
+                                    int32_t* __restrict__ tile_count, int* __restrict__ flag) {
   int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= M) return;
   const int Nt[3] = {Nt0, Nt1, Nt2};
@@ -32,7 +32,10 @@ __global__ void reduce_nodes_kernel(const T* __restrict__ k, int D, int64_t M, i
   for (int d = 0; d < D; ++d) {
     int32_t t;
     T e;
-    reduce_coord<T>(k[int64_t(d) + int64_t(D) * j], Nt[d], t, e);
+    const T x = k[int64_t(d) + int64_t(D) * j];
+    // checkNodes, as in check_nodes_kernel; reduce_coord clamps what it rejects
+    if (flag && !(fabs(x) <= T(0.5))) atomicOr(flag, 1);
+    reduce_coord<T>(x, Nt[d], t, e);
     ti[int64_t(d) * M + j] = t;
     te[int64_t(d) * M + j] = e;
     b[d] = t / bs[d];
@@ -162,13 +165,73 @@ __global__ void task_counts_kernel(const int32_t* __restrict__ tstart, int64_t n
 }
 
 __global__ void fill_tasks_kernel(const int32_t* __restrict__ tstart, const int32_t* __restrict__ toff,
-                                  int64_t ntiles, int chunk, TileOrder order, int4* __restrict__ tasks) {
+                                  int64_t ntiles, int chunk, TileOrder order, int4* __restrict__ tasks,
+                                  int* __restrict__ ntasks) {
   int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= ntiles) return;
+  if (q == 0) *ntasks = toff[ntiles];
   const int t = order.tile(q);
   const int s = tstart[t], e = tstart[t + 1];
   int pos = toff[q];
   for (int b = s; b < e; b += chunk) tasks[pos++] = make_int4(t, b, min(e, b + chunk), 0);
+}
+
+// Small grids: the CSR of the tiles and the task list by one CTA, in place of
+// three launches with their scans.  Each thread takes `cpt` consecutive tiles,
+// then `cpt` consecutive places of the task order.
+constexpr int kListThreads = 1024;
+constexpr int kListTiles = 8 * kListThreads;  // largest tile count
+
+// Exclusive scan of one value per thread over the CTA; *total gets the sum.
+__device__ __forceinline__ int cta_exclusive_scan(int v, int* s_warp, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();  // (s_warp of an earlier scan has been read)
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int w = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+      if (lane >= o) w += y;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  *total = s_warp[31];
+  return x - v + (warp > 0 ? s_warp[warp - 1] : 0);
+}
+
+__global__ void __launch_bounds__(kListThreads) tile_lists_kernel(const int32_t* __restrict__ tcount, int ntiles,
+                                                                  int chunk, TileOrder order, int32_t* tstart,
+                                                                  int4* __restrict__ tasks, int* __restrict__ ntasks) {
+  static_assert(kListThreads == 32 * 32, "one warp sum per lane");
+  __shared__ int s_warp[32];
+  const int cpt = (ntiles + kListThreads - 1) / kListThreads;
+  const int q0 = int(threadIdx.x) * cpt, q1 = min(q0 + cpt, ntiles);
+  int sum = 0, total;
+  for (int t = q0; t < q1; ++t) sum += tcount[t];
+  int at = cta_exclusive_scan(sum, s_warp, &total);
+  for (int t = q0; t < q1; ++t) {
+    tstart[t] = at;
+    at += tcount[t];
+  }
+  if (threadIdx.x == 0) tstart[ntiles] = total;
+  if (chunk == 0) return;  // no task list (plain path)
+  sum = 0;
+  for (int q = q0; q < q1; ++q) sum += (tcount[order.tile(q)] + chunk - 1) / chunk;
+  at = cta_exclusive_scan(sum, s_warp, &total);  // (its barriers also publish tstart to the CTA)
+  for (int q = q0; q < q1; ++q) {
+    const int t = order.tile(q), b0 = tstart[t], e = b0 + tcount[t];
+    for (int b = b0; b < e; b += chunk) tasks[at++] = make_int4(t, b, min(e, b + chunk), 0);
+  }
+  if (threadIdx.x == 0) *ntasks = total;
 }
 
 }  // namespace
@@ -197,20 +260,20 @@ int launch_check_node_values(int precision, const void* k, int64_t n, int* flag,
 
 template <typename T>
 static int reduce_t(const nfft_plan* p, const void* k, int32_t* ti_u, void* te_u, uint32_t* key, int32_t* val,
-                    int32_t* tile_count) {
+                    int32_t* tile_count, int* flag) {
   if (p->M == 0) return NFFT_OK;
   reduce_nodes_kernel<T><<<unsigned((p->M + 255) / 256), 256, 0, p->stream>>>(
       static_cast<const T*>(k), p->D, p->M, int(p->Nt[0]), int(p->Nt[1]), int(p->Nt[2]), int(p->bs[0]),
       int(p->bs[1]), int(p->bs[2]), int(p->ntiles[0]), int(p->ntiles[1]), ti_u, static_cast<T*>(te_u), key, val,
-      tile_count);
+      tile_count, flag);
   NFFT_LAUNCH_CHECK();
   return NFFT_OK;
 }
 
 int launch_reduce_nodes(const nfft_plan* p, const void* k, int32_t* ti_u, void* te_u, uint32_t* key,
-                        int32_t* val, int32_t* tile_count) {
-  return p->precision == 32 ? reduce_t<float>(p, k, ti_u, te_u, key, val, tile_count)
-                            : reduce_t<double>(p, k, ti_u, te_u, key, val, tile_count);
+                        int32_t* val, int32_t* tile_count, int* flag) {
+  return p->precision == 32 ? reduce_t<float>(p, k, ti_u, te_u, key, val, tile_count, flag)
+                            : reduce_t<double>(p, k, ti_u, te_u, key, val, tile_count, flag);
 }
 
 template <typename T>
@@ -255,32 +318,37 @@ int launch_deconv_factors(nfft_plan* p) {
   return NFFT_OK;
 }
 
-// Chunk the non-empty home tiles (CSR p->tile_start) into spreading tasks of
-// at most `chunk` nodes.  Allocates p->tasks.
-int launch_build_tasks(nfft_plan* p, int chunk) {
+// The CSR of the nodes per tile from their counts, and (chunk > 0) the
+// spreading tasks of at most `chunk` nodes of the non-empty tiles, in the
+// order above.  Allocates p->tasks for the most tasks these nodes can make;
+// the number made goes to `ntasks` (device): nothing waits for it here.
+int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks) {
   const int64_t nt = p->ntiles_total;
-  const size_t sb = scan_scratch_bytes(nt + 1);
+  const TileOrder order{int(p->ntiles[0]), int(p->ntiles[1]), int(p->ntiles[2])};
+  if (chunk > 0) {
+    const int64_t most = std::min(nt, p->M) + p->M / chunk;
+    p->tasks = static_cast<int4*>(node_buffer(p, nfft_plan::NB_TASKS, sizeof(int4) * size_t(most)));
+    if (!p->tasks) return NFFT_ERR_ALLOC;
+  }
+  if (nt <= kListTiles) {
+    tile_lists_kernel<<<1, kListThreads, 0, p->stream>>>(tcount, int(nt), chunk, order, p->tile_start, p->tasks,
+                                                         ntasks);
+    NFFT_LAUNCH_CHECK();
+    return NFFT_OK;
+  }
+  int rc = exclusive_scan_i32(tcount, p->tile_start, nt + 1, scr, scr_bytes, p->stream);
+  if (rc || chunk == 0) return rc;
   auto* tcnt = static_cast<int32_t*>(node_buffer(p, nfft_plan::NB_TCNT, sizeof(int32_t) * (nt + 1)));
   auto* toff = static_cast<int32_t*>(node_buffer(p, nfft_plan::NB_TOFF, sizeof(int32_t) * (nt + 1)));
-  void* scr = node_buffer(p, nfft_plan::NB_SCR, std::max(sb, p->nbuf_cap[nfft_plan::NB_SCR]));
-  if (!tcnt || !toff || !scr) return NFFT_ERR_ALLOC;
-  const TileOrder order{int(p->ntiles[0]), int(p->ntiles[1]), int(p->ntiles[2])};
+  if (!tcnt || !toff) return NFFT_ERR_ALLOC;
   task_counts_kernel<<<unsigned((nt + 255) / 256), 256, 0, p->stream>>>(p->tile_start, nt, chunk, order, tcnt);
   NFFT_LAUNCH_CHECK();
   NFFT_CUDA_TRY(cudaMemsetAsync(tcnt + nt, 0, sizeof(int32_t), p->stream));
-  int rc = exclusive_scan_i32(tcnt, toff, nt + 1, scr, p->nbuf_cap[nfft_plan::NB_SCR], p->stream);
+  rc = exclusive_scan_i32(tcnt, toff, nt + 1, scr, scr_bytes, p->stream);
   if (rc) return rc;
-  int32_t ntasks = 0;
-  NFFT_CUDA_TRY(cudaMemcpyAsync(&ntasks, toff + nt, sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream));
-  NFFT_CUDA_TRY(cudaStreamSynchronize(p->stream));  // the task count sizes the launches
-  p->n_tasks = ntasks;
-  p->tasks = static_cast<int4*>(node_buffer(p, nfft_plan::NB_TASKS, sizeof(int4) * size_t(ntasks)));
-  if (!p->tasks) return NFFT_ERR_ALLOC;
-  if (ntasks > 0) {
-    fill_tasks_kernel<<<unsigned((nt + 255) / 256), 256, 0, p->stream>>>(p->tile_start, toff, nt, chunk, order,
-                                                                          p->tasks);
-    NFFT_LAUNCH_CHECK();
-  }
+  fill_tasks_kernel<<<unsigned((nt + 255) / 256), 256, 0, p->stream>>>(p->tile_start, toff, nt, chunk, order,
+                                                                        p->tasks, ntasks);
+  NFFT_LAUNCH_CHECK();
   return NFFT_OK;
 }
 
