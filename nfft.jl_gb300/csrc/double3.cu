@@ -1,0 +1,75 @@
+// Launches of the 3-D FP64 gather and spreader (double3.cuh).
+#include "double3.cuh"
+
+namespace nfft {
+namespace {
+
+template <int L, bool TABLE> int gather_launch(const nfft_plan* p, const double2* g, double2* fhat) {
+  const int pitch = gather3d_pitch(int(p->bs[0]) + L - 1);
+  const size_t smem = Gather3D<L>::stage_bytes() +
+                      sizeof(double2) * size_t(pitch) * size_t(p->bs[1] + L - 1) * size_t(p->bs[2] + L - 1);
+  if (smem > 227 * 1024) return -1;
+  auto kern = gather_double3_kernel<L, TABLE>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<unsigned(p->n_tasks), kD3GatherThreads, smem, p->stream>>>(make_geom<double>(p), make_nodes<double>(p),
+                                                                    p->tasks, g, fhat, pitch);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
+template <int L, bool TABLE> int spread_launch(const nfft_plan* p, const double2* fhat, double* g) {
+  const int64_t rows = (p->bs[1] + L - 1) * (p->bs[2] + L - 1);
+  const int64_t limit = (int64_t(227) * 1024 - int64_t(Spread3D<L>::STAGE)) / (16 * rows);
+  const int P0 = int(p->bs[0]) + L - 1;
+  if (P0 > limit) return -1;
+  const int pitch = warp2_pitch(p->m, P0, 16, limit);
+  const size_t smem = Spread3D<L>::STAGE + 16 * size_t(pitch) * size_t(rows);
+  auto kern = spread_double3_kernel<L, TABLE>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<unsigned(p->n_tasks), Spread3D<L>::THREADS, smem, p->stream>>>(make_geom<double>(p), make_nodes<double>(p),
+                                                                       p->tasks, fhat, g, pitch);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
+}  // namespace
+
+#define NFFT_D3_DISPATCH(CALL)                                                  \
+  switch (p->m) {                                                               \
+    case 2: return p->wtab ? CALL<4, true> NFFT_D3_ARGS : CALL<4, false> NFFT_D3_ARGS;    \
+    case 3: return p->wtab ? CALL<6, true> NFFT_D3_ARGS : CALL<6, false> NFFT_D3_ARGS;    \
+    NFFT_D3_CASE8(CALL)                                                         \
+    case 5: return p->wtab ? CALL<10, true> NFFT_D3_ARGS : CALL<10, false> NFFT_D3_ARGS;  \
+    case 6: return p->wtab ? CALL<12, true> NFFT_D3_ARGS : CALL<12, false> NFFT_D3_ARGS;  \
+    case 7: return p->wtab ? CALL<14, true> NFFT_D3_ARGS : CALL<14, false> NFFT_D3_ARGS;  \
+    case 8: return p->wtab ? CALL<16, true> NFFT_D3_ARGS : CALL<16, false> NFFT_D3_ARGS;  \
+  }                                                                             \
+  return -1
+
+// -1: not applicable (no task list, a tile that does not fit, or too few
+// nodes per task, or in all, to pay for bringing their tile into shared
+// memory.  Forward transform, us tiled / direct, m = 5: 4096 tasks, 20,000 nodes
+// 486 / 332, 100,000 797 / 1014, 262,144 1.31 / 1.99 ms in the gather; 225 tasks, 20,000
+// nodes 248 / 225, 100,000 785 / 903.  m = 3: 4096 tasks, 20,000 nodes 278 / 232, 100,000
+// 332 / 468; 225 tasks, 4000 nodes 83 / 82, 100,000 262 / 359).
+int launch_gather_double3(const nfft_plan* p, const void* g, void* fhat) {
+  if (!p->tasks || p->n_tasks == 0 || p->M < 16 * p->n_tasks || p->M < 65536) return -1;
+#define NFFT_D3_ARGS (p, static_cast<const double2*>(g), static_cast<double2*>(fhat))
+#define NFFT_D3_CASE8(CALL) case 4: return p->wtab ? CALL<8, true> NFFT_D3_ARGS : CALL<8, false> NFFT_D3_ARGS;
+  NFFT_D3_DISPATCH(gather_launch);
+#undef NFFT_D3_CASE8
+#undef NFFT_D3_ARGS
+}
+
+// Spreading into a zeroed grid (values in the caller's order); -1: m = 4
+// (spread_owned_kernel is as good there), or the tile and its staging do not
+// fit in shared memory.
+int launch_spread_double3(const nfft_plan* p, const void* fhat, void* g) {
+#define NFFT_D3_ARGS (p, static_cast<const double2*>(fhat), static_cast<double*>(g))
+#define NFFT_D3_CASE8(CALL)
+  NFFT_D3_DISPATCH(spread_launch);
+#undef NFFT_D3_CASE8
+#undef NFFT_D3_ARGS
+}
+
+}  // namespace nfft

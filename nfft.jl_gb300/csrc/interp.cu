@@ -508,6 +508,10 @@ int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int6
       NFFT_LAUNCH_CHECK();
       return NFFT_OK;
     }
+    if constexpr (D == 3 && sizeof(T) == 8) {
+      const int rc = launch_gather_double3(p, g, fhat);
+      if (rc != -1) return rc;
+    }
     if constexpr (D == 3 && sizeof(T) == 4) {
       const int rc = L == 8 ? interp_tile3(p, G, Nd, gp, fp) : launch_gather_plane3(p, g, fhat);
       if (rc != -1) return rc;

@@ -231,6 +231,9 @@ int launch_real_to_complex(const nfft_plan* p, const void* in, void* out, int64_
 int launch_real_part(const nfft_plan* p, const void* in, void* out, int64_t n);
 // gather3.cu: -1 = not applicable
 int launch_gather_plane3(const nfft_plan* p, const void* g, void* fhat);
+// double3.cu: -1 = not applicable
+int launch_gather_double3(const nfft_plan* p, const void* g, void* fhat);
+int launch_spread_double3(const nfft_plan* p, const void* fhat, void* g);
 // spread3.cu: -1 = not applicable
 int launch_spread_plane3(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fcol, int64_t gcol_t);
 // spread.cu: the plan's buffer of zeros that clears spreading tiles (null: not available)

@@ -22,6 +22,10 @@ template <> __device__ __forceinline__ void red_add2<double>(double* g, double x
   atomicAdd(g + 1, y);
 }
 
+// v != 0 (FP64 by its bits: a comparison would take the FP64 units).
+__device__ __forceinline__ bool is_nonzero(float v) { return v != 0.f; }
+__device__ __forceinline__ bool is_nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+
 // Accumulator element: (re, im) or, compensated, (re, im, comp re, comp im).
 template <typename T, bool KAHAN> struct Acc;
 template <> struct Acc<float, false> { using type = float2; };
@@ -91,7 +95,7 @@ __device__ __forceinline__ void flush_tile(const Geom<T>& G, const typename Acc<
       }
       T vr, vi;
       acc_value<T, typename Acc<T, KAHAN>::type, KAHAN>(srow[j], vr, vi);
-      if (vr != T(0) || vi != T(0)) {
+      if (is_nonzero(vr) || is_nonzero(vi)) {
         const int gx = small ? wrap_any(x0 + j, Nt0) : wrap_once(x0 + j, Nt0);
         red_add2<T>(grow + 2 * gx, vr, vi);
       }
