@@ -1,6 +1,7 @@
 // 3-D FP32 gather from padded tiles in shared memory for any window width
-// L = 2m = 4 .. 12 and the tile shapes fixed at compile time (tile3.cuh); L = 8
-// has its own kernel (interp_tile3_kernel, interp.cu).
+// L = 2m = 4 .. 12 and the tile shapes fixed at compile time (tile3.cuh); for
+// L = 8, grids whose tiles rarely wrap have their own kernel
+// (interp_tile3_kernel, interp.cu).
 //
 // One CTA per task.  A tile inside the grid comes in by one bulk tensor copy, one
 // that wraps around it by asynchronous 8-byte copies with the periodic
@@ -250,18 +251,23 @@ template <int L> int gather3_shape(nfft_plan* p, const float2* g, float2* fhat) 
 }  // namespace
 
 // -1: the plan's tiles or window have no compiled kernel, or too few nodes per
-// task to pay for bringing their tile into shared memory (L = 10: 60 KB a
-// tile, 8 KB of taps a node; below six nodes per task the direct gather moves
-// less).
+// task to pay for bringing their tile (L = 10: 60 KB) into shared memory.
+// Forward transform, us tiled / direct: m = 5, 2048 tasks: 20,000 nodes 71 / 48, 40,000
+// 75 / 67, 100,000 92 / 134; 9,300 tasks: 100,000 nodes 265 / 239, 600,000 385 / 635; 360
+// tasks (one or two CTAs per SM): 20,000 nodes 65 / 61, 40,000 74 / 81.  m = 3, 2048
+// tasks: 40,000 nodes 55 / 43, 100,000 63 / 67; 360 tasks: 40,000 57 / 54, 100,000 71 / 79.
+// m = 4, 2048 tasks: 100,000 uniform / radial nodes 71, 83 / 72, 300,000 102, 113 / 138,
+// 10^6 212, 213 / 382; 360 tasks: 100,000 76, 100 / 85, 300,000 130, 126 / 149.
 int launch_gather_plane3(const nfft_plan* cp, const void* g, void* fhat) {
   nfft_plan* p = const_cast<nfft_plan*>(cp);  // the tensor-map cache only
   if (!p->gather_tma || !p->tasks || p->n_tasks == 0 || p->D != 3 || p->precision != 32 || p->bs[2] != 8) return -1;
-  if (p->M < 6 * p->n_tasks) return -1;
+  if (p->m >= 5 ? p->M < 32 * p->n_tasks || p->M < 32768 : p->M < 64 * p->n_tasks || p->M < 131072) return -1;
   const float2* gp = static_cast<const float2*>(g);
   float2* f = static_cast<float2*>(fhat);
   switch (p->m) {
     case 2: return gather3_shape<4>(p, gp, f);
     case 3: return gather3_shape<6>(p, gp, f);
+    case 4: return gather3_shape<8>(p, gp, f);
     case 5: return gather3_shape<10>(p, gp, f);
     case 6: return gather3_shape<12>(p, gp, f);
   }

@@ -391,6 +391,22 @@ int interp_tile3_launch(const nfft_plan* p, const CUtensorMap* map, const Geom<f
   return NFFT_OK;
 }
 
+// Whether the kernel above is the right one for an m = 4 plan.  It moves tiles
+// inside the grid only (nodes of wrapping tiles gather from L1, on one CTA per
+// task), so it wants few nodes in wrapping tiles (counted by nodes!), fewer
+// still where gather3.cu has many nodes per task to pay for its own tiles; with
+// under 24 nodes per task the direct gather moves less.  Forward, us, here /
+// gather3.cu / direct: 128^3, 10^6 uniform nodes, 23 % in wrapping tiles 351 / 371 /
+// 477; 64^3, 43 %: 100,000 nodes 64 / 71 / 72, 10^6 351 / 212 / 382; 240 x 216 x 180 grid
+// (not centred), 10^6 radial nodes 495 / 331 / 495; 256^3 grid, 8192 tasks, 100,000
+// nodes 175 / - / 156, 300,000 207 / - / 220.
+bool tile3_pays(const nfft_plan* p) {
+  if (p->M < 24 * p->n_tasks) return false;
+  if (p->bs[1] != 8 || p->bs[0] > 16) return true;  // tile shapes that gather3.cu does not have
+  const int64_t w = p->wrap_nodes;
+  return 4 * w <= p->M || (2 * w <= p->M && p->M < 96 * p->n_tasks);
+}
+
 // The TMA-tiled 3-D gather when the plan has one of the fixed tile shapes and
 // the grid's tensor map can be made; -1 = not applicable.
 int interp_tile3(const nfft_plan* cp, const Geom<float>& G, const Nodes<float>& Nd, const float2* g, float2* fhat) {
@@ -513,7 +529,7 @@ int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int6
       if (rc != -1) return rc;
     }
     if constexpr (D == 3 && sizeof(T) == 4) {
-      const int rc = L == 8 ? interp_tile3(p, G, Nd, gp, fp) : launch_gather_plane3(p, g, fhat);
+      const int rc = L == 8 && tile3_pays(p) ? interp_tile3(p, G, Nd, gp, fp) : launch_gather_plane3(p, g, fhat);
       if (rc != -1) return rc;
     }
     if (p->tasks && p->gather_tiled) {

@@ -143,6 +143,7 @@ struct nfft_plan {
   // spreading tasks: (home tile, first node, end node, 0), hot tiles split
   int64_t n_tasks = 0;
   int4* tasks = nullptr;
+  int64_t wrap_nodes = 0;          // 3-D FP32 m = 4: nodes in tiles whose padded box wraps around the (centred) grid
   int task_chunk = 1024;           // most nodes of a task
   int64_t task_columns = 1;        // columns that every launch over the tasks covers (directional plans)
   int spread_pitch = 0;            // shared-memory row pitch of the padded spreading tile
@@ -182,7 +183,7 @@ struct nfft_plan {
          NB_KEY2, NB_VAL2, NB_TCOUNT, NB_SCR, NB_TCNT, NB_TOFF, NB_COUNT };
   void* nbuf[NB_COUNT] = {};
   size_t nbuf_cap[NB_COUNT] = {};
-  int* dflag = nullptr;            // device words: [0] node check, [1] an async copy wait that timed out, [2] task count
+  int* dflag = nullptr;            // device words: [0] node check, [1] an async copy wait that timed out, [2] task count, [3] wrap_nodes
   size_t scratch_bytes = 0;
 
   // TimingStats: every forward/adjoint records 4 events into a ring slot; the
@@ -212,6 +213,7 @@ int launch_build_node_tables(const nfft_plan* p, const int32_t* perm, const int3
 int launch_build_weight_table(const nfft_plan* p);
 int launch_deconv_factors(nfft_plan* p);
 int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks);
+int launch_wrap_nodes(const nfft_plan* p, const int32_t* tcount, int* out);
 // autotune.cu
 int apply_block_size(nfft_plan* p, const int64_t* bs, const void* k, int ny);
 // spread.cu: bank-conflict-free row pitch of a padded spreading tile

@@ -727,7 +727,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
   // (the node check runs with the reduction below: its verdict and the task
   // count are read back together, the only wait of this call)
   NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag, 0, sizeof(int), s));
-  NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag + 2, 0, sizeof(int), s));
+  NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag + 2, 0, 2 * sizeof(int), s));
   int rc = NFFT_OK;
   int chunk = 0;
   if (p->prm.blocking) {
@@ -743,7 +743,16 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
     // D = 1: 2048, so that tiles of about 1024 nodes are not cut into a task
     // of 1024 and one of a few (line1.cuh takes a task in equal batches).
+    // D = 3: as for D = 2, hot tiles of small sets are cut short (radial nodes,
+    // whole transform, us with 128 / 256 / 1024: adjoint, m = 5, 64^3, 100,000 nodes
+    // 117 / 128 / 255; adjoint, m = 4, 300,000 nodes 143 / 145 / 199; uniform, 34 x 32
+    // x 17, 300,000 nodes forward 133 / 117 / 129; FP64 forward 100,000 nodes 471 / 533 /
+    // 841).
     chunk = D == 1 ? 2048 : 1024;
+    if (D == 3 && !p->prm.compensated && M >= 4096) {
+      if (M < (int64_t(1) << 19)) chunk = M < (int64_t(1) << 17) || p->precision == 64 ? 128 : 256;
+      else if (M < (int64_t(1) << 20)) chunk = 512;
+    }
     if (D == 2 && !p->prm.compensated) {
       const int64_t work = M * p->task_columns;
       chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
@@ -776,6 +785,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     if (rc) return rc;
     rc = launch_tile_lists(p, tcount, chunk, scr, sb, p->dflag + 2);
     if (rc) return rc;
+    if (D == 3 && p->m == 4 && p->precision == 32 && (rc = launch_wrap_nodes(p, tcount, p->dflag + 3))) return rc;
     uint32_t* ko = nullptr;
     int32_t* vo = nullptr;
     rc = radix_sort_pairs(key, val, key2, val2, M, kbits, scr, sb, s, &ko, &vo);
@@ -795,7 +805,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     if (!p->fsorted) return NFFT_ERR_ALLOC;
     p->scratch_bytes += 2 * rs * size_t(M);
   }
-  int words[3] = {0, 0, 0};
+  int words[4] = {0, 0, 0, 0};
   NFFT_CUDA_TRY(cudaMemcpyAsync(words, p->dflag, sizeof(words), cudaMemcpyDeviceToHost, s));
   NFFT_CUDA_TRY(cudaStreamSynchronize(s));
   NFFT_CUDA_TRY(cudaGetLastError());
@@ -805,6 +815,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     return NFFT_ERR_NODE_OUT_OF_RANGE;
   }
   p->n_tasks = words[2];
+  p->wrap_nodes = words[3];
   p->scratch_bytes += sizeof(int4) * size_t(p->n_tasks);
   p->has_nodes = true;
   p->nodes_version += 1;

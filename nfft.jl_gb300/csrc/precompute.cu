@@ -234,7 +234,42 @@ __global__ void __launch_bounds__(kListThreads) tile_lists_kernel(const int32_t*
   if (threadIdx.x == 0) *ntasks = total;
 }
 
+// Nodes in tiles whose box padded by `pad` points on each side wraps around the grid.
+struct WrapGeom {
+  int n[3], bs[3], Nt[3], sh[3], pad;
+};
+__global__ void __launch_bounds__(256) wrap_nodes_kernel(const int32_t* __restrict__ tcount, int64_t ntiles,
+                                                         WrapGeom W, int* __restrict__ out) {
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  int c = 0;
+  if (t < ntiles) {
+    const int q[3] = {int(t % W.n[0]), int((t / W.n[0]) % W.n[1]), int(t / (int64_t(W.n[0]) * W.n[1]))};
+    bool wraps = false;
+    for (int d = 0; d < 3; ++d) {
+      const int o = wrap_once(q[d] * W.bs[d] + W.sh[d], W.Nt[d]);
+      wraps = wraps || o - W.pad < 0 || o + W.bs[d] + W.pad > W.Nt[d];
+    }
+    if (wraps) c = tcount[t];
+  }
+  c = __reduce_add_sync(0xFFFFFFFFu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
+}
+
 }  // namespace
+
+int launch_wrap_nodes(const nfft_plan* p, const int32_t* tcount, int* out) {
+  WrapGeom W{};
+  for (int d = 0; d < 3; ++d) {
+    W.n[d] = int(p->ntiles[d]);
+    W.bs[d] = int(p->bs[d]);
+    W.Nt[d] = int(p->Nt[d]);
+    W.sh[d] = int(p->sh[d]);
+  }
+  W.pad = p->m;
+  wrap_nodes_kernel<<<unsigned((p->ntiles_total + 255) / 256), 256, 0, p->stream>>>(tcount, p->ntiles_total, W, out);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
 
 template <typename T> static int check_nodes_t(const nfft_plan* p, const void* k, int* flag) {
   const int64_t n = p->M * p->D;
