@@ -12,6 +12,9 @@
 //                  (n + Ntilde - N/2) mod Ntilde, times prod 1/phi-hat; for
 //                  pre > 1 a shared-memory transposition (pre <-> image index)
 //   FFT            cuFFT along dims, batched over the contiguous grid columns
+//                  (pre = 1, 2-D with power-of-two grids: the pruned line FFTs
+//                  of fft.cu with pad, crop and factors inside; 64 slices of
+//                  256^2: pad + cuFFT 217 -> 77 us, cuFFT + crop 131 -> 75 us)
 //   gather         the core plan's tiled gather, all columns per launch, into
 //                  node values in column order, transposed to (pre, node, post)
 //   spread         node values transposed to column order, then the core
@@ -51,6 +54,7 @@ struct nfft_dplan {
   // tiled: grid columns contiguous (column c = a + pre b), the core plan's
   // tiled gather / atomic-free spreader run over all columns
   bool tiled = false;
+  bool fused = false;              // the pruned line FFTs instead of pad / crop and cuFFT
   int64_t ncols = 1;               // pre x post
   void* sorted = nullptr;          // tiled: bin-sorted node values of a launch's columns (M x <= 65535 complex)
   void* vals = nullptr;            // tiled, pre > 1: node values in column order (M x ncols complex)
@@ -432,6 +436,10 @@ template <typename T> int dforward(nfft_dplan* q, const void* f, void* fhat) {
   using C = typename Cplx<T>::type;
   DGeom<T> G = make_dgeom<T>(q);
   int rc = NFFT_OK;
+  if (q->fused) {
+    if ((rc = fused_cols(q->core, q->grid, const_cast<void*>(f), q->ncols, true))) return rc;
+    return dgather_cols<T>(q, fhat);
+  }
   if (q->tiled && q->pre > 1) {  // transposing pad into zeroed grid columns
     NFFT_CUDA_TRY(cudaMemsetAsync(q->grid, 0, 2 * sizeof(T) * size_t(q->ncols * q->Rnt), q->stream));
     if ((rc = dtranspose<T, true, true>(q, G, f, q->grid, q->Rn, q->Rnt))) return rc;
@@ -461,6 +469,7 @@ template <typename T> int dadjoint(nfft_dplan* q, const void* fhat, void* f) {
     rc = dconv<T>(q, fhat, q->grid, true);
   }
   if (rc) return rc;
+  if (q->fused) return fused_cols(q->core, q->grid, f, q->ncols, false);
   if ((rc = dexec_fft(q, CUFFT_INVERSE))) return rc;
   if (q->tiled && q->pre > 1) return dtranspose<T, false, true>(q, G, q->grid, f, q->Rn, q->Rnt);
   dcrop_kernel<T><<<blocks_for(q->pre * q->Rn * q->post), 256, 0, q->stream>>>(G, static_cast<const C*>(q->grid),
@@ -559,6 +568,12 @@ extern "C" int nfft_dplan_create(nfft_dplan** out, int precision, int D, const i
       return NFFT_ERR_ALLOC;
     }
   }
+  q->fused = q->tiled && q->pre == 1 && q->R == 2 && q->core->fused_fft &&
+             q->core->N[1] * q->ncols < (int64_t(1) << 31);
+  if (q->fused) {
+    *out = q;
+    return NFFT_OK;
+  }
   // cuFFT along the transform dims (C order: reversed), columns batched
   int n[3];
   for (int d = 0; d < q->R; ++d) n[d] = int(q->Nt[dim_hi - d]);
@@ -615,7 +630,7 @@ extern "C" int nfft_dplan_set_nodes(nfft_dplan* q, const void* k, int k_on_devic
 extern "C" int nfft_dplan_set_stream(nfft_dplan* q, void* stream) {
   if (!q) return NFFT_ERR_INVALID_ARG;
   q->stream = static_cast<cudaStream_t>(stream);
-  if (cufftSetStream(q->fft, q->stream) != CUFFT_SUCCESS) {
+  if (q->fft_ok && cufftSetStream(q->fft, q->stream) != CUFFT_SUCCESS) {
     set_error("cufftSetStream failed");
     return NFFT_ERR_CUFFT;
   }

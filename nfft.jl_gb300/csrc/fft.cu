@@ -219,6 +219,7 @@ template <typename T, int N, bool FWD> constexpr int fft_min_blocks() {
 struct FftGeom {
   int N[3], Nt[3];
   int64_t plane;  // Nt0 * Nt1
+  int zs, zinv;   // grid z of image z = (z - zs) mod Ntilde[2]; its factor is inv.d[2][z * zinv] (columns: 0, 0)
 };
 
 template <typename T> struct Inv3 {
@@ -247,9 +248,9 @@ __global__ void __launch_bounds__(NT, NT < kFftThreads ? 1 : fft_min_blocks<T, N
     int64_t go = 0;
     if (r < rows) {
       const int y = int(r % G.N[1]), z = int(r / G.N[1]);
-      s = __ldg(inv.d[1] + y) * __ldg(inv.d[2] + z);
+      s = __ldg(inv.d[1] + y) * __ldg(inv.d[2] + z * G.zinv);
       go = int64_t(NX) * (wrap_once(y - G.N[1] / 2, G.Nt[1]) +
-                          int64_t(G.Nt[1]) * wrap_once(z - G.N[2] / 2, G.Nt[2]));
+                          int64_t(G.Nt[1]) * wrap_once(z - G.zs, G.Nt[2]));
     }
     s_row[threadIdx.x] = s;
     s_goff[threadIdx.x] = go;
@@ -315,9 +316,9 @@ __global__ void __launch_bounds__(NT, NT < kFftThreads ? 1 : fft_min_blocks<T, N
     int64_t go = 0;
     if (r < rows) {
       const int y = int(r % G.N[1]), z = int(r / G.N[1]);
-      s = __ldg(inv.d[1] + y) * __ldg(inv.d[2] + z);
+      s = __ldg(inv.d[1] + y) * __ldg(inv.d[2] + z * G.zinv);
       go = int64_t(NX) * (wrap_once(y - G.N[1] / 2, G.Nt[1]) +
-                          int64_t(G.Nt[1]) * wrap_once(z - G.N[2] / 2, G.Nt[2]));
+                          int64_t(G.Nt[1]) * wrap_once(z - G.zs, G.Nt[2]));
     }
     s_row[threadIdx.x] = s;
     s_goff[threadIdx.x] = go;
@@ -766,9 +767,9 @@ __global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : (FWD ? 3 : 2)) fft4_x_ke
     int64_t goff = 0;
     if (r < rows) {
       const int yy = int(r % G.N[1]), zz = int(r / G.N[1]);
-      sc = __ldg(inv.d[1] + yy) * __ldg(inv.d[2] + zz);
+      sc = __ldg(inv.d[1] + yy) * __ldg(inv.d[2] + zz * G.zinv);
       goff = int64_t(NX) * (wrap_once(yy - G.N[1] / 2, G.Nt[1]) +
-                            int64_t(G.Nt[1]) * wrap_once(zz - G.N[2] / 2, G.Nt[2]));
+                            int64_t(G.Nt[1]) * wrap_once(zz - G.zs, G.Nt[2]));
     }
     s_row[threadIdx.x] = sc;
     s_goff[threadIdx.x] = goff;
@@ -950,6 +951,12 @@ FftGeom make_fft_geom(const nfft_plan* p) {
     G.Nt[d] = int(p->Nt[d]);
   }
   G.plane = p->Nt[0] * p->Nt[1];
+  G.zs = G.N[2] / 2;
+  G.zinv = 1;
+  if (p->fft_cols > 1) {  // 2-D transforms of contiguous columns: the column is the third index
+    G.N[2] = G.Nt[2] = int(p->fft_cols);
+    G.zs = G.zinv = 0;
+  }
   return G;
 }
 
@@ -970,7 +977,7 @@ template <typename K> int set_smem(K kern, size_t bytes) {
 
 template <typename T, int NX, int W> int x_pass_w(nfft_plan* p, const void* src, void* dst, bool fwd, void* const* slot) {
   using C = Cx<T>;
-  const unsigned blocks = unsigned((p->N[1] * p->N[2] + W - 1) / W);
+  const unsigned blocks = unsigned((p->N[1] * p->N[2] * p->fft_cols + W - 1) / W);
   if constexpr (sizeof(T) == 4 && NX <= 512 && NFFT_FFT_FOURSTEP) {
     const size_t smem = size_t(W) * Split4<NX>::R2 * (Split4<NX>::R1 + 1) * sizeof(float2);
     const float2* tw = static_cast<const float2*>(p->fft_tw[0]);
@@ -1004,7 +1011,7 @@ bool few_ctas(const nfft_plan* p, int64_t lines, int W) { return 2 * lines <= in
 
 template <typename T, int NX> int x_pass_t(nfft_plan* p, const void* src, void* dst, bool fwd, void* const* slot) {
   static_assert(kW4 == lines_per_cta<float>(), "lines per CTA");
-  if (few_ctas(p, p->N[1] * p->N[2], lines_per_cta<T>()))
+  if (few_ctas(p, p->N[1] * p->N[2] * p->fft_cols, lines_per_cta<T>()))
     return x_pass_w<T, NX, small_x_lines<T>()>(p, src, dst, fwd, slot);
   return x_pass_w<T, NX, lines_per_cta<T>()>(p, src, dst, fwd, slot);
 }
@@ -1019,7 +1026,7 @@ LineGeom make_line_geom(const nfft_plan* p, int axis, int W, int64_t* outer_coun
     L.outer_stride = p->Nt[0] * p->Nt[1];
     L.outer_N = p->D == 3 ? int(p->N[2]) : 0;
     L.outer_Nt = int(p->Nt[2]);
-    *outer_count = p->D == 3 ? p->N[2] : 1;
+    *outer_count = p->D == 3 ? p->N[2] : p->fft_cols;
   } else {          // z lines of every (x, y)
     L.stride = p->Nt[0] * p->Nt[1];
     L.outer_stride = p->Nt[0];
@@ -1274,6 +1281,30 @@ int fused_adjoint_lines(nfft_plan* p) {
 int fused_adjoint_x(nfft_plan* p, void* f, void* const* f_slot) {
   return p->precision == 32 ? x_pass<float>(p, p->grid, f, false, f_slot)
                             : x_pass<double>(p, p->grid, f, false, f_slot);
+}
+
+// The 2-D transforms of ncols contiguous images (forward: f -> grid columns;
+// adjoint: grid columns -> f), the plan's factors and lengths, in the same
+// launches as one image's.
+int fused_cols(nfft_plan* p, void* grid, void* f, int64_t ncols, bool fwd) {
+  struct Scope {
+    nfft_plan* p;
+    void* own;
+    Scope(nfft_plan* q, void* g, int64_t n) : p(q), own(q->grid) {
+      p->grid = g;
+      p->fft_cols = n;
+    }
+    ~Scope() {
+      p->grid = own;
+      p->fft_cols = 1;
+    }
+  } scope(p, grid, ncols);
+  if (fwd) {
+    const int rc = fused_forward_x(p, f);
+    return rc ? rc : fused_forward_lines(p);
+  }
+  const int rc = fused_adjoint_lines(p);
+  return rc ? rc : fused_adjoint_x(p, f);
 }
 
 // Toeplitz convolution y <- crop(IFFT(lambda . FFT(pad(y)))) on a

@@ -111,6 +111,7 @@ struct nfft_plan {
   // fused pruned FFT (fft.cu): used instead of pad + cuFFT / cuFFT + crop on
   // the transform path when every Ntilde_d is a power of two in [64, 1024]
   bool fused_fft = false;
+  int64_t fft_cols = 1;       // 2-D: contiguous images per fused transform (directional plans)
   void* fft_tw[3] = {};       // per dimension: exp(-2 pi i q / Ntilde_d), q < Ntilde_d (T complex)
   size_t real_size = 4;
 
@@ -258,6 +259,7 @@ int fused_forward_x(nfft_plan* p, const void* f, void* const* f_slot = nullptr);
 int fused_forward_lines(nfft_plan* p);
 int fused_adjoint_lines(nfft_plan* p);
 int fused_adjoint_x(nfft_plan* p, void* f, void* const* f_slot = nullptr);
+int fused_cols(nfft_plan* p, void* grid, void* f, int64_t ncols, bool fwd);
 // y <- crop(IFFT(scale * lambda . FFT(pad(y)))) on a transform-only plan (N image, Ntilde = 2N)
 int fused_toeplitz(nfft_plan* p, const void* lam, double scale, void* y);
 // gradk.cu

@@ -66,3 +66,23 @@ def test_warp2_columns(m):
     for c in range(C):
         assert oracle.rel_l2(y[:, c].cpu().numpy(), (one * f[:, :, c]).cpu().numpy()) < 1e-5
         assert oracle.rel_l2(x[:, :, c].cpu().numpy(), (nf.adjoint(one) * v[:, c].contiguous()).cpu().numpy()) < 1e-5
+
+
+@pytest.mark.parametrize("N,C", [((32, 32), 3), ((64, 128), 7), ((256, 64), 65), ((512, 32), 2)])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_fused_columns(monkeypatch, N, C, dtype):
+    """Directional plans with power-of-two grids run the pruned line FFTs over
+    all columns; each column equals the cuFFT path's."""
+    k, rng = nodes(N, 900, dtype)
+    cd = torch.complex64 if dtype == np.float32 else torch.complex128
+    f = nf.as_colmajor(rng.standard_normal(N + (C,)) + 1j * rng.standard_normal(N + (C,)), N + (C,), cd)
+    v = nf.as_colmajor(rng.standard_normal((900, C)) + 1j * rng.standard_normal((900, C)), (900, C), cd)
+    p = nf.plan_nfft(k, N + (C,), dims=(1, 2), m=4, sigma=2.0)
+    y, x = (p * f).cpu().numpy(), (nf.adjoint(p) * v).cpu().numpy()
+    monkeypatch.setenv("NFFT_GB300_FFT", "cufft")
+    q = nf.plan_nfft(k, N + (C,), dims=(1, 2), m=4, sigma=2.0)
+    ref_y, ref_x = (q * f).cpu().numpy(), (nf.adjoint(q) * v).cpu().numpy()
+    tol = 1e-5 if dtype == np.float32 else 1e-11
+    for c in range(C):
+        assert oracle.rel_l2(y[:, c], ref_y[:, c]) < tol
+        assert oracle.rel_l2(x[:, :, c], ref_x[:, :, c]) < tol
