@@ -175,6 +175,16 @@ int nfft_convolve(nfft_plan* plan, const void* g, int g_real, void* fhat, int fh
  * src/convolution.jl:115-149).  Complex fHat with real g is rejected. */
 int nfft_convolve_transpose(nfft_plan* plan, const void* fhat, int fhat_real, void* g, int g_real);
 
+/* The iterations of NFFTTools' sdc! (NFFTTools/src/samplingDensity.jl:59-137):
+ * `iters` times g = real(convolve_transpose!(w)) / s, t = real(convolve!(g)) / s,
+ * w = w ./ t, with s the maximum of the first iteration's g.  weights (length
+ * M, real, device) is updated in place; weights_tmp (length M) and workg (size
+ * Ntilde, real) receive the last t and g when not NULL.  *non_positive is set to
+ * 1 if some t was <= 0 (the reference asserts that none is).  Waits for the
+ * result; the plan's grid (tmpVec) is overwritten. */
+int nfft_sdc_weights(nfft_plan* plan, int iters, void* weights, void* weights_tmp, void* workg,
+                     int32_t* non_positive);
+
 /* deconvolve!(p, f, g) (src/deconvolution.jl:2-45): writes the whole
  * oversampled grid g (zeros outside the image). */
 int nfft_deconvolve(nfft_plan* plan, const void* f, void* g);

@@ -23,7 +23,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 SOURCES = ["plan.cu", "precompute.cu", "sort.cu", "deconv.cu", "interp.cu", "gather3.cu", "spread.cu", "spread3.cu", "double3.cu", "gradk.cu", "batch.cu",
            "directional.cu", "fft.cu", "plain.cu", "noalloc.cu", "autotune.cu", "toeplitz.cu", "direct.cu", "trig.cu", "nnfft.cu",
-           "sortnodes.cu"]
+           "sortnodes.cu", "sdc.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -140,6 +140,7 @@ struct nfft_plan {
   void* wtab = nullptr;       // M * D * 2m (T), sorted window tensor (not for POLYNOMIAL)
   int32_t* tile_start = nullptr;   // ntiles_total + 1: CSR of nodes per home tile
   void* cbuf = nullptr;       // M complex scratch for real-valued convolve calls (lazy)
+  void* sdc = nullptr;        // scale and status of nfft_sdc_weights (lazy)
   void* fsorted = nullptr;    // M complex: fHat in bin-sorted order (spreading input)
   // spreading tasks: (home tile, first node, end node, 0), hot tiles split
   int64_t n_tasks = 0;
@@ -269,6 +270,8 @@ int launch_plain_interp(const nfft_plan* p, const void* g, int g_real, void* fha
 int launch_plain_spread(const nfft_plan* p, const void* fhat, int fhat_real, void* g, int g_real);
 
 template <typename T> Geom<T> make_geom(const nfft_plan* p);
+// plan.cu: allocates p->cbuf
+int ensure_cbuf(nfft_plan* p);
 // plan.cu: node buffer `which` of at least `bytes` (grown, contents not kept)
 void* node_buffer(nfft_plan* p, int which, size_t bytes);
 // plan.cu: recompute sh and inv_c after the tiles or the factors changed

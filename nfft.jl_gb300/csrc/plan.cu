@@ -436,6 +436,15 @@ void finish_record(nfft_plan* p, int slot, int dir) {
 
 int exec_fft_plan(nfft_plan* p, int dir) { return exec_fft(p, dir); }
 
+int ensure_cbuf(nfft_plan* p) {
+  if (p->cbuf) return NFFT_OK;
+  if (cudaMalloc(&p->cbuf, 2 * p->real_size * size_t(p->M > 0 ? p->M : 1)) != cudaSuccess) {
+    set_error("cudaMalloc of the node scratch failed");
+    return NFFT_ERR_ALLOC;
+  }
+  return NFFT_OK;
+}
+
 }  // namespace nfft
 
 using namespace nfft;
@@ -677,6 +686,7 @@ int nfft_plan_destroy(nfft_plan* p) {
   cudaFree(p->lut);
   cudaFree(p->dflag);
   cudaFree(p->cbuf);
+  cudaFree(p->sdc);
   if (p->fft_ok) cufftDestroy(p->fft);
   if (p->fft_tail_ok) cufftDestroy(p->fft_tail);
   if (p->fft_line_ok) cufftDestroy(p->fft_line);
@@ -960,15 +970,6 @@ int nfft_adjoint(nfft_plan* p, const void* fhat, void* f) {
   if (rc) return rc;
   record(p, slot, 3);
   finish_record(p, slot, 1);
-  return NFFT_OK;
-}
-
-static int ensure_cbuf(nfft_plan* p) {
-  if (p->cbuf) return NFFT_OK;
-  if (cudaMalloc(&p->cbuf, 2 * p->real_size * size_t(p->M > 0 ? p->M : 1)) != cudaSuccess) {
-    set_error("cudaMalloc of the node scratch failed");
-    return NFFT_ERR_ALLOC;
-  }
   return NFFT_OK;
 }
 

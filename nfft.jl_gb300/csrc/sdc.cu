@@ -1,0 +1,159 @@
+// The iterations of NFFTTools' sampling density compensation
+// (NFFTTools/src/samplingDensity.jl:59-137) in one call:
+//
+//   g   <- real(spread(w)) / s        s = max(g) of the first iteration
+//   t   <- real(gather(g)) / s
+//   w_j <- w_j / t_j
+//
+// The real convolutions of the plan go through complex arrays, which took a
+// conversion pass on each side of both directions, each a call of its own
+// beside the element-wise steps and a host test of t per iteration.  Here the
+// weights stay complex between the steps, the conversions, divisions, the
+// update and the test of t are parts of two kernels, and the test is read once
+// at the end.  Per iteration: zero-fill, spread, scale, gather, update.  32 x
+// 2048 spiral on a 256^2 image, 20 iterations: 2.78 -> 0.92 ms with the same
+// convolution kernels.
+#include "nfft_internal.cuh"
+
+#include <algorithm>
+
+namespace nfft {
+namespace {
+
+constexpr int kSdcBlocks = 1024;  // partial maxima
+
+template <typename T> struct SdcState {
+  T partial[kSdcBlocks];
+  T scale;
+  int bad;  // some t_j <= 0
+};
+
+template <typename T> __device__ __forceinline__ T max_nan(T a, T b) {
+  return (b > a || b != b) && !(a != a) ? b : a;  // NaN wins, as in Julia's and torch's maximum
+}
+
+template <typename T> __device__ T cta_max(T v) {
+  __shared__ T s[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max_nan(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+  if (lane == 0) s[warp] = v;
+  __syncthreads();
+  v = s[lane < int(blockDim.x >> 5) ? lane : 0];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max_nan(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+  return v;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sdc_begin_kernel(const T* __restrict__ w, typename Cplx<T>::type* __restrict__ c,
+                                                        int64_t M, SdcState<T>* st) {
+  const int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (j == 0) st->bad = 0;
+  if (j < M) c[j] = {w[j], T(0)};
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sdc_max_kernel(const typename Cplx<T>::type* __restrict__ g, int64_t n,
+                                                      SdcState<T>* st) {
+  int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  T v = g[i < n ? i : n - 1].x;
+  for (i += int64_t(gridDim.x) * blockDim.x; i < n; i += int64_t(gridDim.x) * blockDim.x) v = max_nan(v, g[i].x);
+  v = cta_max(v);
+  if (threadIdx.x == 0) st->partial[blockIdx.x] = v;
+}
+
+template <typename T> __global__ void __launch_bounds__(kSdcBlocks) sdc_scale_kernel(SdcState<T>* st, int n) {
+  const T v = cta_max(st->partial[int(threadIdx.x) < n ? threadIdx.x : 0]);
+  if (threadIdx.x == 0) st->scale = v;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sdc_grid_kernel(typename Cplx<T>::type* __restrict__ g, int64_t n,
+                                                       const SdcState<T>* __restrict__ st, T* __restrict__ real_out) {
+  const T s = st->scale;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const T v = g[i].x / s;
+    g[i] = {v, T(0)};
+    if (real_out) real_out[i] = v;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) sdc_update_kernel(typename Cplx<T>::type* __restrict__ c, T* __restrict__ w,
+                                                         T* __restrict__ tmp, int64_t M, SdcState<T>* st) {
+  const int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (j >= M) return;
+  const T t = c[j].x / st->scale;
+  if (t <= T(0)) atomicOr(&st->bad, 1);
+  const T v = w[j] / t;
+  if (tmp) tmp[j] = t;
+  w[j] = v;
+  c[j] = {v, T(0)};
+}
+
+template <typename T>
+int sdc_run(nfft_plan* p, int iters, T* w, T* tmp, T* workg, int32_t* non_positive) {
+  using C = typename Cplx<T>::type;
+  const int64_t M = p->M, n = p->Nt[0] * p->Nt[1] * p->Nt[2];
+  if (!p->sdc && cudaMalloc(&p->sdc, sizeof(SdcState<T>)) != cudaSuccess) {
+    p->sdc = nullptr;
+    set_error("cudaMalloc of the density compensation state failed");
+    return NFFT_ERR_ALLOC;
+  }
+  auto* st = static_cast<SdcState<T>*>(p->sdc);
+  C* c = static_cast<C*>(p->cbuf);
+  C* g = static_cast<C*>(p->grid);
+  cudaStream_t s = p->stream;
+  const unsigned nb = unsigned((M + 255) / 256);
+  const unsigned gb = unsigned(std::min<int64_t>((n + 255) / 256, kSdcBlocks));
+  const unsigned gg = unsigned(std::min<int64_t>((n + 255) / 256, int64_t(p->sms) * 32));
+  sdc_begin_kernel<T><<<nb, 256, 0, s>>>(w, c, M, st);
+  NFFT_LAUNCH_CHECK();
+  for (int i = 0; i < iters; ++i) {
+    int rc = p->prm.blocking ? launch_spread(p, c, 0, g, 0) : launch_plain_spread(p, c, 0, g, 0);
+    if (rc) return rc;
+    if (i == 0) {
+      sdc_max_kernel<T><<<gb, 256, 0, s>>>(g, n, st);
+      NFFT_LAUNCH_CHECK();
+      sdc_scale_kernel<T><<<1, kSdcBlocks, 0, s>>>(st, int(gb));
+      NFFT_LAUNCH_CHECK();
+    }
+    sdc_grid_kernel<T><<<gg, 256, 0, s>>>(g, n, st, i + 1 == iters ? workg : nullptr);
+    NFFT_LAUNCH_CHECK();
+    rc = p->prm.blocking ? launch_interp(p, g, 0, c, 0) : launch_plain_interp(p, g, 0, c, 0);
+    if (rc) return rc;
+    sdc_update_kernel<T><<<nb, 256, 0, s>>>(c, w, tmp, M, st);
+    NFFT_LAUNCH_CHECK();
+  }
+  int bad = 0;
+  NFFT_CUDA_TRY(cudaMemcpyAsync(&bad, &st->bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+  NFFT_CUDA_TRY(cudaStreamSynchronize(s));
+  *non_positive = bad;
+  return NFFT_OK;
+}
+
+}  // namespace
+}  // namespace nfft
+
+using namespace nfft;
+
+extern "C" int nfft_sdc_weights(nfft_plan* p, int iters, void* weights, void* weights_tmp, void* workg,
+                                int32_t* non_positive) {
+  if (!p || !non_positive || iters < 0 || (!weights && p->M > 0)) {
+    set_error("null argument");
+    return NFFT_ERR_INVALID_ARG;
+  }
+  *non_positive = 0;
+  if (!p->has_nodes) {
+    set_error("plan has no nodes: call nfft_set_nodes first");
+    return NFFT_ERR_NO_NODES;
+  }
+  if (p->M == 0 || iters == 0) return NFFT_OK;
+  if (int rc = ensure_cbuf(p)) return rc;
+  return p->precision == 32
+             ? sdc_run<float>(p, iters, static_cast<float*>(weights), static_cast<float*>(weights_tmp),
+                              static_cast<float*>(workg), non_positive)
+             : sdc_run<double>(p, iters, static_cast<double*>(weights), static_cast<double*>(weights_tmp),
+                               static_cast<double*>(workg), non_positive);
+}

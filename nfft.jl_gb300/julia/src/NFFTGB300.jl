@@ -221,6 +221,19 @@ function AbstractNFFTs.convolve_transpose!(p::GB300NFFTPlan{T,D}, fHat::CuVector
   return g
 end
 
+# The iterations of NFFTTools' sdc! (NFFTTools/src/samplingDensity.jl:59-137) in
+# one library call: weights is updated in place.
+function sdc_weights!(p::GB300NFFTPlan{T,D}, weights::CuArray{T,1}; iters::Integer = 20) where {T,D}
+  size(weights) == (p.J,) || throw(DimensionMismatch("size(weights)=$(size(weights)) ≠ J = $(p.J)"))
+  bind_stream!(p)
+  bad = Ref{Int32}(0)
+  check(ccall((:nfft_sdc_weights, libnfft[]), Cint,
+              (Ptr{Cvoid}, Cint, CuPtr{T}, CuPtr{T}, CuPtr{T}, Ref{Int32}),
+              p.handle, iters, weights, CU_NULL, CU_NULL, bad))
+  bad[] == 0 || throw(AssertionError("non-positive weights"))
+  return weights
+end
+
 function AbstractNFFTs.deconvolve!(p::GB300NFFTPlan{T,D}, f::CuArray{Complex{T},D}, g::CuArray{Complex{T},D}) where {T,D}
   bind_stream!(p)
   check(ccall((:nfft_deconvolve, libnfft[]), Cint, (Ptr{Cvoid}, CuPtr{Complex{T}}, CuPtr{Complex{T}}),

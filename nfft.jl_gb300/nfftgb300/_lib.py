@@ -77,6 +77,7 @@ SIGNATURES = {
     "nfft_adjoint": (_I, [_P, _P, _P]),
     "nfft_convolve": (_I, [_P, _P, _I, _P, _I]),
     "nfft_convolve_transpose": (_I, [_P, _P, _I, _P, _I]),
+    "nfft_sdc_weights": (_I, [_P, _I, _P, _P, _P, _I32P]),
     "nfft_deconvolve": (_I, [_P, _P, _P]),
     "nfft_deconvolve_transpose": (_I, [_P, _P, _P]),
     "nfft_grad_nodes": (_I, [_P, _P, _P, _P]),

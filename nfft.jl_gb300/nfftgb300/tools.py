@@ -1,9 +1,10 @@
 """NFFTTools clients on the GPU plan.
 
 ``sdc`` restates NFFTTools' sampling density compensation
-(NFFTTools/src/samplingDensity.jl:59-155) on top of the plan's real-valued
-``convolve!`` / ``convolve_transpose!`` and ``mul!``, the way NFFTTools uses the
-reference's GPU plan (test/gpu.jl:52-65).
+(NFFTTools/src/samplingDensity.jl:59-155): its iterations of real-valued
+``convolve!`` / ``convolve_transpose!`` run in one library call
+(``nfft_sdc_weights``), the final scaling on the plan's ``mul!``, the way
+NFFTTools uses the reference's GPU plan (test/gpu.jl:52-65).
 
 The Toeplitz tools (NFFTTools/src/Toeplitz.jl) mirror
 ``calculateToeplitzKernel``, ``calculateToeplitzKernel!``,
@@ -25,30 +26,30 @@ from . import plan as P
 def sdc(p, iters=20, weights=None, weights_tmp=None, workg=None, workf=None, workv=None):
     """Density compensation weights (real, length J) with the final scaling
     c = real(sum(v)) / ||v||^2 of sdc! (:138-155).  The work buffers may be
-    passed in to avoid allocation, as in the reference."""
+    passed in, as in the reference; weights_tmp and workg are not needed and only
+    filled when given."""
     T = p.dtype
     dev = p.device
     if weights is None:
         weights = torch.ones(p.J, dtype=T, device=dev)
-    if weights_tmp is None:
-        weights_tmp = torch.empty_like(weights)
-    if workg is None:
-        workg = P.empty_image(p.Ñ, T, dev)
     if workf is None:
         workf = torch.empty(p.J, dtype=p.cdtype, device=dev)
     if workv is None:
         workv = P.empty_image(p.N, p.cdtype, dev)
-    scaling = None
-    for i in range(iters):
-        p.convolve_transpose_(weights, workg)
-        if i == 0:
-            scaling = workg.max()
-        workg.div_(scaling)
-        p.convolve_(workg, weights_tmp)
-        weights_tmp.div_(scaling)
-        if bool((weights_tmp <= 0).any()):
-            raise ValueError("non-positive weights")
-        weights.div_(weights_tmp)
+    for x, shape in ((weights, (p.J,)), (weights_tmp, (p.J,)), (workg, p.Ñ)):
+        if x is None:
+            continue
+        if tuple(x.shape) != tuple(shape):
+            raise P.DimensionMismatch(f"work array of size {tuple(x.shape)}, expected {tuple(shape)}")
+        if x.dtype != T or x.device != dev or not P._is_colmajor(x):
+            raise P.ArgumentError(f"sdc needs column-major {T} arrays on {dev}")
+    bad = ctypes.c_int32(0)
+    p._sync_stream()
+    P._check(L.load().nfft_sdc_weights(p._handle, int(iters), P._ptr(weights),
+                                       None if weights_tmp is None else P._ptr(weights_tmp),
+                                       None if workg is None else P._ptr(workg), ctypes.byref(bad)))
+    if bad.value:
+        raise ValueError("non-positive weights")
     u = workv
     u.fill_(1)
     p.forward_(workf, u)
