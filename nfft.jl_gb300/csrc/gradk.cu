@@ -68,6 +68,14 @@ __device__ __forceinline__ void tap_weight_deriv(const Geom<T>& G, const T* cs, 
   }
 }
 
+}  // namespace
+}  // namespace nfft
+
+#include "gradwarp2.cuh"
+
+namespace nfft {
+namespace {
+
 template <int L, int D, typename T> __device__ __forceinline__ T wsel(T W0, T W1, int q) {
   if (D * L <= 32) return shfl(W0, q & 31);
   T a = shfl(W0, q & 31);
@@ -169,11 +177,41 @@ __global__ void __launch_bounds__(kGradThreads) grad_nodes_kernel(Geom<T> G, Nod
   }
 }
 
+// D = 2 by tiles (gradwarp2.cuh); -1: no task list, tile too large, or too few
+// nodes per task to pay for bringing their tile into shared memory (the rule
+// of the gather, interp.cu).
+template <int L, typename T, bool POLY>
+int grad_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* g,
+                      const typename Cplx<T>::type* w, T* dk) {
+  if (!p->tasks || p->n_tasks == 0) return -1;
+  const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
+  if (p->M * 256 < p->n_tasks * int64_t(P0) * P1) return -1;
+  const int64_t limit = (int64_t(227) * 1024 - int64_t(GradWarp2<L, T>::STAGE)) / (int64_t(2 * sizeof(T)) * P1);
+  if (P0 > limit) return -1;
+  const int pitch = warp2_pitch(p->m, P0, 2 * sizeof(T), limit);
+  const size_t smem = GradWarp2<L, T>::STAGE + 2 * sizeof(T) * size_t(pitch) * P1;
+  WinPoly<L, T, !POLY> wp{};
+  if constexpr (POLY)
+    for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  auto kern = grad_warp2_kernel<L, T, POLY>;
+  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kern<<<unsigned(p->n_tasks), 32, smem, p->stream>>>(G, Nd, p->tasks, g, w, dk, pitch, wp);
+  NFFT_LAUNCH_CHECK();
+  return NFFT_OK;
+}
+
 template <int D, int L, typename T> int grad_c(const nfft_plan* p, const void* g, const void* w, void* dk) {
   Geom<T> G = make_geom<T>(p);
   Nodes<T> Nd = make_nodes<T>(p);
   if (Nd.M == 0) return NFFT_OK;
   using C = typename Cplx<T>::type;
+  if constexpr (D == 2) {
+    const C* gp = static_cast<const C*>(g);
+    const C* w2 = static_cast<const C*>(w);
+    const int rc = G.mode == WIN_POLY ? grad_warp2_launch<L, T, true>(p, G, Nd, gp, w2, static_cast<T*>(dk))
+                                      : grad_warp2_launch<L, T, false>(p, G, Nd, gp, w2, static_cast<T*>(dk));
+    if (rc != -1) return rc;
+  }
   int64_t blocks = (Nd.M + 7) / 8;
   if (blocks > 152 * 64) blocks = 152 * 64;
   grad_nodes_kernel<D, L, T><<<unsigned(blocks), kGradThreads, 0, p->stream>>>(

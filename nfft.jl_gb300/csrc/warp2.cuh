@@ -289,6 +289,54 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
   flush_tile<2, T, false, 1>(G, acc, g, o0, o1, 0, P0, P1, 1, pitch);
 }
 
+// The task's padded tile by asynchronous copies with the periodic wrap (not committed).
+template <int L, typename T>
+__device__ __forceinline__ void warp2_load_tile(const Geom<T>& G, const typename Cplx<T>::type* __restrict__ g,
+                                                typename Cplx<T>::type* tile, int pitch, int o0, int o1, int P0, int P1,
+                                                int lane) {
+  using C = typename Cplx<T>::type;
+  const int x0 = o0 + G.sh[0] - (L / 2 - 1), y0 = o1 + G.sh[1] - (L / 2 - 1);
+  for (int x = lane; x < P0; x += 32) {
+    const int gx = wrap_any(x0 + x, G.Nt[0]);
+    int gy = wrap_any(y0, G.Nt[1]);
+    for (int y = 0; y < P1; ++y) {
+      const C* src = g + int64_t(gy) * G.Nt[0] + gx;
+      if constexpr (sizeof(C) == 8) cp_async8(tile + y * pitch + x, src);
+      else cp_async16(tile + y * pitch + x, src);
+      gy = gy + 1 == G.Nt[1] ? 0 : gy + 1;
+    }
+  }
+}
+
+// Sums two values of eight nodes over the warp together (transposed
+// butterfly, 18 shuffles): lane l ends with node l / 4's sums in a[0], b[0].
+template <typename T> __device__ __forceinline__ void warp2_reduce8(T (&a)[8], T (&b)[8], int lane) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const T sa = h16 ? a[k] : a[k + 4], sb = h16 ? b[k] : b[k + 4];
+    a[k] = (h16 ? a[k + 4] : a[k]) + __shfl_xor_sync(FULL, sa, 16);
+    b[k] = (h16 ? b[k + 4] : b[k]) + __shfl_xor_sync(FULL, sb, 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const T sa = h8 ? a[k] : a[k + 2], sb = h8 ? b[k] : b[k + 2];
+    a[k] = (h8 ? a[k + 2] : a[k]) + __shfl_xor_sync(FULL, sa, 8);
+    b[k] = (h8 ? b[k + 2] : b[k]) + __shfl_xor_sync(FULL, sb, 8);
+  }
+  {
+    const T sa = h4 ? a[0] : a[1], sb = h4 ? b[0] : b[1];
+    a[0] = (h4 ? a[1] : a[0]) + __shfl_xor_sync(FULL, sa, 4);
+    b[0] = (h4 ? b[1] : b[0]) + __shfl_xor_sync(FULL, sb, 4);
+  }
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) {
+    a[0] += __shfl_xor_sync(FULL, a[0], o);
+    b[0] += __shfl_xor_sync(FULL, b[0], o);
+  }
+}
+
 // Gathers one task's nodes from its padded tile, brought into shared memory by
 // asynchronous copies with the periodic wrap.  smem: GATHER_STAGE bytes, then
 // pitch x (bs[1] + L - 1) grid values.
@@ -300,7 +348,6 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
   using W = Warp2<L, T, TABLE>;
   using C = typename Cplx<T>::type;
   using St = Warp2Stage<L, T, TABLE>;
-  constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int NK = 8;  // nodes reduced together
   typename W::Rec* rec = reinterpret_cast<typename W::Rec*>(smem);
   T* win = reinterpret_cast<T*>(smem + W::REC_BYTES);
@@ -309,22 +356,9 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
   const int tc0 = task.x % G.ntiles[0], tc1 = task.x / G.ntiles[0];
   const int P0 = G.bs[0] + L - 1, P1 = G.bs[1] + L - 1;
   const int o0 = tc0 * G.bs[0], o1 = tc1 * G.bs[1];
-  const int m1 = G.m - 1;
   if (task.y >= task.z) return;
-  {
-    const int x0 = o0 + G.sh[0] - m1, y0 = o1 + G.sh[1] - m1;
-    for (int x = lane; x < P0; x += 32) {
-      const int gx = wrap_any(x0 + x, G.Nt[0]);
-      int gy = wrap_any(y0, G.Nt[1]);
-      for (int y = 0; y < P1; ++y) {
-        const C* src = g + int64_t(gy) * G.Nt[0] + gx;
-        if constexpr (sizeof(C) == 8) cp_async8(tile + y * pitch + x, src);
-        else cp_async16(tile + y * pitch + x, src);
-        gy = gy + 1 == G.Nt[1] ? 0 : gy + 1;
-      }
-    }
-    cp_async_commit();
-  }
+  warp2_load_tile<L, T>(G, g, tile, pitch, o0, o1, P0, P1, lane);
+  cp_async_commit();
   St st;
   St::copy_rows(Nd, win, task.y, task.z, 0, lane);
   st.load(Nd, task.y, task.z, lane);
@@ -376,29 +410,7 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
         ar[k] = sr;
         ai[k] = si;
       }
-      // transposed butterfly: lane l ends with node l / 4 summed over all lanes
-      const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const T sa = h16 ? ar[k] : ar[k + 4], sb = h16 ? ai[k] : ai[k + 4];
-        ar[k] = (h16 ? ar[k + 4] : ar[k]) + __shfl_xor_sync(FULL, sa, 16);
-        ai[k] = (h16 ? ai[k + 4] : ai[k]) + __shfl_xor_sync(FULL, sb, 16);
-      }
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const T sa = h8 ? ar[k] : ar[k + 2], sb = h8 ? ai[k] : ai[k + 2];
-        ar[k] = (h8 ? ar[k + 2] : ar[k]) + __shfl_xor_sync(FULL, sa, 8);
-        ai[k] = (h8 ? ai[k + 2] : ai[k]) + __shfl_xor_sync(FULL, sb, 8);
-      }
-      {
-        const T sa = h4 ? ar[0] : ar[1], sb = h4 ? ai[0] : ai[1];
-        ar[0] = (h4 ? ar[1] : ar[0]) + __shfl_xor_sync(FULL, sa, 4);
-        ai[0] = (h4 ? ai[1] : ai[0]) + __shfl_xor_sync(FULL, sb, 4);
-      }
-      ar[0] += __shfl_xor_sync(FULL, ar[0], 2);
-      ai[0] += __shfl_xor_sync(FULL, ai[0], 2);
-      ar[0] += __shfl_xor_sync(FULL, ar[0], 1);
-      ai[0] += __shfl_xor_sync(FULL, ai[0], 1);
+      warp2_reduce8(ar, ai, lane);
       const int s = s0 + (lane >> 2);
       if ((lane & 3) == 0 && s < n) {
         C r;
