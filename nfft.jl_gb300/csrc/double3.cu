@@ -22,7 +22,7 @@ template <int L, bool TABLE> int spread_launch(const nfft_plan* p, const double2
   const int64_t limit = (int64_t(227) * 1024 - int64_t(Spread3D<L>::STAGE)) / (16 * rows);
   const int P0 = int(p->bs[0]) + L - 1;
   if (P0 > limit) return -1;
-  const int pitch = warp2_pitch(p->m, P0, 16, limit);
+  const int pitch = warp2_pitch(2 * p->m, 8, P0, limit);
   const size_t smem = Spread3D<L>::STAGE + 16 * size_t(pitch) * size_t(rows);
   auto kern = spread_double3_kernel<L, TABLE>;
   NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));

@@ -188,7 +188,7 @@ int grad_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, 
   if (p->M * 256 < p->n_tasks * int64_t(P0) * P1) return -1;
   const int64_t limit = (int64_t(227) * 1024 - int64_t(GradWarp2<L, T>::STAGE)) / (int64_t(2 * sizeof(T)) * P1);
   if (P0 > limit) return -1;
-  const int pitch = warp2_pitch(p->m, P0, 2 * sizeof(T), limit);
+  const int pitch = warp2_pitch(L, 128 / int(2 * sizeof(T)), P0, limit);
   const size_t smem = GradWarp2<L, T>::STAGE + 2 * sizeof(T) * size_t(pitch) * P1;
   WinPoly<L, T, !POLY> wp{};
   if constexpr (POLY)

@@ -2,12 +2,15 @@
 // of a hot one), shared by the single-plan and multi-column launches
 // (spread.cu, interp.cu) and the batched ones (batch.cu).
 //
-// Both directions hold the tile padded by the window in shared memory and
-// treat a node's L x L taps (L = 2m) as one flat list t = lane + 32 step:
-// tap t is column t mod L of row t div L.  With a row pitch = L (mod the
+// Both directions hold the tile padded by the window in shared memory.
+// Spreading treats a node's L x L taps (L = 2m) as one flat list t = lane + 32
+// step: tap t is column t mod L of row t div L.  With a row pitch = L (mod the
 // elements of one 128-byte wavefront) tap t lies in bank t (mod the same), so
 // every access of a step is free of conflicts for any L and any node, and
-// L x L taps take ceil(L L / 32) steps without idle rows.
+// L x L taps take ceil(L L / 32) steps without idle rows.  Gathering gives each
+// half-warp a node of its own, 16 div L rows (one for L > 8) a step: one column per
+// lane, so that the x window value is read once and multiplied in at the end, and the
+// weights of two nodes share a wavefront.
 //
 // A warp works alone: no CTA barrier, its tasks are independent, and as many
 // warps as shared memory allows hide each other's latencies.  Nodes go through
@@ -15,13 +18,20 @@
 // value), window values (table rows copied by cp.async one batch ahead, or
 // evaluated by Horner, lane = node).
 //
-// What bounds it (FP32, L = 8): shared-memory wavefronts, 8 for the taps'
-// read-modify-writes of a spread node (4 for the reads of a gathered one),
-// 4 for record and window values, ~1 for staging and, gathering, 2.25 for
-// the reduction of eight nodes together.  64 slices of a 256^2 stack, 8.4e6 node
-// values: gather 876 -> 357 us against one node per warp straight from L1,
-// spreading 618 (with the value sort) -> 438 us against two warps sharing a
-// tile; a radial 300 x 210 image with 98,304 nodes, m = 5: spreading 118 -> 13 us.
+// What bounds it (FP32, L = 8): shared-memory wavefronts at 89 % (gather) and
+// 94 % (spread) of one per clock and SM.  A spread node takes 13.7: 8 for the
+// taps' read-modify-writes, 4 for record and window values, the rest staging,
+// zero fill and flush.  A gathered one takes 8.5: 4 for its taps, 2 for record and window
+// values, 1.25 for the sums over the half-warp of eight nodes together, the rest
+// staging.  (One node per warp and step took 14.6 and 11.6.)
+// 64 slices of a 256^2 stack, 8.4e6 node values: gather 876 us straight from L1 with a
+// warp per node -> 361 us from the tile with 32 lanes per node -> 269 us
+// with 16; spreading 618 (with the value sort, two warps sharing a tile) -> 437
+// -> 412 us; a radial 300 x 210 image with 98,304 nodes, m = 5: spreading 118 -> 13 us.
+// 400,000 uniform nodes on a 512^2 grid, forward transform with 32 and with 16
+// lanes per node: m = 2 41.6 -> 31.5, m = 5 56.5 -> 48.0, m = 7 83.3 -> 57.1, m = 8 74.6 ->
+// 62.2 us; FP64 m = 2 224 -> 156, m = 5 570 -> 503, m = 8 1068 -> 856 us (FP64:
+// 2 + 2 / (rows per lane) operations per tap instead of 3).
 #pragma once
 
 #include "spread_body.cuh"
@@ -30,13 +40,12 @@
 namespace nfft {
 namespace {
 
-// Row pitch of the padded tile: >= the padded width, = 2m modulo the elements of a
-// wavefront.  `limit` is the pitch beyond which the tile would not fit
+// Row pitch of the padded tile: >= the padded width, = want modulo `mod`
+// elements.  `limit` is the pitch beyond which the tile would not fit
 // (then the plain width, with conflicts).
-inline int warp2_pitch(int m, int P0, int elem_bytes, int64_t limit) {
-  const int ph = 128 / elem_bytes;
+inline int warp2_pitch(int want, int mod, int P0, int64_t limit) {
   int pitch = P0;
-  while (pitch % ph != (2 * m) % ph) ++pitch;
+  while (pitch % mod != want % mod) ++pitch;
   return pitch <= limit ? pitch : P0;
 }
 
@@ -55,6 +64,11 @@ template <int L, typename T, bool TABLE> struct Warp2 {
   }
   static constexpr int ROW = TABLE ? 2 * L : pad_row(2 * L);
   static constexpr int NBUF = TABLE ? 2 : 1;
+  // L = 8, 16: a lane's taps of two successive steps lie in successive rows, so
+  // that their y window values are one 8-byte read.  L = 8 (FP32) then has
+  // rows two apart in one wavefront: pitch = 4 (mod 8) keeps those on
+  // distinct banks.
+  static constexpr bool PAIR = L == 8 || L == 16;
   // FP64 spreading: c times the y window values per node (the FP64 units
   // bound it: one product per row instead of one per tap)
   static constexpr int CROW = pad_row(2 * L);
@@ -73,7 +87,8 @@ template <int L, typename T, bool TABLE> struct Warp2 {
 template <int L, typename T, bool TABLE> int warp2_plan_pitch(const nfft_plan* p) {
   const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
   const int64_t room = int64_t(227) * 1024 - int64_t(Warp2<L, T, TABLE>::SPREAD_STAGE);
-  return warp2_pitch(p->m, P0, 2 * sizeof(T), room / (int64_t(2 * sizeof(T)) * P1));
+  const bool apart = L == 8 && sizeof(T) == 4;
+  return warp2_pitch(apart ? 2 : L, apart ? 4 : 128 / int(2 * sizeof(T)), P0, room / (int64_t(2 * sizeof(T)) * P1));
 }
 
 // The polynomial window's coefficients passed by value (uniform reads hit
@@ -168,6 +183,7 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
   using C = typename Cplx<T>::type;
   using St = Warp2Stage<L, T, TABLE>;
   constexpr bool CY = sizeof(T) == 8;
+  constexpr bool PAIR = W::PAIR && !CY;
   typename W::Rec* rec = reinterpret_cast<typename W::Rec*>(smem);
   T* win = reinterpret_cast<T*>(smem + W::REC_BYTES);
   T* cy = reinterpret_cast<T*>(smem + W::REC_BYTES + W::WIN_BYTES);
@@ -199,6 +215,8 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
     const int tt = act[s] ? t : W::TAPS - 1;
     iy[s] = tt / L;
     ix[s] = tt - iy[s] * L;
+    if constexpr (L == 8 && PAIR) iy[s] = 4 * ((lane >> 3) & 1) + 2 * (lane >> 4) + s;
+    if constexpr (L == 16 && PAIR) iy[s] = 4 * (s / 2) + 2 * (lane >> 4) + (s & 1);
     lofs[s] = iy[s] * pitch + ix[s];
   }
   int buf = 0;
@@ -250,7 +268,12 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
       for (int q = 0; q < W::NSTEP; ++q) {
         wx[q] = (32 % L == 0 && q > 0) ? wx[0] : row[ix[q]];
         if constexpr (CY) cw[q] = *reinterpret_cast<const C*>(cy + s * W::CROW + 2 * iy[q]);
-        else wy[q] = row[L + iy[q]];
+        else if constexpr (!PAIR) wy[q] = row[L + iy[q]];
+        else if (q % 2 == 0) {
+          const C v = *reinterpret_cast<const C*>(row + L + iy[q]);
+          wy[q] = v.x;
+          wy[q + 1] = v.y;
+        }
       }
     };
     fetch(0);
@@ -348,6 +371,7 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
   using W = Warp2<L, T, TABLE>;
   using C = typename Cplx<T>::type;
   using St = Warp2Stage<L, T, TABLE>;
+  constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int NK = 8;  // nodes reduced together
   typename W::Rec* rec = reinterpret_cast<typename W::Rec*>(smem);
   T* win = reinterpret_cast<T*>(smem + W::REC_BYTES);
@@ -362,17 +386,14 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
   St st;
   St::copy_rows(Nd, win, task.y, task.z, 0, lane);
   st.load(Nd, task.y, task.z, lane);
-  int lofs[W::NSTEP], ix[W::NSTEP], iy[W::NSTEP];
-  bool act[W::NSTEP];
-#pragma unroll
-  for (int s = 0; s < W::NSTEP; ++s) {
-    const int t = lane + 32 * s;
-    act[s] = W::TAPS % 32 == 0 || t < W::TAPS;
-    const int tt = act[s] ? t : W::TAPS - 1;
-    iy[s] = tt / L;
-    ix[s] = tt - iy[s] * L;
-    lofs[s] = iy[s] * pitch + ix[s];
-  }
+  // a half-warp per node, RP rows at a time: lane -> column, row of the step
+  constexpr int RP = L <= 8 ? 16 / L : 1, NS = L / RP;
+  constexpr bool PAIRS = RP == 1 || W::PAIR;  // rows of steps 2i, 2i + 1 are neighbours in a lane
+  const int half = lane >> 4;
+  const bool act = (lane & 15) < RP * L;
+  const int ix = act ? (lane & 15) % L : L - 1, ir = act ? (lane & 15) / L : 0;
+  const int iy0 = PAIRS ? ir * NS : ir;            // this lane's first row
+  const int lofs = iy0 * pitch + ix, step = PAIRS ? pitch : RP * pitch;
   int buf = 0;
   for (int b = task.y; b < task.z; b += W::NB) {
     const int n = min(W::NB, task.z - b);
@@ -391,27 +412,54 @@ __device__ __forceinline__ void gather_warp2_body(const Geom<T>& G, const Nodes<
     else cp_async_wait<0>();
     __syncwarp();
     for (int s0 = 0; s0 < n; s0 += NK) {
-      T ar[NK], ai[NK];
+      T ar[NK / 2], ai[NK / 2];
 #pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        const int s = min(s0 + k, n - 1);  // (nodes past the end repeat the last one and are dropped)
-        const C* p = tile + rec[s].off;
+      for (int k = 0; k < NK / 2; ++k) {
+        const int s = min(s0 + 2 * k + half, n - 1);  // (nodes past the end repeat the last one and are dropped)
+        const C* p = tile + rec[s].off + lofs;
         const T* row = wb + s * W::ROW;
-        T sr = T(0), si = T(0);
+        T sr = T(0), si = T(0), wy[NS];
 #pragma unroll
-        for (int q = 0; q < W::NSTEP; ++q) {
-          const T w = row[ix[q]] * row[L + iy[q]];
-          if (act[q]) {  // (idle lanes of the last step make no request)
-            const C v = p[lofs[q]];
-            sr = fma(w, v.x, sr);
-            si = fma(w, v.y, si);
+        for (int q = 0; q < NS; ++q) {
+          if constexpr (!PAIRS) wy[q] = row[L + iy0 + q * RP];
+          else if (q % 2 == 0) {
+            const C v = *reinterpret_cast<const C*>(row + L + iy0 + q);
+            wy[q] = v.x;
+            wy[q + 1] = v.y;
           }
         }
-        ar[k] = sr;
-        ai[k] = si;
+        const T wx = row[ix];
+        if constexpr (NS == 1) wy[0] *= wx;
+#pragma unroll
+        for (int q = 0; q < NS; ++q, p += step)
+          if (act) {  // (idle lanes make no request)
+            const C v = *p;
+            sr = fma(wy[q], v.x, sr);
+            si = fma(wy[q], v.y, si);
+          }
+        ar[k] = NS == 1 ? sr : sr * wx;
+        ai[k] = NS == 1 ? si : si * wx;
       }
-      warp2_reduce8(ar, ai, lane);
-      const int s = s0 + (lane >> 2);
+      // transposed butterfly within the half-warps: lane l ends with the sums
+      // of pair 2 (l & 8) / 8 + (l & 4) / 4, node l / 16 of it
+      const bool h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const T sa = h8 ? ar[k] : ar[k + 2], sb = h8 ? ai[k] : ai[k + 2];
+        ar[k] = (h8 ? ar[k + 2] : ar[k]) + __shfl_xor_sync(FULL, sa, 8);
+        ai[k] = (h8 ? ai[k + 2] : ai[k]) + __shfl_xor_sync(FULL, sb, 8);
+      }
+      {
+        const T sa = h4 ? ar[0] : ar[1], sb = h4 ? ai[0] : ai[1];
+        ar[0] = (h4 ? ar[1] : ar[0]) + __shfl_xor_sync(FULL, sa, 4);
+        ai[0] = (h4 ? ai[1] : ai[0]) + __shfl_xor_sync(FULL, sb, 4);
+      }
+#pragma unroll
+      for (int o = 2; o > 0; o >>= 1) {
+        ar[0] += __shfl_xor_sync(FULL, ar[0], o);
+        ai[0] += __shfl_xor_sync(FULL, ai[0], o);
+      }
+      const int s = s0 + 2 * (2 * int(h8) + int(h4)) + half;
       if ((lane & 3) == 0 && s < n) {
         C r;
         r.x = ar[0];
