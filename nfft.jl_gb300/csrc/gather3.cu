@@ -5,19 +5,22 @@
 //
 // One CTA per task.  A tile inside the grid comes in by one bulk tensor copy, one
 // that wraps around it by asynchronous 8-byte copies with the periodic
-// index.  A warp takes a node's x-y planes as flat lists of L x L taps
-// (t = lane + 32 step: conflict-free, the row pitch is L mod 16): it sums each
-// of its taps' columns over z, weights the sums by phi_x phi_y and adds the
-// lanes' partial sums of four nodes at once.  Nodes go through shared memory in
-// warp-private batches of four, the next batch's records and window values in
-// flight by cp.async.
+// index.  A half-warp takes a node's x-y planes as flat lists of L x L taps
+// (t = (lane mod 16) + 16 step: conflict-free, the row pitch is L mod 16): it
+// sums each of its taps' columns over z, weights the sums by phi_x phi_y and
+// adds the lanes' partial sums of two nodes at once.  Nodes go through shared memory
+// in warp-private batches of four, the next batch's records and window values in
+// flight by cp.async; rows of window values are spaced so that two nodes' reads
+// fall in distinct banks.
 //
-// Bound: shared-memory wavefronts and instruction issue.  L = 10: 100
-// wavefronts a node (70 for the taps, 13 for the window values, 3 for the
-// sums) at 70 % of one per clock and SM, 63 % of the issue slots.  240 x 216 x 180
-// grid, 600,000 radial nodes: 528 -> 263 us against the warp-per-node gather
-// straight from L1 (30 of 32 lanes, shuffled weights).  Without `act` the
-// idle lanes of the last step read a tap's bank again: 119 wavefronts, 311 us.
+// Bound: shared-memory wavefronts and instruction issue.  L = 10: 95
+// wavefronts a node (70 for the taps, 10 for the window values, 2 for the
+// sums) at 76 % of one per clock and SM, 64 % of the issue slots.  240 x 216 x 180
+// grid, 600,000 radial nodes: 528 us with the warp-per-node gather
+// straight from L1 (30 of 32 lanes, shuffled weights), 263 with a whole warp
+// per node of a tile, 251 now (128^3 transform, 10^6 uniform nodes, m = 6:
+// 820 -> 772 us).  Without `act` the idle lanes of the last step read a tap's
+// bank again: 19 wavefronts a node more; with rows of 32 floats 9 more, 261 us.
 #include "tile3.cuh"
 #include "warp2.cuh"
 
@@ -31,12 +34,20 @@ template <int BX, int BY, int BZ, int L, bool TABLE> struct Gather3 {
   using TC = Tile3<BX, BY, BZ, L>;
   static constexpr int NB = 4;                      // nodes per warp and batch
   static constexpr int TAPS = L * L;
-  static constexpr int NSTEP = (TAPS + 31) / 32;
+  static constexpr int NSTEP = (TAPS + 15) / 16;    // of a half-warp
   static constexpr int NWIN = 3 * L;
-  static constexpr int WROW = (NWIN + 3) / 4 * 4;   // staged window values of a node (16-byte rows)
+  // staged window values of a node: the values of one dimension of two
+  // neighbouring rows, read together, fall in distinct banks
+  static constexpr int row_floats() {
+    int w = NWIN;
+    while (w % 32 < L || w % 32 > 32 - L) w += 2;
+    return w;
+  }
+  static constexpr int WROW = row_floats();
   static constexpr int FRAC = TABLE ? 0 : 4;        // POLYNOMIAL: fractional offsets
   static constexpr int NODE_BYTES = 16 + WROW * 4 + FRAC * 4;
   static constexpr int SLOT = NB * NODE_BYTES;
+  static_assert(SLOT % 16 == 0 && NB * WROW % 4 == 0, "16-byte records and offsets");
   static constexpr size_t STAGE_BYTES = size_t(kG3Warps) * 2 * SLOT;
   static constexpr size_t SMEM = TC::ACC_BYTES + 16 + STAGE_BYTES;
   static constexpr int PER_SM = int((227 * 1024) / (SMEM + 1024)) < 1 ? 1 : int((227 * 1024) / (SMEM + 1024));
@@ -51,7 +62,7 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
                          int* status) {
   using TC = Tile3<BX, BY, BZ, L>;
   using GC = Gather3<BX, BY, BZ, L, TABLE>;
-  constexpr int PITCH = TC::PITCH, PLANE = TC::PLANE, NB = GC::NB, NSTEP = GC::NSTEP, NK = 4;
+  constexpr int PITCH = TC::PITCH, PLANE = TC::PLANE, NB = GC::NB, NSTEP = GC::NSTEP;
   constexpr unsigned FULL = 0xFFFFFFFFu;
   extern __shared__ __align__(1024) unsigned char smem_g3[];
   float2* tile = reinterpret_cast<float2*>(smem_g3);
@@ -123,12 +134,14 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
       for (int i = 0; i <= L; ++i) pc[r][i] = v < GC::NWIN ? __ldg(G.coeffs + (v % L) * (L + 1) + i) : 0.f;
     }
   }
+  // a half-warp per node: tap t = (lane mod 16) + 16 step of a plane
+  const int half = lane >> 4;
   int lofs[NSTEP], ix[NSTEP], iy[NSTEP];
   bool act[NSTEP];
 #pragma unroll
   for (int q = 0; q < NSTEP; ++q) {
-    const int t = lane + 32 * q;
-    act[q] = GC::TAPS % 32 == 0 || t < GC::TAPS;
+    const int t = (lane & 15) + 16 * q;
+    act[q] = GC::TAPS % 16 == 0 || t < GC::TAPS;
     const int tt = act[q] ? t : GC::TAPS - 1;
     iy[q] = tt / L;
     ix[q] = tt - iy[q] * L;
@@ -169,56 +182,51 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
       }
       __syncwarp();
     }
-    for (int s0 = 0; s0 < n; s0 += NK) {
-      float ar[NK], ai[NK];
+    float ar[NB / 2], ai[NB / 2];
 #pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        const int s = min(s0 + k, n - 1);  // (nodes past the end repeat the last one and are dropped)
-        const int4 nd = rec[s];
-        const float* wn = win + s * GC::WROW;
-        const float2* p = tile + (nd.z * PLANE + nd.y * PITCH + nd.x);
-        float sr[NSTEP], si[NSTEP];
+    for (int k = 0; k < NB / 2; ++k) {
+      const int s = min(2 * k + half, n - 1);  // (nodes past the end repeat the last one and are dropped)
+      const int4 nd = rec[s];
+      const float* wn = win + s * GC::WROW;
+      const float2* p = tile + (nd.z * PLANE + nd.y * PITCH + nd.x);
+      float sr[NSTEP], si[NSTEP];
 #pragma unroll
-        for (int q = 0; q < NSTEP; ++q) sr[q] = si[q] = 0.f;
+      for (int q = 0; q < NSTEP; ++q) sr[q] = si[q] = 0.f;
 #pragma unroll
-        for (int iz = 0; iz < L; iz += 2) {
-          const float2 wz = *reinterpret_cast<const float2*>(wn + 2 * L + iz);
+      for (int iz = 0; iz < L; iz += 2) {
+        const float2 wz = *reinterpret_cast<const float2*>(wn + 2 * L + iz);
 #pragma unroll
-          for (int q = 0; q < NSTEP; ++q)
-            if (act[q]) {  // (idle lanes of the last step make no request)
-              const float2 v0 = p[iz * PLANE + lofs[q]], v1 = p[(iz + 1) * PLANE + lofs[q]];
-              sr[q] = fmaf(wz.x, v0.x, sr[q]);
-              si[q] = fmaf(wz.x, v0.y, si[q]);
-              sr[q] = fmaf(wz.y, v1.x, sr[q]);
-              si[q] = fmaf(wz.y, v1.y, si[q]);
-            }
-        }
-        float tr = 0.f, ti = 0.f;
-#pragma unroll
-        for (int q = 0; q < NSTEP; ++q) {
-          const float w = wn[ix[q]] * wn[L + iy[q]];  // (idle lanes: zero sums)
-          tr = fmaf(w, sr[q], tr);
-          ti = fmaf(w, si[q], ti);
-        }
-        ar[k] = tr;
-        ai[k] = ti;
+        for (int q = 0; q < NSTEP; ++q)
+          if (act[q]) {  // (idle lanes of the last step make no request)
+            const float2 v0 = p[iz * PLANE + lofs[q]], v1 = p[(iz + 1) * PLANE + lofs[q]];
+            sr[q] = fmaf(wz.x, v0.x, sr[q]);
+            si[q] = fmaf(wz.x, v0.y, si[q]);
+            sr[q] = fmaf(wz.y, v1.x, sr[q]);
+            si[q] = fmaf(wz.y, v1.y, si[q]);
+          }
       }
-      // transposed butterfly: lane l ends with node l / 8 summed over all lanes
-      const bool h = (lane & 16) != 0, e = (lane & 8) != 0;
-      const float a0 = (h ? ar[2] : ar[0]) + __shfl_xor_sync(FULL, h ? ar[0] : ar[2], 16);
-      const float a1 = (h ? ar[3] : ar[1]) + __shfl_xor_sync(FULL, h ? ar[1] : ar[3], 16);
-      const float b0 = (h ? ai[2] : ai[0]) + __shfl_xor_sync(FULL, h ? ai[0] : ai[2], 16);
-      const float b1 = (h ? ai[3] : ai[1]) + __shfl_xor_sync(FULL, h ? ai[1] : ai[3], 16);
-      float sr = (e ? a1 : a0) + __shfl_xor_sync(FULL, e ? a0 : a1, 8);
-      float si = (e ? b1 : b0) + __shfl_xor_sync(FULL, e ? b0 : b1, 8);
+      float tr = 0.f, ti = 0.f;
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        sr += __shfl_xor_sync(FULL, sr, o);
-        si += __shfl_xor_sync(FULL, si, o);
+      for (int q = 0; q < NSTEP; ++q) {
+        const float w = (16 % L == 0 ? wn[ix[0]] : wn[ix[q]]) * wn[L + iy[q]];  // (idle lanes: zero sums)
+        tr = fmaf(w, sr[q], tr);
+        ti = fmaf(w, si[q], ti);
       }
-      const int s = s0 + (lane >> 3);
-      if ((lane & 7) == 0 && s < n) fhat[rec[s].w] = make_float2(sr, si);
+      ar[k] = tr;
+      ai[k] = ti;
     }
+    // transposed butterfly: lanes l = 0, 8 (mod 16) end with pair l / 8 mod 2's node l / 16
+    static_assert(NB == 4, "two pairs of nodes");
+    const bool e = (lane & 8) != 0;
+    float tr = (e ? ar[1] : ar[0]) + __shfl_xor_sync(FULL, e ? ar[0] : ar[1], 8);
+    float ti = (e ? ai[1] : ai[0]) + __shfl_xor_sync(FULL, e ? ai[0] : ai[1], 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      tr += __shfl_xor_sync(FULL, tr, o);
+      ti += __shfl_xor_sync(FULL, ti, o);
+    }
+    const int s = 2 * int(e) + half;
+    if ((lane & 7) == 0 && s < n) fhat[rec[s].w] = make_float2(tr, ti);
     __syncwarp();  // the slot is read before it is staged again
   }
   asm volatile("cp.async.wait_all;" ::: "memory");

@@ -166,16 +166,19 @@ __global__ void __launch_bounds__(kInterpThreads) interp_tile_kernel(Geom<T> G, 
 // Shape-specialised 3-D FP32 gather (m = 4, the tiles of tile3.cuh).  One CTA
 // per spreading task; a tile whose padded box lies inside the grid is brought
 // into shared memory by one bulk tensor copy (TMA, completion on an
-// mbarrier), and each warp then interpolates one node at a time from shared
-// memory: lane (x = lane mod 8, row = lane / 8) reads its 8 z values of rows
-// iy and iy + 4 at constant offsets (16 loads, 2 wavefronts each), sums over
-// z and weights by phi_x phi_y; the warp adds the 32 partial sums of four
-// nodes at once.  Window values come straight from the table (broadcast
-// loads): shuffles share the shared-memory pipe with the tile reads.  Tiles
-// whose box wraps around the grid gather their nodes straight from L1/L2 as
-// interp_kernel does.  The wait for the copy is bounded: on timeout the CTA
-// raises status word 1 (reported by nfft_sync) and skips its nodes.
-
+// mbarrier), and each half-warp then interpolates one node at a time from
+// shared memory: lane (x = lane mod 8, row = lane / 8 mod 2) reads its 8 z values of
+// rows iy, iy + 2, iy + 4 and iy + 6 at constant offsets (32 loads, one
+// wavefront each), sums over z and weights by phi_x phi_y; the half-warp adds the
+// 16 partial sums of two nodes at once.  Window values come straight from the
+// table (broadcast loads, two nodes to a wavefront): shuffles share the
+// shared-memory pipe with the tile reads.  Tiles whose box wraps around the
+// grid gather their nodes straight from L1/L2 as interp_kernel does.  The wait for
+// the copy is bounded: on timeout the CTA raises status word 1 (reported by
+// nfft_sync) and skips its nodes.
+// Bound: 41.7 shared-memory wavefronts per node (32 for the taps) at 82 % of one
+// per clock and SM, the rest waiting for tiles; 256^3, 4.2e6 radial
+// nodes: 750 (46 wavefronts, a whole warp per node) -> 686 us.
 
 // Per-warp staging of the TMA gather: NK nodes per group, WCH 16-byte chunks
 // of window data per node (24 table values, or the 4 fractional offsets),
@@ -232,7 +235,8 @@ __global__ void __launch_bounds__(kInterpThreads, 4) interp_tile3_kernel(const _
   // group is summed; the first group's while the tile arrives.
   constexpr int NK = Tile3Gather<TABLE>::NK, WCH = Tile3Gather<TABLE>::WCH, SLOT = Tile3Gather<TABLE>::SLOT;
   constexpr int NS = Tile3Gather<TABLE>::NS;
-  const int ix = lane & 7, ry = lane >> 3;
+  // a half-warp per node: column lane mod 8, rows ry, ry + 2, ry + 4, ry + 6
+  const int ix = lane & 7, ry = (lane >> 3) & 1, half = lane >> 4;
   unsigned char* stage_base = smem_raw + TC::ACC_BYTES + 16 + warp * NS * SLOT;
   // this lane's copy in a stage: window chunk c of node k (lanes < NK WCH)
   // or the record of node lane - 24 (lanes 24 .. 24 + NK - 1); node indices
@@ -309,64 +313,61 @@ __global__ void __launch_bounds__(kInterpThreads, 4) interp_tile3_kernel(const _
     }
     const int4* rec = reinterpret_cast<const int4*>(st);
     const float* win = reinterpret_cast<const float*>(st + NK * 16);
-    float ar[NK], ai[NK];
+    float ar[NK / 2], ai[NK / 2];
     // node k's partial sums (tail groups: nodes past the task end add zero)
-    auto node = [&](int k, bool valid) {
+    auto node = [&](int j, bool valid) {
+      const int k = 2 * j + half;
       const int4 nd = rec[k];
-      // window values: x at the lane's column, y at its two rows, all 8 z
-      float wx, wy0, wy1, wz[8];
-      {  // broadcast reads of the staged window values
-        const float* wt = win + k * 24;
-        wx = wt[ix];
-        wy0 = wt[8 + ry];
-        wy1 = wt[12 + ry];
-        const float4 z0 = *reinterpret_cast<const float4*>(wt + 16);
-        const float4 z1 = *reinterpret_cast<const float4*>(wt + 20);
-        wz[0] = z0.x, wz[1] = z0.y, wz[2] = z0.z, wz[3] = z0.w;
-        wz[4] = z1.x, wz[5] = z1.y, wz[6] = z1.z, wz[7] = z1.w;
-      }
+      // window values: x at the lane's column, y at its four rows, all 8 z
+      const float* wt = win + k * 24;
+      const float wx = wt[ix];
+      float wy[4], wz[8];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) wy[r] = wt[8 + ry + 2 * r];
+      const float4 z0 = *reinterpret_cast<const float4*>(wt + 16);
+      const float4 z1 = *reinterpret_cast<const float4*>(wt + 20);
+      wz[0] = z0.x, wz[1] = z0.y, wz[2] = z0.z, wz[3] = z0.w;
+      wz[4] = z1.x, wz[5] = z1.y, wz[6] = z1.z, wz[7] = z1.w;
       // (a node past the task end reads tap 0 of the tile and is dropped)
       const float2* bp = tile + (valid ? nd.z * PLANE + nd.y * PITCH + nd.x + lane_off : 0);
-      float2 v0[8], v1[8];
+      float sr[4], si[4];
 #pragma unroll
-      for (int iz = 0; iz < 8; ++iz) {
-        v0[iz] = bp[iz * PLANE];
-        v1[iz] = bp[iz * PLANE + 4 * PITCH];
-      }
-      float s0r = 0.f, s0i = 0.f, s1r = 0.f, s1i = 0.f;
+      for (int r = 0; r < 4; ++r) sr[r] = si[r] = 0.f;
 #pragma unroll
-      for (int iz = 0; iz < 8; ++iz) {
-        s0r = fmaf(wz[iz], v0[iz].x, s0r);
-        s0i = fmaf(wz[iz], v0[iz].y, s0i);
-        s1r = fmaf(wz[iz], v1[iz].x, s1r);
-        s1i = fmaf(wz[iz], v1[iz].y, s1i);
+      for (int iz = 0; iz < 8; ++iz)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float2 v = bp[iz * PLANE + 2 * r * PITCH];
+          sr[r] = fmaf(wz[iz], v.x, sr[r]);
+          si[r] = fmaf(wz[iz], v.y, si[r]);
+        }
+      float tr = 0.f, ti = 0.f;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        tr = fmaf(wy[r], sr[r], tr);
+        ti = fmaf(wy[r], si[r], ti);
       }
-      ar[k] = valid ? wx * fmaf(wy0, s0r, wy1 * s1r) : 0.f;
-      ai[k] = valid ? wx * fmaf(wy0, s0i, wy1 * s1i) : 0.f;
+      ar[j] = valid ? wx * tr : 0.f;
+      ai[j] = valid ? wx * ti : 0.f;
     };
     if (base + NK <= task.z) {
 #pragma unroll
-      for (int k = 0; k < NK; ++k) node(k, true);
+      for (int j = 0; j < NK / 2; ++j) node(j, true);
     } else {
 #pragma unroll
-      for (int k = 0; k < NK; ++k) node(k, base + k < task.z);
+      for (int j = 0; j < NK / 2; ++j) node(j, base + 2 * j + half < task.z);
     }
-    // transposed reduction: after the xor-16 and xor-8 steps lane l holds
-    // node l / 8 summed over 4 lanes' worth of partials; three more steps
-    // finish it on the lanes l = 8 k
-    const bool h = (lane & 16) != 0, q = (lane & 8) != 0;
-    float a0 = (h ? ar[2] : ar[0]) + __shfl_xor_sync(0xFFFFFFFFu, h ? ar[0] : ar[2], 16);
-    float a1 = (h ? ar[3] : ar[1]) + __shfl_xor_sync(0xFFFFFFFFu, h ? ar[1] : ar[3], 16);
-    float b0 = (h ? ai[2] : ai[0]) + __shfl_xor_sync(0xFFFFFFFFu, h ? ai[0] : ai[2], 16);
-    float b1 = (h ? ai[3] : ai[1]) + __shfl_xor_sync(0xFFFFFFFFu, h ? ai[1] : ai[3], 16);
-    float sr = (q ? a1 : a0) + __shfl_xor_sync(0xFFFFFFFFu, q ? a0 : a1, 8);
-    float si = (q ? b1 : b0) + __shfl_xor_sync(0xFFFFFFFFu, q ? b0 : b1, 8);
+    // transposed reduction within the half-warps: lanes l = 0, 8 (mod 16) end
+    // with pair (l / 8) mod 2's node l / 16
+    const bool e = (lane & 8) != 0;
+    float sr = (e ? ar[1] : ar[0]) + __shfl_xor_sync(0xFFFFFFFFu, e ? ar[0] : ar[1], 8);
+    float si = (e ? ai[1] : ai[0]) + __shfl_xor_sync(0xFFFFFFFFu, e ? ai[0] : ai[1], 8);
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
       sr += __shfl_xor_sync(0xFFFFFFFFu, sr, o);
       si += __shfl_xor_sync(0xFFFFFFFFu, si, o);
     }
-    const int kk = lane >> 3;
+    const int kk = 2 * int(e) + half;
     if ((lane & 7) == 0 && base + kk < task.z) fhat[rec[kk].w] = make_float2(sr, si);
     __syncwarp();  // the slot is read before it is staged again
     buf = buf + 1 == NS ? 0 : buf + 1;
