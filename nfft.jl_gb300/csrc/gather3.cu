@@ -260,16 +260,23 @@ template <int L> int gather3_shape(nfft_plan* p, const float2* g, float2* fhat) 
 
 // -1: the plan's tiles or window have no compiled kernel, or too few nodes per
 // task to pay for bringing their tile (L = 10: 60 KB) into shared memory.
-// Forward transform, us tiled / direct: m = 5, 2048 tasks: 20,000 nodes 71 / 48, 40,000
-// 75 / 67, 100,000 92 / 134; 9,300 tasks: 100,000 nodes 265 / 239, 600,000 385 / 635; 360
-// tasks (one or two CTAs per SM): 20,000 nodes 65 / 61, 40,000 74 / 81.  m = 3, 2048
-// tasks: 40,000 nodes 55 / 43, 100,000 63 / 67; 360 tasks: 40,000 57 / 54, 100,000 71 / 79.
-// m = 4, 2048 tasks: 100,000 uniform / radial nodes 71, 83 / 72, 300,000 102, 113 / 138,
-// 10^6 212, 213 / 382; 360 tasks: 100,000 76, 100 / 85, 300,000 130, 126 / 149.
+// Forward transform, us tiled / direct, uniform (radial) nodes:
+//   m = 2: 64^3, 2048 tasks, 48 nodes per task 50 / 48 (41 / 47), 96: 55 / 62 (46 / 62);
+//          128^3, 16,384 tasks, 48: 218 / 232 (167 / 227), 96: 252 / 357 (201 / 353)
+//   m = 3: 64^3, 24: 56 / 46 (46 / 46), 48: 60 / 67 (50 / 66); 128^3, 24: 253 / 235
+//          (180 / 229), 48: 290 / 357 (221 / 355)
+//   m = 5: 64^3, 24: 79 / 75 (61 / 74), 48: 91 / 132 (72 / 130); 128^3, 12: 333 / 290
+//          (198 / 285), 24: 364 / 448 (262 / 441)
+//   m = 6: 64^3, 12: 97 / 87 (69 / 86), 24: 106 / 145 (82 / 145); 128^3, 12: 478 / 561
+//          (255 / 561), 24: 535 / 931 (359 / 927)
+// 27^3, 360 tasks (one or two CTAs per SM): m = 3, 34,560 nodes 46 / 44, m = 5, 17,280
+// 52 / 50, 34,560 60 / 68.  m = 4, 2048 tasks: 100,000 uniform / radial nodes 71, 83 /
+// 72, 300,000 102, 113 / 138.
 int launch_gather_plane3(const nfft_plan* cp, const void* g, void* fhat) {
   nfft_plan* p = const_cast<nfft_plan*>(cp);  // the tensor-map cache only
   if (!p->gather_tma || !p->tasks || p->n_tasks == 0 || p->D != 3 || p->precision != 32 || p->bs[2] != 8) return -1;
-  if (p->m >= 5 ? p->M < 32 * p->n_tasks || p->M < 32768 : p->M < 64 * p->n_tasks || p->M < 131072) return -1;
+  const int per_task = p->m == 2 ? 64 : p->m <= 4 ? 48 : p->m == 5 ? 32 : 24;
+  if (p->M < per_task * p->n_tasks || p->M < (p->m >= 5 ? 32768 : 65536)) return -1;
   const float2* gp = static_cast<const float2*>(g);
   float2* f = static_cast<float2*>(fhat);
   switch (p->m) {
