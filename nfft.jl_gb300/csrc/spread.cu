@@ -271,6 +271,13 @@ int spread_dispatch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t 
 // memory to clear each CTA's tile (allocated once per plan).
 const float4* zero_tile_for(nfft_plan* p) {
   if (!p->zero_tile && p->spread_zero_copy) {
+    // nothing is allocated while the caller captures a graph (the copy source
+    // is made by the first call outside one): plain stores clear the tile
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(p->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return nullptr;
+    }
     if (cudaMalloc(&p->zero_tile, kZeroTileBytes) != cudaSuccess ||
         cudaMemsetAsync(p->zero_tile, 0, kZeroTileBytes, p->stream) != cudaSuccess) {
       cudaFree(p->zero_tile);

@@ -59,3 +59,23 @@ def test_plane3_without_bulk_copies(monkeypatch, m):
 def test_plane3_sparse_and_tiny(m):
     check((40, 40, 40), 61, m, oracle.POLYNOMIAL, (16, 8, 8))   # fewer than six nodes per task
     check((10, 9, 8), 1500, m, oracle.TENSOR, (8, 8, 8))         # every tile wraps, boxes exceed the grid
+
+
+@pytest.mark.parametrize("m", [3, 4, 5])
+def test_first_adjoint_inside_a_capture(m):
+    """The first adjoint of a plan, captured into a graph by the caller: nothing is allocated for it."""
+    N = (48, 40, 32)
+    k, _, v = problem(N, 3000, 7)
+    want = (nf.adjoint(nf.plan_nfft(k, N, m=m, sigma=2.0)) * torch.as_tensor(v)).cpu().numpy()
+    p = nf.plan_nfft(k, N, m=m, sigma=2.0)
+    x = torch.as_tensor(v).cuda()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = nf.adjoint(p) * x
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert oracle.rel_l2(y.cpu().numpy().ravel(), want.ravel()) < TOL32
+    y = (nf.adjoint(p) * x).cpu().numpy()  # and outside one
+    assert oracle.rel_l2(y.ravel(), want.ravel()) < TOL32
