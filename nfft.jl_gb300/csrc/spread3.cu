@@ -7,11 +7,11 @@
 namespace nfft {
 namespace {
 
-template <int BX, int BY, int BZ, int L, bool TABLE>
+template <int BX, int BY, int BZ, int L, int NW, bool TABLE>
 int plane3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fhat, float* gp, int ncols,
                   int64_t fcol, int64_t gcol_t) {
   using TC = Tile3<BX, BY, BZ, L>;
-  using PC = Plane3<BX, BY, BZ, L>;
+  using PC = Plane3<BX, BY, BZ, L, NW>;
   static_assert(TC::NACC * 8 <= kZeroTileBytes, "zero tile buffer");
   const CUtensorMap* map = (ncols == 1 && p->spread_tma) ? tile3_map<BX, BY, BZ, L>(p, gp) : nullptr;
   CUtensorMap none{};
@@ -19,7 +19,7 @@ int plane3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, co
   Plane3Poly<L, TABLE> wp{};
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = float(p->coeffs_host[q]);
-  auto kern = spread_plane3_kernel<BX, BY, BZ, L, TABLE>;
+  auto kern = spread_plane3_kernel<BX, BY, BZ, L, NW, TABLE>;
   NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PC::SMEM)));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), PC::THREADS, PC::SMEM, p->stream>>>(
       map ? *map : none, map ? 1 : 0, G, Nd, p->tasks, fhat, gp, ncols > 1 ? fcol : 0, gcol_t, zeros, p->dflag + 1, wp);
@@ -27,11 +27,35 @@ int plane3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, co
   return NFFT_OK;
 }
 
-template <int BX, int BY, int BZ, int L>
+template <int BX, int BY, int BZ, int L, int NW>
 int plane3_table(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fhat, float* gp, int ncols,
                  int64_t fcol, int64_t gcol_t) {
-  return p->wtab ? plane3_launch<BX, BY, BZ, L, true>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t)
-                 : plane3_launch<BX, BY, BZ, L, false>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+  return p->wtab ? plane3_launch<BX, BY, BZ, L, NW, true>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t)
+                 : plane3_launch<BX, BY, BZ, L, NW, false>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+}
+
+// Two or four warps per tile.  Two read a node's weights half as often, four
+// hide more latency where a tile has few nodes; L = 12's 68 KB tiles leave two CTAs per
+// SM and want four.  Adjoint, us with two / four warps, uniform (radial) nodes:
+//   m = 2: 64^3: 5,000 nodes 45 / 45 (40 / 42), 10^6 133 / 166 (124 / 160)
+//   m = 3: 64^3: 50,000 67 / 63 (57 / 60), 200,000 97 / 102 (90 / 100), 4e6 875 / 1024;
+//          128^3: 200,000 242 / 232 (182 / 188), 500,000 291 / 294 (242 / 254), 4e6 940 / 1094
+//   m = 4: 64^3: 2e6 705 / 693 (686 / 708), 4e6 1275 / 1308 (1279 / 1322);
+//          128^3: 10^6 519 / 499 (450 / 453), 4e6 1372 / 1399 (1310 / 1356)
+//   m = 5: 128^3: 10^6 902 / 870 (789 / 796), 2e6 1482 / 1482, 4e6 2658 / 2723 (2573 / 2662)
+template <int L> bool plane3_two_warps(const nfft_plan* p) {
+  if (L == 4) return true;
+  if (L == 6) return p->M >= (int64_t(1) << 17) && p->M >= 24 * p->n_tasks;
+  return L < 12 && p->M >= 3 * (int64_t(1) << 20);
+}
+
+template <int BX, int BY, int BZ, int L>
+int plane3_warps(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, const float2* fhat, float* gp, int ncols,
+                 int64_t fcol, int64_t gcol_t) {
+  if constexpr (L < 12)
+    if (plane3_two_warps<L>(p)) return plane3_table<BX, BY, BZ, L, 2>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+  if constexpr (L > 4) return plane3_table<BX, BY, BZ, L, 4>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+  return -1;
 }
 
 template <int L>
@@ -39,11 +63,11 @@ int plane3_shape(nfft_plan* p, const Nodes<float>& Nd, const float2* fhat, float
                  int64_t gcol_t) {
   const Geom<float> G = make_geom<float>(p);
   const int64_t bx = p->bs[0], by = p->bs[1];
-  if (bx == 16 && by == 8) return plane3_table<16, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-  if (bx == 8 && by == 8) return plane3_table<8, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+  if (bx == 16 && by == 8) return plane3_warps<16, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+  if (bx == 8 && by == 8) return plane3_warps<8, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
   if constexpr (L == 8) {
-    if (bx == 16 && by == 16) return plane3_table<16, 16, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
-    if (bx == 32 && by == 8) return plane3_table<32, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+    if (bx == 16 && by == 16) return plane3_warps<16, 16, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
+    if (bx == 32 && by == 8) return plane3_warps<32, 8, 8, L>(p, G, Nd, fhat, gp, ncols, fcol, gcol_t);
   }
   return -1;
 }

@@ -1,15 +1,15 @@
 // 3-D FP32 spreading by plane owners, for any window width L = 2m and tile
 // shapes fixed at compile time (tile3.cuh).
 //
-// Four warps share the padded tile; warp w owns its z planes = w mod 4, so
-// every point has one writer and the accumulation is a plain read-modify-write.
-// A node has ceil(L / 4) or floor(L / 4) planes per warp, each a flat list of
-// L x L taps t = lane + 32 step (tap t: column t mod L of row t div L), free of
-// bank conflicts because the row pitch is L mod 16.  The x-y weight products
-// of a node are read once per warp and used for all of its planes.
+// NW (two or four) warps share the padded tile; warp w owns its z planes = w
+// mod NW, so every point has one writer and the accumulation is a plain
+// read-modify-write.  A node has ceil(L / NW) or floor(L / NW) planes per warp, each a
+// flat list of L x L taps t = lane + 32 step (tap t: column t mod L of row t div L),
+// free of bank conflicts because the row pitch is L mod 16.  The x-y weight
+// products of a node are read once per warp and used for all of its planes.
 //
-// Staging (16 nodes at a time, eight threads per node, loads one batch ahead
-// in registers): thread j of a node writes rows j and j + 8 of the products
+// Staging (16 nodes at a time, 2 NW threads per node, loads one batch ahead
+// in registers): thread j of a node writes rows j, j + 2 NW, .. of the products
 // and the planes' records {offset of the warp's first tap, planes, value x z
 // window values of the planes}.  The tile is cleared by one bulk copy of
 // zeros and, where it does not wrap around the grid, added to it by one bulk
@@ -17,11 +17,12 @@
 // wrapping tiles and grids without a tensor map use the per-point flush of
 // spread_body.cuh.
 //
-// Bound: shared-memory wavefronts.  L = 8: 94 per node measured, of which 64
-// are the taps', 8 the products' and 8 the records' (with eight warps that own
-// one plane of a node each, 107: every warp reads the products again), at
-// 89 % of one per clock and SM; 256^3 radial set (4.2e6 nodes) 1.58 -> 1.49 ms.
-// L = 10: 195 (140 + 16 + 8 and the staging) against ~410 of the generic
+// Bound: shared-memory wavefronts, of which a node's taps take 64 (L = 8) or 140 (L =
+// 10).  L = 8: 89 per node with two warps at 86 % of one per clock and SM, 94 at 89 %
+// with four (more warps read the products and records again, but fewer do not
+// hide the latencies as well), 107 with eight; 256^3 radial set (4.2e6 nodes) 1.58
+// (eight) -> 1.49 (four) -> 1.46 ms (two).
+// L = 10: 195 (140 + 16 + 8 and the staging) with four warps against ~410 of the generic
 // kernel of spread_body.cuh; 300,001 uniform nodes, 202 x 174 x 150 grid 393 -> 246 us.
 #pragma once
 
@@ -31,10 +32,12 @@
 namespace nfft {
 namespace {
 
-template <int BX, int BY, int BZ, int L> struct Plane3 {
+template <int BX, int BY, int BZ, int L, int NW_> struct Plane3 {
   using TC = Tile3<BX, BY, BZ, L>;
-  static constexpr int NW = 4, THREADS = NW * 32;
+  static constexpr int NW = NW_, THREADS = NW * 32;
   static constexpr int NB = 16;                     // nodes per staged batch
+  static constexpr int TPN = THREADS / NB;          // threads that stage a node
+  static constexpr int RPT = (L + TPN - 1) / TPN;   // window rows and planes of each
   static constexpr int TAPS = L * L;
   static constexpr int NSTEP = (TAPS + 31) / 32;
   static constexpr int KS = (L + NW - 1) / NW;      // planes of a node per warp (most)
@@ -61,14 +64,15 @@ template <int L> __device__ __forceinline__ float plane3_horner(const float* c, 
   return v;
 }
 
-template <int BX, int BY, int BZ, int L, bool TABLE>
-__global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_plane3_kernel(
+template <int BX, int BY, int BZ, int L, int NW, bool TABLE>
+__global__ void __launch_bounds__((Plane3<BX, BY, BZ, L, NW>::THREADS), (Plane3<BX, BY, BZ, L, NW>::PER_SM)) spread_plane3_kernel(
     const __grid_constant__ CUtensorMap tmap, int use_tma, Geom<float> G, Nodes<float> Nd,
     const int4* __restrict__ tasks, const float2* __restrict__ fhat, float* __restrict__ g, int64_t fcol, int64_t gcol,
     const float4* __restrict__ zeros, int* status, const __grid_constant__ Plane3Poly<L, TABLE> wp) {
   using TC = Tile3<BX, BY, BZ, L>;
-  using PC = Plane3<BX, BY, BZ, L>;
+  using PC = Plane3<BX, BY, BZ, L, NW>;
   constexpr int NB = PC::NB, PITCH = TC::PITCH, PLANE = TC::PLANE, KS = PC::KS, NSTEP = PC::NSTEP, RW = PC::RW;
+  constexpr int TPN = PC::TPN, RPT = PC::RPT;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   fhat += blockIdx.y * fcol;  // column of a multi-column launch
   g += blockIdx.y * gcol;
@@ -98,22 +102,21 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
   }
   bool zeroed = zeros == nullptr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int s = threadIdx.x >> 3, j = threadIdx.x & 7;  // staged node, its rows / planes j and j + 8
-  constexpr bool ROW0 = L >= 8, ROW2 = L > 8;
-  const bool has1 = ROW0 || j < L, has2 = ROW2 && j + 8 < L;
+  const int s = threadIdx.x / TPN, j = threadIdx.x % TPN;  // staged node, its rows / planes j, j + TPN, ..
 
   int4 r_nd = make_int4(0, 0, 0, 0);
   float2 r_c = make_float2(0.f, 0.f);
-  float r_x[L], r_y[2] = {0.f, 0.f}, r_z[2] = {0.f, 0.f};
+  float r_x[L], r_y[RPT], r_z[RPT];
   float4 r_f = make_float4(0.f, 0.f, 0.f, 0.f);
-  float c1[TABLE ? 1 : L + 1], c2[TABLE || !ROW2 ? 1 : L + 1];  // Horner: coefficients of columns j and j + 8
+  float cj[RPT][TABLE ? 1 : L + 1];  // Horner: coefficients of this thread's columns
 #pragma unroll
   for (int i = 0; i < L; ++i) r_x[i] = 0.f;
-  if constexpr (!TABLE) {
 #pragma unroll
-    for (int i = 0; i <= L; ++i) {
-      c1[i] = has1 ? __ldg(G.coeffs + j * (L + 1) + i) : 0.f;
-      if constexpr (ROW2) c2[i] = has2 ? __ldg(G.coeffs + (j + 8) * (L + 1) + i) : 0.f;
+  for (int h = 0; h < RPT; ++h) {
+    r_y[h] = r_z[h] = 0.f;
+    if constexpr (!TABLE) {
+#pragma unroll
+      for (int i = 0; i <= L; ++i) cj[h][i] = j + TPN * h < L ? __ldg(G.coeffs + (j + TPN * h) * (L + 1) + i) : 0.f;
     }
   }
   // the node's record two batches ahead (its index addresses the value), the
@@ -135,14 +138,12 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
           r_x[q] = v.x;
           r_x[q + 1] = v.y;
         }
-        if (has1) {
-          r_y[0] = __ldg(wt + L + j);
-          r_z[0] = __ldg(wt + 2 * L + j);
-        }
-        if (has2) {
-          r_y[1] = __ldg(wt + L + j + 8);
-          r_z[1] = __ldg(wt + 2 * L + j + 8);
-        }
+#pragma unroll
+        for (int h = 0; h < RPT; ++h)
+          if (j + TPN * h < L) {
+            r_y[h] = __ldg(wt + L + j + TPN * h);
+            r_z[h] = __ldg(wt + 2 * L + j + TPN * h);
+          }
       } else {
         r_f = __ldg(reinterpret_cast<const float4*>(Nd.frac4) + i);
       }
@@ -169,24 +170,23 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
         const float tx = r_f.x - 0.5f, ty = r_f.y - 0.5f, tz = r_f.z - 0.5f;
 #pragma unroll
         for (int l = 0; l < L; ++l) r_x[l] = plane3_horner<L>(wp.c + l * (L + 1), tx);
-        r_y[0] = plane3_horner<L>(c1, ty);
-        r_z[0] = plane3_horner<L>(c1, tz);
-        if constexpr (ROW2) {
-          r_y[1] = plane3_horner<L>(c2, ty);
-          r_z[1] = plane3_horner<L>(c2, tz);
+#pragma unroll
+        for (int h = 0; h < RPT; ++h) {
+          r_y[h] = plane3_horner<L>(cj[h], ty);
+          r_z[h] = plane3_horner<L>(cj[h], tz);
         }
       }
       const int z0 = r_nd.z - o2;
       const int oxy = (r_nd.y - o1) * PITCH + (r_nd.x - o0 + TC::LEAD);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 0 ? !has1 : !has2) continue;
-        const int i = j + 8 * h;  // window row and plane
+      for (int h = 0; h < RPT; ++h) {
+        const int i = j + TPN * h;  // window row and plane
+        if (L % TPN != 0 && i >= L) continue;
         float* row = s_xy + s * PC::XYS + i * L;
         if constexpr (L % 4 == 0) {
           // (L = 8: the two halves in an order that keeps the eight rows of a
-          // 128-bit store phase on distinct banks)
-          const int swap = L == 8 ? (j >> 2) & 1 : 0;
+          // 128-bit store phase, of one or two nodes, on distinct banks)
+          const int swap = L != 8 ? 0 : TPN == 8 ? j >> 2 : s & 1;
 #pragma unroll
           for (int q = 0; q < L; q += 4) {
             float4 v = make_float4(r_x[q] * r_y[h], r_x[q + 1] * r_y[h], r_x[q + 2] * r_y[h], r_x[q + 3] * r_y[h]);
@@ -199,11 +199,12 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
           for (int q = 0; q < L; q += 2)
             *reinterpret_cast<float2*>(row + q) = make_float2(r_x[q] * r_y[h], r_x[q + 1] * r_y[h]);
         }
-        // window plane i is tile plane z0 + i, owned by warp (z0 + i) mod 4
-        // as its plane number i / 4
-        float2* rec = s_rec + s * PC::RECS + ((z0 + i) & 3) * RW;
-        rec[1 + (i >> 2)] = make_float2(r_c.x * r_z[h], r_c.y * r_z[h]);
-        if (i < 4) rec[0] = make_float2(__int_as_float((z0 + i) * PLANE + oxy), __int_as_float((L - i + 3) >> 2));
+        // window plane i is tile plane z0 + i, owned by warp (z0 + i) mod NW
+        // as its plane number i / NW
+        float2* rec = s_rec + s * PC::RECS + ((z0 + i) % NW) * RW;
+        rec[1 + i / NW] = make_float2(r_c.x * r_z[h], r_c.y * r_z[h]);
+        if (i < NW)
+          rec[0] = make_float2(__int_as_float((z0 + i) * PLANE + oxy), __int_as_float((L - i + NW - 1) / NW));
       }
     }
     __syncthreads();
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
     fetch(0);
     for (int q = 0; q < n; ++q) {
       float2* p = acc + __float_as_int(rt[0].x);
-      const bool last = L % 4 == 0 || __float_as_int(rt[0].y) == KS;  // this warp has KS planes of the node
+      const bool last = L % NW == 0 || __float_as_int(rt[0].y) == KS;  // this warp has KS planes of the node
       float2 cz[KS];
       float wc[NSTEP];
 #pragma unroll
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
         if (k + 1 < KS || last) {
 #pragma unroll
           for (int i = 0; i < NSTEP; ++i)
-            if (act[i]) a[k][i] = p[4 * k * PLANE + lofs[i]];
+            if (act[i]) a[k][i] = p[NW * k * PLANE + lofs[i]];
         }
       fetch(q + 1 < n ? q + 1 : q);
 #pragma unroll
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
             if (act[i]) {
               a[k][i].x = fmaf(cz[k].x, wc[i], a[k][i].x);
               a[k][i].y = fmaf(cz[k].y, wc[i], a[k][i].y);
-              p[4 * k * PLANE + lofs[i]] = a[k][i];
+              p[NW * k * PLANE + lofs[i]] = a[k][i];
             }
         }
     }
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(128, (Plane3<BX, BY, BZ, L>::PER_SM)) spread_p
     }
     return;
   }
-  flush_tile<3, float, false, 4>(G, acc + TC::LEAD, g, o0, o1, o2, BX + L - 1, TC::P1, TC::P2, PITCH);
+  flush_tile<3, float, false, NW>(G, acc + TC::LEAD, g, o0, o1, o2, BX + L - 1, TC::P1, TC::P2, PITCH);
 }
 
 }  // namespace

@@ -79,3 +79,15 @@ def test_first_adjoint_inside_a_capture(m):
         assert oracle.rel_l2(y.cpu().numpy().ravel(), want.ravel()) < TOL32
     y = (nf.adjoint(p) * x).cpu().numpy()  # and outside one
     assert oracle.rel_l2(y.ravel(), want.ravel()) < TOL32
+
+
+@pytest.mark.parametrize("m,M", [(3, 140001), (4, 3 * 2**20 + 7), (5, 3 * 2**20 + 7)])
+@pytest.mark.parametrize("pre", [oracle.TENSOR, oracle.POLYNOMIAL])
+def test_many_nodes(m, M, pre):
+    """Two warps per tile (node sets beyond the rule's lines), against the same adjoint in double precision."""
+    N = (40, 36, 44)
+    k, _, v = problem(N, M, 11)
+    x = (nf.adjoint(nf.plan_nfft(k, N, m=m, sigma=2.0, precompute=pre)) * torch.as_tensor(v)).cpu().numpy()
+    q = nf.plan_nfft(k.astype(np.float64), N, m=m, sigma=2.0, precompute=pre)
+    y = (nf.adjoint(q) * torch.as_tensor(v.astype(np.complex128))).cpu().numpy()
+    assert oracle.rel_l2(x.ravel(), y.ravel()) < TOL32
