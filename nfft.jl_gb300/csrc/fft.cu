@@ -562,6 +562,21 @@ __device__ __forceinline__ void twiddle4(C (&v)[R1], int n2, const C* __restrict
 
 constexpr int kW4 = 16;  // lines per CTA
 
+// The same from the table's copy in shared memory, exp(-2 pi i n2 k1 / N) at k1 R2 + n2.
+template <int S, int R1, int R2, typename C>
+__device__ __forceinline__ void twiddle4_smem(C (&v)[R1], int n2, const C* s_tw) {
+#pragma unroll
+  for (int k1 = 1; k1 < R1; ++k1) {
+    C tt = s_tw[k1 * R2 + n2];
+    if constexpr (S > 0) tt.y = -tt.y;
+    if (n2 > 0) v[k1] = c_mul(v[k1], tt);
+  }
+}
+template <int N, int NT, typename C> __device__ __forceinline__ void twiddle4_fill(C* s_tw, const C* __restrict__ tw) {
+  constexpr int R2 = Split4<N>::R2;
+  for (int q = threadIdx.x; q < N; q += NT) s_tw[q] = __ldg(tw + (((q / R2) * (q % R2)) & (N - 1)));
+}
+
 // Split of the fused Toeplitz pass (fft4_toeplitz_kernel): 512 = 32 x 16, so
 // the 16-point pass carries the twiddles and the kernel product (no spills
 // at two CTAs per SM; 16 x 32 spills).
@@ -661,7 +676,8 @@ __global__ void zmask_kernel(const int32_t* __restrict__ tstart, int nt0, int nt
 // they read (row R2 k1 + n2), and the R2-point DFTs of k1 read rows
 // R2 k1 .. R2 k1 + R2 - 1; half-warps cover the 16 columns of one row in every
 // access, so no access has a bank conflict.  W x NL x 8 bytes of shared
-// memory (64 KB at NL = 512).
+// memory (64 KB at NL = 512), and NL twiddles (kept there instead of read from
+// global memory: 512^3 grid, y 159 -> 153 us, z 274 -> 270).
 //
 // MASK = 2 (z lines): bit b of zmask[y * tiles_x + x tile] says whether grid
 // positions z in [8 b, 8 b + 8) of those lines lie in the padded tile of some
@@ -696,6 +712,8 @@ __global__ void __launch_bounds__(16 * W, W == kW4 ? 3 : 1) fft4_lines_staged_ke
                    : "memory");
     }
   }
+  C* s_tw = buf + NL * W;
+  if constexpr (W == kW4) twiddle4_fill<NL, NT>(s_tw, tw);
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   // R1-point DFTs in place: thread (w, n2) owns rows R2 n1 + n2 of column w
@@ -714,7 +732,8 @@ __global__ void __launch_bounds__(16 * W, W == kW4 ? 3 : 1) fft4_lines_staged_ke
         if ((!FWD || n < head || n >= tail0) && (FWD || used(n))) v[n1] = buf[n * W + w];
       }
       dft_reg<S, R1>(v);
-      twiddle4<S, NL, R1>(v, n2, tw);
+      if constexpr (W == kW4) twiddle4_smem<S, R1, R2>(v, n2, s_tw);
+      else twiddle4<S, NL, R1>(v, n2, tw);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) buf[(R2 * k1 + n2) * W + w] = v[k1];
     }
@@ -740,10 +759,19 @@ __global__ void __launch_bounds__(16 * W, W == kW4 ? 3 : 1) fft4_lines_staged_ke
   }
 }
 
+// Whether the x pass stages its lines and twiddles in shared memory: with full
+// CTAs, from 128 points.  A CTA then has all of its lines in flight at once
+// and reads a step's twiddles from consecutive addresses (each lane has another
+// n2: a gather of 15 loads per thread from the table).  512 points, 65,536 lines,
+// forward (134 MB read, 268 written) 117 -> 109 us, inverse 107 -> 102; 64^3 adjoint (128
+// points) 54.4 -> 53.0 us.  Few-line CTAs (small transforms) wait for one load's
+// latency either way and skip the extra pass.
+template <int NX, int W> constexpr bool x4_staged() { return W == kW4 && NX >= 128; }
+
 // x lines of the image rows: forward pad + deconvolution + FFT (FWD), or
 // backward FFT + crop + deconvolution.
 template <int NX, bool FWD, int W = kW4>
-__global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : (FWD ? 3 : 2)) fft4_x_kernel(FftGeom G, Inv3<float> inv,
+__global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : 3) fft4_x_kernel(FftGeom G, Inv3<float> inv,
                                                                   const float2* __restrict__ src,
                                                                   float2* __restrict__ dst,
                                                                   const float2* __restrict__ tw,
@@ -756,24 +784,44 @@ __global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : (FWD ? 3 : 2)) fft4_x_ke
   }
   extern __shared__ __align__(16) unsigned char fft_smem[];
   C* y = reinterpret_cast<C*>(fft_smem);
+  constexpr bool STAGED = x4_staged<NX, W>();
+  C* s_tw = y + W * PW;
   __shared__ float s_row[W];
   __shared__ int64_t s_goff[W];
-  const int64_t rows = int64_t(G.N[1]) * G.N[2];
+  const int64_t rows = int64_t(G.N[1]) * G.N[2];  // (below 2^31: a grid of 2^31 lines does not fit the device)
   const int64_t r0 = int64_t(blockIdx.x) * W;
   const int N0 = G.N[0], h0 = G.N[0] / 2;
+  auto grid_line = [&](unsigned yy, unsigned zz) {  // the line's first element in the grid
+    return int64_t(NX) * (wrap_once(int(yy) - G.N[1] / 2, G.Nt[1]) +
+                          int64_t(G.Nt[1]) * wrap_once(int(zz) - G.zs, G.Nt[2]));
+  };
+  if constexpr (STAGED) {  // position n = R2 n1 + n2 of line w at [w][n2][n1]; all loads before any other work
+    for (int w = threadIdx.x >> 5; w < W && r0 + w < rows; w += NT / 32) {
+      const unsigned r = unsigned(r0 + w);
+      const C* line = FWD ? src + int64_t(N0) * r : src + grid_line(r % unsigned(G.N[1]), r / unsigned(G.N[1]));
+      const int count = FWD ? N0 : NX;
+#pragma unroll 8
+      for (int q = threadIdx.x & 31; q < count; q += 32) {
+        const int n = FWD ? (q >= h0 ? q - h0 : q - h0 + NX) : q;
+        const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(y + w * PW + (n % R2) * PR + n / R2));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(at), "l"(line + q) : "memory");
+      }
+    }
+    twiddle4_fill<NX, NT>(s_tw, tw);
+  }
   if (threadIdx.x < W) {
     const int64_t r = r0 + threadIdx.x;
     float sc = 0.f;
     int64_t goff = 0;
     if (r < rows) {
-      const int yy = int(r % G.N[1]), zz = int(r / G.N[1]);
-      sc = __ldg(inv.d[1] + yy) * __ldg(inv.d[2] + zz * G.zinv);
-      goff = int64_t(NX) * (wrap_once(yy - G.N[1] / 2, G.Nt[1]) +
-                            int64_t(G.Nt[1]) * wrap_once(zz - G.zs, G.Nt[2]));
+      const unsigned yy = unsigned(r) % unsigned(G.N[1]), zz = unsigned(r) / unsigned(G.N[1]);
+      sc = __ldg(inv.d[1] + yy) * __ldg(inv.d[2] + int64_t(zz) * G.zinv);
+      goff = grid_line(yy, zz);
     }
     s_row[threadIdx.x] = sc;
     s_goff[threadIdx.x] = goff;
   }
+  if constexpr (STAGED) asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   constexpr int T1 = W * R2, B1 = (T1 + NT - 1) / NT;
 #pragma unroll
@@ -791,17 +839,18 @@ __global__ void __launch_bounds__(16 * W, W < kW4 ? 1 : (FWD ? 3 : 2)) fft4_x_ke
         if (FWD) {
           const int nx = wrap_once(n + h0, NX);
           if (live && nx < N0) {
-            const C a = src[nx + int64_t(N0) * (r0 + w)];
+            const C a = STAGED ? y[w * PW + n2 * PR + n1] : src[nx + int64_t(N0) * (r0 + w)];
             const float sc = __ldg(inv.d[0] + nx) * s_row[w];
             v[n1].x = a.x * sc;
             v[n1].y = a.y * sc;
           }
         } else if (live) {
-          v[n1] = src[s_goff[w] + n];
+          v[n1] = STAGED ? y[w * PW + n2 * PR + n1] : src[s_goff[w] + n];
         }
       }
       dft_reg<S, R1>(v);
-      twiddle4<S, NX, R1>(v, n2, tw);
+      if constexpr (STAGED) twiddle4_smem<S, R1, R2>(v, n2, s_tw);
+      else twiddle4<S, NX, R1>(v, n2, tw);
 #pragma unroll
       for (int k1 = 0; k1 < R1; ++k1) y[w * PW + n2 * PR + k1] = v[k1];
     }
@@ -992,7 +1041,7 @@ template <typename T, int NX, int W> int x_pass_w(nfft_plan* p, const void* src,
   using C = Cx<T>;
   const unsigned blocks = unsigned((p->N[1] * p->N[2] * p->fft_cols + W - 1) / W);
   if constexpr (sizeof(T) == 4 && NX <= 512 && NFFT_FFT_FOURSTEP) {
-    const size_t smem = size_t(W) * Split4<NX>::R2 * (Split4<NX>::R1 + 1) * sizeof(float2);
+    const size_t smem = (size_t(W) * Split4<NX>::R2 * (Split4<NX>::R1 + 1) + (x4_staged<NX, W>() ? NX : 0)) * sizeof(float2);
     const float2* tw = static_cast<const float2*>(p->fft_tw[0]);
     auto kern = fwd ? fft4_x_kernel<NX, true, W> : fft4_x_kernel<NX, false, W>;
     if (int rc = set_smem(kern, smem)) return rc;
@@ -1126,7 +1175,7 @@ template <typename T, int NL> int line_pass_t(nfft_plan* p, int axis, bool fwd) 
       return NFFT_OK;
     }
     if (p->fft_staged) {  // tile staged by cp.async, in-place four-step
-      const size_t smem_s = size_t(NL) * kW4 * sizeof(float2);
+      const size_t smem_s = size_t(NL) * (kW4 + 1) * sizeof(float2);  // tile, twiddles
       const unsigned long long* zm = axis == 2 ? zmask_for(p) : nullptr;
       // (the y passes take no mask: the row bitmap costs more than it saves)
       auto ks = zm && axis == 2 ? (fwd ? fft4_lines_staged_kernel<NL, true, 2> : fft4_lines_staged_kernel<NL, false, 2>)
