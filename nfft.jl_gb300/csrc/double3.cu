@@ -10,7 +10,7 @@ template <int L, bool TABLE> int gather_launch(const nfft_plan* p, const double2
                       sizeof(double2) * size_t(pitch) * size_t(p->bs[1] + L - 1) * size_t(p->bs[2] + L - 1);
   if (smem > 227 * 1024) return -1;
   auto kern = gather_double3_kernel<L, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<unsigned(p->n_tasks), kD3GatherThreads, smem, p->stream>>>(make_geom<double>(p), make_nodes<double>(p),
                                                                     p->tasks, g, fhat, pitch);
   NFFT_LAUNCH_CHECK();
@@ -25,7 +25,7 @@ template <int L, bool TABLE> int spread_launch(const nfft_plan* p, const double2
   const int pitch = warp2_pitch(2 * p->m, 8, P0, limit);
   const size_t smem = Spread3D<L>::STAGE + 16 * size_t(pitch) * size_t(rows);
   auto kern = spread_double3_kernel<L, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<unsigned(p->n_tasks), Spread3D<L>::THREADS, smem, p->stream>>>(make_geom<double>(p), make_nodes<double>(p),
                                                                        p->tasks, fhat, g, pitch);
   NFFT_LAUNCH_CHECK();
@@ -61,12 +61,17 @@ int launch_gather_double3(const nfft_plan* p, const void* g, void* fhat) {
 #undef NFFT_D3_ARGS
 }
 
-// Spreading into a zeroed grid (values in the caller's order); -1: m = 4
-// (spread_owned_kernel is as good there), or the tile and its staging do not
-// fit in shared memory.
+// Spreading into a zeroed grid (values in the caller's order); -1: m = 4 and 6
+// (spread_owned_kernel is as good or better there), fewer tasks than fill the
+// GPU (a task's latency counts, and eight warps have less of it), or the tile
+// and its staging do not fit in shared memory.  Adjoint, us here / there, 64^3, 4096
+// tasks: m = 3, 24,576 uniform nodes 297 / 337, 196,608 549 / 624; m = 5 505 / 574,
+// 1291 / 1540; m = 6 906 / 734, 2451 / 2402.  24^3, 150 tasks: m = 3, 3,600 radial
+// nodes 133 / 127, m = 5 234 / 223, uniform 125 / 123.
 int launch_spread_double3(const nfft_plan* p, const void* fhat, void* g) {
 #define NFFT_D3_ARGS (p, static_cast<const double2*>(fhat), static_cast<double*>(g))
 #define NFFT_D3_CASE8(CALL)
+  if (p->n_tasks < 4 * int64_t(p->sms) || p->m == 6) return -1;
   NFFT_D3_DISPATCH(spread_launch);
 #undef NFFT_D3_CASE8
 #undef NFFT_D3_ARGS

@@ -1033,7 +1033,7 @@ template <typename T> Inv3<T> make_inv3(const nfft_plan* p) {
 }
 
 template <typename K> int set_smem(K kern, size_t bytes) {
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  NFFT_CUDA_TRY(allow_smem(kern, bytes));
   return NFFT_OK;
 }
 

@@ -238,7 +238,7 @@ int gather3_launch(nfft_plan* p, const float2* g, float2* fhat) {
   const CUtensorMap* map = p->gather_tma ? tile3_map<BX, BY, BZ, L>(p, const_cast<float2*>(g)) : nullptr;
   CUtensorMap none{};
   auto kern = gather_plane3_kernel<BX, BY, BZ, L, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(GC::SMEM)));
+  NFFT_CUDA_TRY(allow_smem(kern, GC::SMEM));
   kern<<<unsigned(p->n_tasks), kG3Threads, GC::SMEM, p->stream>>>(map ? *map : none, map ? 1 : 0, make_geom<float>(p),
                                                                   make_nodes<float>(p), p->tasks, g, fhat,
                                                                   p->dflag + 1);

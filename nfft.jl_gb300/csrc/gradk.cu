@@ -194,7 +194,7 @@ int grad_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, 
   if constexpr (POLY)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
   auto kern = grad_warp2_kernel<L, T, POLY>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<unsigned(p->n_tasks), 32, smem, p->stream>>>(G, Nd, p->tasks, g, w, dk, pitch, wp);
   NFFT_LAUNCH_CHECK();
   return NFFT_OK;

@@ -382,7 +382,7 @@ int interp_tile3_launch(const nfft_plan* p, const CUtensorMap* map, const Geom<f
   const size_t smem =
       TC::ACC_BYTES + 16 + (p->wtab ? Tile3Gather<true>::STAGE_BYTES : Tile3Gather<false>::STAGE_BYTES);
   auto kern = p->wtab ? interp_tile3_kernel<BX, BY, BZ, true> : interp_tile3_kernel<BX, BY, BZ, false>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     sms = 0;
@@ -445,6 +445,14 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   if (!p->tasks || p->n_tasks == 0) return -1;
   const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
   if (p->M * 256 < p->n_tasks * int64_t(P0) * P1) return -1;
+  // (few nodes: a warp per node spreads them over more SMs, which in FP64 is
+  // what counts: the window values alone are 2 L (L + 1) operations of a unit with
+  // two lanes per SM.  Forward, us tiled / direct, POLYNOMIAL: 3,000 radial nodes, 64 x 56,
+  // m = 5, FP64 145 / 65, FP32 36 / 35; FP64, 16,384 nodes, 64 x 56: m = 3 1.06 times as
+  // fast, m = 5 0.89, m = 8 0.77; 60,000 nodes, 300 x 263 (86 per task): m = 5 266 / 283,
+  // m = 8 1.02; 900 x 788 (11 per task): m = 5 1932 / 1913)
+  if (ncols == 1 && (p->M < 4096 || (sizeof(T) == 8 && (p->M < (L >= 10 ? 49152 : 16384) || p->M < 12 * p->n_tasks))))
+    return -1;
   const int pitch = warp2_plan_pitch<L, T, TABLE>(p);
   const size_t smem = W::GATHER_STAGE + 2 * sizeof(T) * size_t(pitch) * P1;
   if (smem > 227 * 1024) return -1;
@@ -452,7 +460,7 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
   auto kern = gather_warp2_kernel<L, T, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), 32, smem, p->stream>>>(G, Nd, p->tasks, g, fhat, pitch, gcol,
                                                                             fcol, wp);
   NFFT_LAUNCH_CHECK();
@@ -468,9 +476,12 @@ int gather_line_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd,
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
   const size_t smem = 2 * sizeof(T) * size_t(p->bs[0] + L - 1);
-  if (p->tasks && p->n_tasks > 0 && p->M >= 16 * p->n_tasks && smem <= 227 * 1024) {
+  // (and with few tasks per SM the nodes spread better without them: FP64, m = 8,
+  // 20,000 nodes 1.1 times as fast)
+  if (p->tasks && p->n_tasks > 0 && p->M >= 16 * p->n_tasks && p->M >= (sizeof(T) == 8 ? 131072 : 16384) &&
+      smem <= 227 * 1024) {
     auto kern = gather_line_kernel<L, T, TABLE, true>;
-    NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NFFT_CUDA_TRY(allow_smem(kern, smem));
     // phases of the scattered stores: about 32 MB of output each from 64 MB on
     // (2^24 nodes, 134 MB: 478 us in one phase, 291 in four; forward + adjoint
     // 1356 / 1245 / 1233 / 1298 us with 1 / 2 / 4 / 8, 2^23 nodes 639 / 624 / 615 / 649)
@@ -480,8 +491,10 @@ int gather_line_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd,
     kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols), unsigned(phases)), kLineThreads, smem, p->stream>>>(
         G, Nd, p->tasks, g, fhat, gcol, fcol, wp);
   } else {
-    const unsigned blocks = unsigned((p->M + kLineThreads - 1) / kLineThreads);
-    gather_line_kernel<L, T, TABLE, false><<<dim3(blocks, unsigned(ncols)), kLineThreads, 0, p->stream>>>(
+    // (few nodes: one warp per CTA, so that they reach all SMs)
+    const int nt = p->M < int64_t(kLineThreads) * p->sms ? 32 : kLineThreads;
+    const unsigned blocks = unsigned((p->M + nt - 1) / nt);
+    gather_line_kernel<L, T, TABLE, false><<<dim3(blocks, unsigned(ncols)), nt, 0, p->stream>>>(
         G, Nd, nullptr, g, fhat, gcol, fcol, wp);
   }
   NFFT_LAUNCH_CHECK();
@@ -539,7 +552,7 @@ int interp_launch(const nfft_plan* p, const void* g, void* fhat, int ncols, int6
       const size_t smem = sizeof(C) * size_t(p->gather_pitch) * P1 * P2;
       if (smem <= 227 * 1024 && p->n_tasks > 0) {
         auto kern = p->wtab ? interp_tile_kernel<D, L, T, true> : interp_tile_kernel<D, L, T, false>;
-        NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        NFFT_CUDA_TRY(allow_smem(kern, smem));
         kern<<<unsigned(p->n_tasks), kInterpThreads, smem, p->stream>>>(G, Nd, p->tasks, gp, fp, p->gather_pitch);
         NFFT_LAUNCH_CHECK();
         return NFFT_OK;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kLineThreads) gather_line_kernel(Geom<T> G, No
       fhat[nd.w] = s;
     }
   } else {
-    const int64_t i = int64_t(blockIdx.x) * kLineThreads + threadIdx.x;
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= Nd.M) return;
     const int4 nd = __ldg(Nd.node4 + i);
     T w[L];

@@ -48,6 +48,13 @@ void set_error(const char* fmt, ...);
     }                                                                                    \
   } while (0)
 
+// Dynamic shared memory for a kernel, where it needs more than a launch gets
+// unasked (48 KB, less what the kernel has in static arrays).
+template <typename K> inline cudaError_t allow_smem(K kern, size_t bytes) {
+  if (bytes <= 46 * 1024) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+}
+
 // Per-launch geometry shared by the convolution kernels (passed by value).
 template <typename T> struct Geom {
   int D;

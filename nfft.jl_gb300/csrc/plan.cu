@@ -752,20 +752,23 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     // nodes 58 / 63 / 67 / 85, 800,000 nodes 115 / 116 / 121 / 143; 64 slices of
     // 131,072 nodes 1251 / 1191 / 1183 / 1258 (1024).
     // D = 1: 2048, so that tiles of about 1024 nodes are not cut into a task
-    // of 1024 and one of a few (line1.cuh takes a task in equal batches).
+    // of 1024 and one of a few (line1.cuh takes a task in equal batches); 1024 for
+    // fewer nodes, where that would leave SMs without a task.
     // D = 3: as for D = 2, hot tiles of small sets are cut short (radial nodes,
     // whole transform, us with 128 / 256 / 1024: adjoint, m = 5, 64^3, 100,000 nodes
     // 117 / 128 / 255; adjoint, m = 4, 300,000 nodes 143 / 145 / 199; uniform, 34 x 32
     // x 17, 300,000 nodes forward 133 / 117 / 129; FP64 forward 100,000 nodes 471 / 533 /
-    // 841).
-    chunk = D == 1 ? 2048 : 1024;
+    // 841; FP64 adjoint, 56^3, 500,000 uniform nodes, m = 4 1552 with 128, 1500 with 256).
+    // The 256 of few 2-D nodes keeps FP32 sums of a hot tile in one place; FP64 has no
+    // need of it, and its tasks take longer.
+    chunk = D == 1 && M >= (int64_t(1) << 21) ? 2048 : 1024;
     if (D == 3 && !p->prm.compensated && M >= 4096) {
-      if (M < (int64_t(1) << 19)) chunk = M < (int64_t(1) << 17) || p->precision == 64 ? 128 : 256;
+      if (M < (int64_t(1) << 19)) chunk = M < (int64_t(p->precision == 64 ? 3 : 1) << 17) ? 128 : 256;
       else if (M < (int64_t(1) << 20)) chunk = 512;
     }
     if (D == 2 && !p->prm.compensated) {
       const int64_t work = M * p->task_columns;
-      chunk = work < 4096 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
+      chunk = work < 4096 && p->precision == 32 ? 256 : work < (int64_t(1) << 19) ? 64 : work < (int64_t(1) << 22) ? 128 : 256;
     }
     if (const char* e = getenv("NFFT_GB300_TASK_CHUNK")) {
       const int c = atoi(e);

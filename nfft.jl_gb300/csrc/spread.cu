@@ -49,7 +49,7 @@ int spread_line_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
   auto kern = spread_line_kernel<L, T, TABLE, KAHAN>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), kLineThreads, smem, p->stream>>>(G, Nd, p->tasks, fhat, g, fcol,
                                                                                       gcol_t, wp);
   NFFT_LAUNCH_CHECK();
@@ -66,7 +66,7 @@ int spread_warp2_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, cons
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
   auto kern = spread_warp2_kernel<L, T, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  NFFT_CUDA_TRY(allow_smem(kern, smem));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), 32, smem, p->stream>>>(G, Nd, p->tasks, fhat, g, pitch, fcol,
                                                                             gcol_t, wp);
   NFFT_LAUNCH_CHECK();
@@ -109,7 +109,7 @@ int tile3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, con
   const int use_tma = map ? 1 : 0;
   CUtensorMap none{};
   auto kern = p->wtab ? spread_tile3_kernel<BX, BY, BZ, true> : spread_tile3_kernel<BX, BY, BZ, false>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TC::SMEM)));
+  NFFT_CUDA_TRY(allow_smem(kern, TC::SMEM));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), TC::THREADS, TC::SMEM, p->stream>>>(
       map ? *map : none, use_tma, G, Nd, p->tasks, fs, gp, ncols > 1 ? fcol : 0, gcol_t);
   NFFT_LAUNCH_CHECK();
@@ -153,8 +153,18 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
     // the CTA) and from 3 nodes per 2 cells of the occupied tiles on: its sort
     // and scan cost the same for few nodes (forward + adjoint, us, against the
     // per-node kernels below: 0.5 nodes per cell 173 / 162, 1.2 nodes 50 / 49, 2
-    // nodes 1233 / 1540 compensated, 30 nodes 180 / 222, 1500 nodes 243 / 448)
-    if (p->bs[0] <= kLineMaxTile && 2 * p->M >= 3 * p->n_tasks * p->bs[0]) {
+    // nodes 1233 / 1540 compensated, 30 nodes 180 / 222, 1500 nodes 243 / 448).
+    // Without compensation the atomics of short windows are cheaper than the sort,
+    // and in FP64 the serial window values and taps of a CTA's nodes cost more
+    // than atomics over all SMs until there are many CTAs.  Adjoint, times as fast as
+    // the per-node kernels: 300,000 nodes on 4,000 points (75 per cell), m = 2, 4, 5, 6, 8: FP32
+    // 0.77 0.90 1.20 1.09 1.14, compensated 1.15 1.19 1.31 1.34 1.47; FP64 1.17 1.24 0.95 0.83
+    // 0.71, compensated 1.05 1.01 0.72 0.72 0.72; 2e6 nodes on 200,000 points: FP32 0.85 0.90
+    // 1.32 1.40 1.16; FP64 0.93 1.02 1.46 1.26 0.94; 20,000 nodes 0.90 - 1.02.
+    const int64_t occupied = std::min(p->n_tasks, p->ntiles_total) * p->bs[0];
+    const bool many = sizeof(T) == 8 && L >= 10 ? p->M >= (int64_t(1) << 20) : p->M >= 65536;
+    const bool atomics = !p->prm.compensated && (sizeof(T) == 4 ? L <= 8 : L == 4 || L == 16);
+    if (p->bs[0] <= kLineMaxTile && 2 * p->M >= 3 * occupied && many && !atomics) {
       // FP32 TENSOR plans: Horner (2m multiply-adds a value) gives the table's own
       // values for less than reading them; FP64 units are too few for that
       const bool table = p->wtab && !(sizeof(T) == 4 && G.mode == WIN_POLY);
@@ -175,7 +185,7 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
         return NFFT_ERR_UNSUPPORTED;
       }
       auto kern = p->wtab ? spread_line_kahan_kernel<L, T, true> : spread_line_kahan_kernel<L, T, false>;
-      NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      NFFT_CUDA_TRY(allow_smem(kern, smem));
       kern<<<unsigned(p->n_tasks), 32, smem, p->stream>>>(G, Nd, p->tasks, fp, gp);
       NFFT_LAUNCH_CHECK();
       return NFFT_OK;
@@ -186,7 +196,7 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
       return NFFT_ERR_UNSUPPORTED;
     }
     auto kern = p->wtab ? spread_pad1_kernel<L, T, true> : spread_pad1_kernel<L, T, false>;
-    NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NFFT_CUDA_TRY(allow_smem(kern, smem));
     kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), kSpreadThreads, smem, p->stream>>>(G, Nd, p->tasks, fp, gp,
                                                                                           fcol, gcol_t);
   } else {
@@ -196,13 +206,21 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
       set_error("padded spreading tile (%zu bytes) does not fit in shared memory; use a smaller blockSize", smem);
       return NFFT_ERR_UNSUPPORTED;
     }
-    if constexpr (D == 2) {
-      if (!comp)
-        return p->wtab ? spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
-                       : spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
-    }
     auto kern = p->wtab ? spread_owned_kernel<D, L, T, true, true> : spread_owned_kernel<D, L, T, false, true>;
     int threads = OwnedCfg<D, L>::THREADS;
+    if constexpr (D == 2) {
+      // FP64, single plans: two warps per tile from m = 5 on, for few nodes, and for m = 4
+      // where the GPU is full anyway (a task's window values and taps keep one
+      // warp's FP64 operations in a row too long).  Adjoint, us one warp / two warps per task, 60,000 uniform nodes on a
+      // 300 x 263 image: m = 4 275 / 270, m = 5 307 / 297, m = 8 410 / 377; 3,000 radial
+      // nodes, 64 x 56: m = 4 109 / 96, m = 8 232 / 159.
+      const bool two = sizeof(T) == 8 && ncols == 1 && (L >= 10 || p->M < 4096 || (L == 8 && p->M >= 32768));
+      if (!comp && !two)
+        return p->wtab ? spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
+                       : spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+      if constexpr (sizeof(T) == 8)
+        if (!comp) kern = p->wtab ? spread_owned_kernel<D, L, T, true, false> : spread_owned_kernel<D, L, T, false, false>;
+    }
     if constexpr (D == 3) {
       if (!comp) kern = p->wtab ? spread_owned_kernel<D, L, T, true, false> : spread_owned_kernel<D, L, T, false, false>;
       if (!comp && p->spread_layout == 2) {  // 16 warps: slice group x row parity
@@ -223,7 +241,7 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
       const int rc = launch_spread_plane3(p, fhat, g, ncols, fcol, gcol_t);
       if (rc != -1) return rc;
     }
-    NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NFFT_CUDA_TRY(allow_smem(kern, smem));
     C* fs = static_cast<C*>(ncols > 1 ? sorted : p->fsorted);
     int rc = sort_values<T>(p, fp, fs, ncols, fcol);
     if (rc) return rc;

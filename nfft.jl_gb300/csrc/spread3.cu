@@ -20,7 +20,7 @@ int plane3_launch(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, co
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = float(p->coeffs_host[q]);
   auto kern = spread_plane3_kernel<BX, BY, BZ, L, NW, TABLE>;
-  NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(PC::SMEM)));
+  NFFT_CUDA_TRY(allow_smem(kern, PC::SMEM));
   kern<<<dim3(unsigned(p->n_tasks), unsigned(ncols)), PC::THREADS, PC::SMEM, p->stream>>>(
       map ? *map : none, map ? 1 : 0, G, Nd, p->tasks, fhat, gp, ncols > 1 ? fcol : 0, gcol_t, zeros, p->dflag + 1, wp);
   NFFT_LAUNCH_CHECK();
