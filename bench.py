@@ -55,15 +55,15 @@ def config_dict(**kw):
 # launch, tiles 16x8x8): 1.157 GB read + 0.578 GB write.  Not measured in the
 # run itself; the line says so.
 SPREAD_DRAM_BYTES = 1.735e9
-SPREAD_TRAFFIC_SOURCE = ("ncu capture of spread_tile3_rec_kernel on this workload (one launch), "
+SPREAD_TRAFFIC_SOURCE = ("ncu capture of spread_plane3_kernel on this workload (one launch), "
                          "not measured in this run")
 # DRAM bytes (read + write) of one Toeplitz application at 256^3 (the five
 # kernels of the fused path), from an ncu capture of the profiling case:
 # 2.821 GB read + 1.049 GB write.
 TOEPLITZ_DRAM_BYTES = 3.870e9
-SPREAD_LIMITER = ("shared-memory wavefronts: 110 per node (ncu, 128^3 case; 4.6e8 per launch = 1.47 ms at one "
-                  "per clock per SM, ~91% of it reached) -- the read-modify-write of the padded tile in shared "
-                  "memory (16 B per tap; 512 taps per node) bounds the kernel; HBM is not the limiter")
+SPREAD_LIMITER = ("shared-memory wavefronts: 89 per node (ncu; 3.7e8 per launch = 1.18 ms at one "
+                  "per clock per SM, 86% of the pipe's peak reached) -- the read-modify-write of the padded tile in "
+                  "shared memory (16 B per tap; 512 taps per node) bounds the kernel; HBM is not the limiter")
 
 
 def radial_nodes(dtype=np.float32):
@@ -488,7 +488,7 @@ def run_ours(args):
     dom = max(alg, key=lambda s: stages[s])
     t_dom = stages[dom] * 1e-3
     achieved = alg[dom] / t_dom / 1e9
-    kernel_names = {"spread_ms": "spread_tile3_rec_kernel (stage: the kernel alone; its grid was zeroed on a side "
+    kernel_names = {"spread_ms": "spread_plane3_kernel (stage: the kernel alone; its grid was zeroed on a side "
                                  "stream beside the previous gather)",
                     "gather_ms": "interp_tile3_kernel", "deconv_pad_ms": "fft4_x_kernel (forward)",
                     "crop_ms": "fft4_x_kernel (adjoint)"}

@@ -758,7 +758,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     // whole transform, us with 128 / 256 / 1024: adjoint, m = 5, 64^3, 100,000 nodes
     // 117 / 128 / 255; adjoint, m = 4, 300,000 nodes 143 / 145 / 199; uniform, 34 x 32
     // x 17, 300,000 nodes forward 133 / 117 / 129; FP64 forward 100,000 nodes 471 / 533 /
-    // 841; FP64 adjoint, 56^3, 500,000 uniform nodes, m = 4 1552 with 128, 1500 with 256).
+    // 841; FP64 adjoint, 56^3, 500,000 uniform nodes, m = 4 1552 with 128, 1488 with 256).
     // The 256 of few 2-D nodes keeps FP32 sums of a hot tile in one place; FP64 has no
     // need of it, and its tasks take longer.
     chunk = D == 1 && M >= (int64_t(1) << 21) ? 2048 : 1024;
