@@ -443,12 +443,10 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     B->spread_smem = old_smem;
     if (old_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
     B->spread_smem = W::SPREAD_STAGE + tile;
-    NFFT_CUDA_TRY(cudaFuncSetAttribute(batch_spread_warp2_kernel<L, T, TABLE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->spread_smem)));
+    NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
     if (double(B->total[B_NODES]) * 256 >= points) {
       B->gather_smem = W::GATHER_STAGE + tile;
-      NFFT_CUDA_TRY(cudaFuncSetAttribute(batch_gather_warp2_kernel<L, T, TABLE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->gather_smem)));
+      NFFT_CUDA_TRY(allow_smem(batch_gather_warp2_kernel<L, T, TABLE>, B->gather_smem));
     } else {
       int dev = 0, sms = 0;
       cudaGetDevice(&dev);
@@ -465,7 +463,7 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
       for (nfft_plan* p : B->plans) B->spread_smem = std::max(B->spread_smem, owned_smem<D, L, T>(p, false));
       if (B->spread_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
       auto kern = batch_spread_kernel<D, L, T, TABLE>;
-      NFFT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->spread_smem)));
+      NFFT_CUDA_TRY(allow_smem(kern, B->spread_smem));
       int per_sm = 0;
       NFFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, OwnedCfg<D, L>::THREADS,
                                                                   B->spread_smem));

@@ -49,10 +49,18 @@ void set_error(const char* fmt, ...);
   } while (0)
 
 // Dynamic shared memory for a kernel, where it needs more than a launch gets
-// unasked (48 KB, less what the kernel has in static arrays).
+// unasked (48 KB, less what the kernel has in static arrays).  The limit belongs to
+// the function and outlives the launch: it is raised once, to all that an SM
+// has for one CTA, and never lowered, so that neither a plan or batch with
+// smaller tiles nor another thread takes it away from one that launches later.
+constexpr int kSmemMost = 227 * 1024;
 template <typename K> inline cudaError_t allow_smem(K kern, size_t bytes) {
   if (bytes <= 46 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+  cudaFuncAttributes a;
+  if (cudaError_t e = cudaFuncGetAttributes(&a, kern); e != cudaSuccess) return e;
+  if (size_t(a.maxDynamicSharedSizeBytes) >= bytes) return cudaSuccess;
+  const int most = kSmemMost - int(a.sharedSizeBytes);
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes) > most ? int(bytes) : most);
 }
 
 // Per-launch geometry shared by the convolution kernels (passed by value).
