@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
     const int tt = act[q] ? t : GC::TAPS - 1;
     iy[q] = tt / L;
     ix[q] = tt - iy[q] * L;
-    lofs[q] = iy[q] * PITCH + ix[q] + TC::LEAD - o0 - o1 * PITCH - o2 * PLANE;
+    lofs[q] = iy[q] * PITCH + ix[q] + TC::LEAD;
   }
   bool ok = true;
   if (!bulk) asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's part of the tile
@@ -188,7 +188,8 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
       const int s = min(2 * k + half, n - 1);  // (nodes past the end repeat the last one and are dropped)
       const int4 nd = rec[s];
       const float* wn = win + s * GC::WROW;
-      const float2* p = tile + (nd.z * PLANE + nd.y * PITCH + nd.x);
+      // (the tile's origin first: PLANE times a grid index need not fit in 32 bits)
+      const float2* p = tile + ((nd.z - o2) * PLANE + (nd.y - o1) * PITCH + (nd.x - o0));
       float sr[NSTEP], si[NSTEP];
 #pragma unroll
       for (int q = 0; q < NSTEP; ++q) sr[q] = si[q] = 0.f;

@@ -291,8 +291,7 @@ __global__ void __launch_bounds__(kInterpThreads, 4) interp_tile3_kernel(const _
     return;
   }
   int buf = 0;
-  // the lane's tap offset in the tile relative to a node's grid index
-  const int lane_off = ry * PITCH + ix + 1 - o0 - o1 * PITCH - o2 * PLANE;
+  const int lane_off = ry * PITCH + ix + 1;  // the lane's tap in the window
   for (int base = task.y + NK * warp; base < task.z; base += NK * NWARPS) {
     stage(buf == 0 ? NS - 1 : buf - 1, base + (NS - 1) * NK * NWARPS);
     asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");  // this group's slot has landed
@@ -329,7 +328,8 @@ __global__ void __launch_bounds__(kInterpThreads, 4) interp_tile3_kernel(const _
       wz[0] = z0.x, wz[1] = z0.y, wz[2] = z0.z, wz[3] = z0.w;
       wz[4] = z1.x, wz[5] = z1.y, wz[6] = z1.z, wz[7] = z1.w;
       // (a node past the task end reads tap 0 of the tile and is dropped)
-      const float2* bp = tile + (valid ? nd.z * PLANE + nd.y * PITCH + nd.x + lane_off : 0);
+      // (the tile's origin first: PLANE times a grid index need not fit in 32 bits)
+      const float2* bp = tile + (valid ? (nd.z - o2) * PLANE + (nd.y - o1) * PITCH + (nd.x - o0) + lane_off : 0);
       float sr[4], si[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) sr[r] = si[r] = 0.f;
