@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(128, 2) spread_double3_kernel(Geom<double> G, 
       };
       if (L % 4 == 0 || rec.y == KS) run(std::integral_constant<int, STEPS>{});
       else run(std::integral_constant<int, SC::STEPS1 < 1 ? 1 : SC::STEPS1>{});
+      __syncwarp();  // another lane may read these points for the next node
     }
     __syncthreads();
   }

@@ -336,6 +336,7 @@ __device__ __forceinline__ void spread_owned_body(const Geom<T>& G, const Nodes<
             }
           }
         }
+        __syncwarp();  // another lane may read these points for the next node
         so_c = so_n;
         xo_c = xo_n;
 #pragma unroll
@@ -373,6 +374,7 @@ __device__ __forceinline__ void spread_owned_body(const Geom<T>& G, const Nodes<
             acc[off[st]] = a[st];
           }
         }
+        __syncwarp();  // another lane may read these points for the next node
         meta_c = meta_n;
       }
     }

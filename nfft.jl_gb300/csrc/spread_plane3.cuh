@@ -260,6 +260,7 @@ __global__ void __launch_bounds__((Plane3<BX, BY, BZ, L, NW>::THREADS), (Plane3<
               p[NW * k * PLANE + lofs[i]] = a[k][i];
             }
         }
+      __syncwarp();  // another lane may read these points for the next node
     }
     __syncthreads();
   }

@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(256) spread_tile3_kernel(const __grid_constant
       a1.y = fmaf(cz.y, w1, a1.y);
       p[0] = a0;
       p[4 * PITCH] = a1;
+      __syncwarp();  // another lane may read these points for the next node
       mt = mn;
     }
     __syncthreads();

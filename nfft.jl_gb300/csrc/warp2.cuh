@@ -305,6 +305,7 @@ __device__ __forceinline__ void spread_warp2_body(const Geom<T>& G, const Nodes<
           a[q].y = fma(wxc[q], vi[q], a[q].y);
           p[lofs[q]] = a[q];
         }
+      __syncwarp();  // another lane may read these points for the next node
     }
     __syncwarp();
     if constexpr (TABLE) buf ^= 1;
