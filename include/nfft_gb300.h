@@ -180,8 +180,9 @@ int nfft_convolve_transpose(nfft_plan* plan, const void* fhat, int fhat_real, vo
  * w = w ./ t, with s the maximum of the first iteration's g.  weights (length
  * M, real, device) is updated in place; weights_tmp (length M) and workg (size
  * Ntilde, real) receive the last t and g when not NULL.  *non_positive is set to
- * 1 if some t was <= 0 (the reference asserts that none is).  Waits for the
- * result; the plan's grid (tmpVec) is overwritten. */
+ * 1 if some t was <= 0 (the reference asserts that none is): the iterations stop
+ * before that t's division, and weights, weights_tmp and workg hold what they
+ * held there.  Waits for the result; the plan's grid (tmpVec) is overwritten. */
 int nfft_sdc_weights(nfft_plan* plan, int iters, void* weights, void* weights_tmp, void* workg,
                      int32_t* non_positive);
 

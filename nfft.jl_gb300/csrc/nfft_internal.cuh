@@ -155,7 +155,7 @@ struct nfft_plan {
   void* wtab = nullptr;       // M * D * 2m (T), sorted window tensor (not for POLYNOMIAL)
   int32_t* tile_start = nullptr;   // ntiles_total + 1: CSR of nodes per home tile
   void* cbuf = nullptr;       // M complex scratch for real-valued convolve calls (lazy)
-  void* sdc = nullptr;        // scale and status of nfft_sdc_weights (lazy)
+  void* sdc = nullptr;        // scale, status and kept weights of nfft_sdc_weights (lazy)
   void* fsorted = nullptr;    // M complex: fHat in bin-sorted order (spreading input)
   // spreading tasks: (home tile, first node, end node, 0), hot tiles split
   int64_t n_tasks = 0;
