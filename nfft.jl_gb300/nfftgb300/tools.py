@@ -15,6 +15,7 @@ operator A^H A on the 2N grid, and its application to an image.
 from __future__ import annotations
 
 import ctypes
+import operator
 
 import numpy as np
 import torch
@@ -30,6 +31,7 @@ def sdc(p, iters=20, weights=None, weights_tmp=None, workg=None, workf=None, wor
     filled when given."""
     T = p.dtype
     dev = p.device
+    iters = max(0, operator.index(iters))  # (as range(iters): an integer, none if negative)
     if weights is None:
         weights = torch.ones(p.J, dtype=T, device=dev)
     if workf is None:
@@ -45,7 +47,7 @@ def sdc(p, iters=20, weights=None, weights_tmp=None, workg=None, workf=None, wor
             raise P.ArgumentError(f"sdc needs column-major {T} arrays on {dev}")
     bad = ctypes.c_int32(0)
     p._sync_stream()
-    P._check(L.load().nfft_sdc_weights(p._handle, int(iters), P._ptr(weights),
+    P._check(L.load().nfft_sdc_weights(p._handle, iters, P._ptr(weights),
                                        None if weights_tmp is None else P._ptr(weights_tmp),
                                        None if workg is None else P._ptr(workg), ctypes.byref(bad)))
     if bad.value:

@@ -60,3 +60,13 @@ def test_state_where_the_iterations_stop(dtype, value, iters, stop, kw):
     with pytest.raises(ValueError):
         tools.sdc(p, iters=iters, weights=w2)
     assert oracle.rel_l2(w2.cpu().numpy(), w_ref.cpu().numpy()) < tol
+
+
+def test_number_of_iterations_as_in_a_range():
+    k = (np.random.default_rng(2).random((2, 60)) - 0.5).astype(np.float32)
+    p = nf.plan_nfft(k, (16, 16), m=4, sigma=2.0, precompute=nf.TENSOR)
+    none = tools.sdc(p, iters=0)
+    assert oracle.rel_l2(tools.sdc(p, iters=-3).cpu().numpy(), none.cpu().numpy()) < 1e-5
+    assert oracle.rel_l2(tools.sdc(p, iters=np.int64(0)).cpu().numpy(), none.cpu().numpy()) < 1e-5
+    with pytest.raises(TypeError):
+        tools.sdc(p, iters=2.5)
