@@ -43,8 +43,10 @@ struct nfft_batch {
   void* d_items = nullptr;        // BatchItem<T>[n]
   int64_t* d_base = nullptr;      // 5 prefix arrays of n+1: pairs, nodes, tasks, image, grid
   void** d_ptrs = nullptr;        // per call: input/output pointer of each plan
-  int* d_counter = nullptr;       // persistent spreading task counter (D = 3)
+  int* d_counter = nullptr;       // persistent spreading task counter (D = 3, owned)
   int4* d_tasks = nullptr;        // D = 2: every plan's tasks, {tile, first node, end node, plan}
+  int64_t n_tasks = 0;            // ... and how many
+  bool owned = false;             // spreading by spread_owned_body (D = 3; D = 2: two warps per tile)
   size_t gather_smem = 0;         // D = 2: shared memory of the tiled gather (0: the direct gather)
   // pinned ring of per-call pointer tables: a slot is refilled only after the
   // copy that last read it has run (its event), so the copy never stalls the host
@@ -71,7 +73,8 @@ template <typename T> struct BatchItem {
   const int4* tasks;
   const int32_t* tile_start;
   int task_chunk;
-  int pitch;   // D = 2: of the warp2 tiles, else of the spreading tile
+  int pitch;   // of spread_owned_body's tile
+  int pitch2;  // D = 2: of the warp2 tiles
   T* grid;
   typename Cplx<T>::type* fsorted;
   int N[3];
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(32) batch_spread_warp2_kernel(const BatchItem<
   const int4 task = __ldg(tasks + blockIdx.x);
   const BatchItem<T>& it = items[task.w];
   const Geom<T> G = it.G;
-  spread_warp2_body<L, T, TABLE>(G, it.Nd, task, static_cast<const C*>(ptrs[2 * task.w]), it.grid, it.pitch, G.coeffs,
+  spread_warp2_body<L, T, TABLE>(G, it.Nd, task, static_cast<const C*>(ptrs[2 * task.w]), it.grid, it.pitch2, G.coeffs,
                                  smem_raw);
 }
 
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(32) batch_gather_warp2_kernel(const BatchItem<
   const BatchItem<T>& it = items[task.w];
   const Geom<T> G = it.G;
   gather_warp2_body<L, T, TABLE>(G, it.Nd, task, reinterpret_cast<const C*>(it.grid),
-                                 static_cast<C*>(ptrs[2 * task.w + 1]), it.pitch, G.coeffs, smem_raw);
+                                 static_cast<C*>(ptrs[2 * task.w + 1]), it.pitch2, G.coeffs, smem_raw);
 }
 
 int grid_for_items(int64_t work, int per_block) {
@@ -298,7 +301,7 @@ int grid_for_items(int64_t work, int per_block) {
   return int(b < 1 ? 1 : b);
 }
 
-// D = 2: builds d_tasks and sets the task total to its length.
+// D = 2: builds d_tasks.
 template <typename T> int batch_tasks(nfft_batch* B) {
   const int64_t total = B->total[B_TASKS];
   if (total == 0) return NFFT_OK;
@@ -335,7 +338,7 @@ template <typename T> int batch_tasks(nfft_batch* B) {
   batch_tasks_kernel<T><<<grid, 256, 0, B->stream>>>(items, base, B->n, total, most, keep, place, B->d_tasks);
   NFFT_LAUNCH_CHECK();
   NFFT_CUDA_TRY(cudaStreamSynchronize(B->stream));
-  B->total[B_TASKS] = kept;
+  B->n_tasks = kept;
   return NFFT_OK;
 }
 
@@ -386,8 +389,8 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     if (rc) return rc;
     if constexpr (D == 2) {
       if (B->gather_smem > 0) {
-        if (B->total[B_TASKS] == 0) return NFFT_OK;
-        batch_gather_warp2_kernel<L, T, TABLE><<<unsigned(B->total[B_TASKS]), 32, B->gather_smem, B->stream>>>(
+        if (B->n_tasks == 0) return NFFT_OK;
+        batch_gather_warp2_kernel<L, T, TABLE><<<unsigned(B->n_tasks), 32, B->gather_smem, B->stream>>>(
             items, B->d_tasks, B->d_ptrs);
         NFFT_LAUNCH_CHECK();
         return NFFT_OK;
@@ -405,19 +408,22 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
         items, base + B_GRID * (B->n + 1), B->n, B->total[B_GRID]);
     NFFT_LAUNCH_CHECK();
     if constexpr (D == 2) {
-      if (B->total[B_TASKS] > 0) {
-        batch_spread_warp2_kernel<L, T, TABLE><<<unsigned(B->total[B_TASKS]), 32, B->spread_smem, B->stream>>>(
+      if (!B->owned && B->n_tasks > 0) {
+        batch_spread_warp2_kernel<L, T, TABLE><<<unsigned(B->n_tasks), 32, B->spread_smem, B->stream>>>(
             items, B->d_tasks, B->d_ptrs);
         NFFT_LAUNCH_CHECK();
       }
-    } else {
-      batch_sort_values_kernel<T><<<grid_for_items(B->total[B_NODES], 256), 256, 0, B->stream>>>(
-          items, base + B_NODES * (B->n + 1), B->n, B->total[B_NODES], B->d_ptrs);
-      NFFT_LAUNCH_CHECK();
-      NFFT_CUDA_TRY(cudaMemsetAsync(B->d_counter, 0, sizeof(int), B->stream));
-      batch_spread_kernel<D, L, T, TABLE><<<B->spread_ctas, OwnedCfg<D, L>::THREADS, B->spread_smem, B->stream>>>(
-          items, base + B_TASKS * (B->n + 1), B->n, B->total[B_TASKS], B->d_counter);
-      NFFT_LAUNCH_CHECK();
+    }
+    if constexpr (D == 3 || sizeof(T) == 8) {
+      if (B->owned) {
+        batch_sort_values_kernel<T><<<grid_for_items(B->total[B_NODES], 256), 256, 0, B->stream>>>(
+            items, base + B_NODES * (B->n + 1), B->n, B->total[B_NODES], B->d_ptrs);
+        NFFT_LAUNCH_CHECK();
+        NFFT_CUDA_TRY(cudaMemsetAsync(B->d_counter, 0, sizeof(int), B->stream));
+        batch_spread_kernel<D, L, T, TABLE><<<B->spread_ctas, OwnedCfg<D, L>::THREADS, B->spread_smem, B->stream>>>(
+            items, base + B_TASKS * (B->n + 1), B->n, B->total[B_TASKS], B->d_counter);
+        NFFT_LAUNCH_CHECK();
+      }
     }
     int rc = forked_ffts(B, CUFFT_INVERSE);
     if (rc) return rc;
@@ -426,58 +432,54 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     NFFT_LAUNCH_CHECK();
     return NFFT_OK;
   }
-  // D = 2: the tasks in one list, the tile pitches and the shared memory of
-  // the largest tile; the gather goes through tiles when there are enough
-  // nodes per task on the whole (as for one plan, interp.cu)
-  static int setup2(nfft_batch* B) {
-    using W = Warp2<L, T, TABLE>;
-    constexpr size_t E = 2 * sizeof(T);
-    size_t old_smem = 0, tile = 0;
-    double points = 0;
-    for (nfft_plan* p : B->plans) {
-      old_smem = std::max(old_smem, owned_smem<D, L, T>(p, false));
-      const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
-      tile = std::max(tile, E * size_t(warp2_plan_pitch<L, T, TABLE>(p)) * P1);
-      points += double(p->n_tasks) * P0 * P1;
-    }
-    B->spread_smem = old_smem;
-    if (old_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
-    B->spread_smem = W::SPREAD_STAGE + tile;
-    NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
-    if (double(B->total[B_NODES]) * 256 >= points) {
-      B->gather_smem = W::GATHER_STAGE + tile;
-      NFFT_CUDA_TRY(allow_smem(batch_gather_warp2_kernel<L, T, TABLE>, B->gather_smem));
-    } else {
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      const int64_t want = (B->total[B_NODES] + 63) / 64;
-      B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(sms) * 64)));
-    }
-    return batch_tasks<T>(B);
+  // persistent CTAs of batch_spread_kernel with the shared memory of the largest tile
+  static int setup_owned(nfft_batch* B) {
+    auto kern = batch_spread_kernel<D, L, T, TABLE>;
+    NFFT_CUDA_TRY(allow_smem(kern, B->spread_smem));
+    int per_sm = 0;
+    NFFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, OwnedCfg<D, L>::THREADS,
+                                                                B->spread_smem));
+    const int64_t ctas = int64_t(std::max(per_sm, 1)) * B->plans[0]->sms;
+    B->spread_ctas = int(std::max<int64_t>(1, std::min<int64_t>(ctas, B->total[B_TASKS])));
+    return NFFT_OK;
   }
   static int setup(nfft_batch* B) {
+    for (nfft_plan* p : B->plans) B->spread_smem = std::max(B->spread_smem, owned_smem<D, L, T>(p, false));
+    if (B->spread_smem > size_t(kSmemMost)) return NFFT_OK;  // rejected by the caller
+    // direct gather: CTAs of 8 warps, one contiguous node chunk each (8 nodes per warp
+    // and CTA at least), at most 64 CTAs per SM
+    const int64_t want = (B->total[B_NODES] + 63) / 64;
+    B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(B->plans[0]->sms) * 64)));
     if constexpr (D == 2) {
-      return setup2(B);
+      // the tile pitches and the shared memory of the largest tile; the gather goes
+      // through tiles when there are enough nodes per task on the whole (as for one
+      // plan, interp.cu).  FP64 tiles that do not fit with the staging of
+      // warp2.cuh, larger than the owned spreader's, run on the latter.
+      using W = Warp2<L, T, TABLE>;
+      size_t tile = 0;
+      double points = 0;
+      for (nfft_plan* p : B->plans) {
+        const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
+        tile = std::max(tile, 2 * sizeof(T) * size_t(warp2_plan_pitch<L, T, TABLE>(p)) * P1);
+        points += double(p->n_tasks) * P0 * P1;
+      }
+      B->owned = sizeof(T) == 8 && W::SPREAD_STAGE + tile > size_t(kSmemMost);
+      if (!B->owned) {
+        B->spread_smem = W::SPREAD_STAGE + tile;
+        NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
+      }
+      if (double(B->total[B_NODES]) * 256 >= points && W::GATHER_STAGE + tile <= size_t(kSmemMost)) {
+        B->gather_smem = W::GATHER_STAGE + tile;
+        NFFT_CUDA_TRY(allow_smem(batch_gather_warp2_kernel<L, T, TABLE>, B->gather_smem));
+      }
+      if (!B->owned || B->gather_smem > 0)
+        if (int rc = batch_tasks<T>(B)) return rc;
     } else {
-      for (nfft_plan* p : B->plans) B->spread_smem = std::max(B->spread_smem, owned_smem<D, L, T>(p, false));
-      if (B->spread_smem > 227 * 1024) return NFFT_OK;  // rejected by the caller
-      auto kern = batch_spread_kernel<D, L, T, TABLE>;
-      NFFT_CUDA_TRY(allow_smem(kern, B->spread_smem));
-      int per_sm = 0;
-      NFFT_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, OwnedCfg<D, L>::THREADS,
-                                                                  B->spread_smem));
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      int64_t ctas = int64_t(std::max(per_sm, 1)) * sms;
-      B->spread_ctas = int(std::max<int64_t>(1, std::min<int64_t>(ctas, B->total[B_TASKS])));
-      // gather: CTAs of 8 warps, one contiguous node chunk each (8 nodes per warp
-      // and CTA at least), at most 64 CTAs per SM
-      const int64_t want = (B->total[B_NODES] + 63) / 64;
-      B->gather_ctas = int(std::max<int64_t>(1, std::min<int64_t>(want, int64_t(sms) * 64)));
-      return NFFT_OK;
+      B->owned = true;
     }
+    if constexpr (D == 3 || sizeof(T) == 8)
+      if (B->owned) return setup_owned(B);
+    return NFFT_OK;
   }
 };
 
@@ -526,7 +528,8 @@ template <typename T> int fill_items(nfft_batch* B) {
     it.tasks = p->tasks;
     it.tile_start = p->tile_start;
     it.task_chunk = p->task_chunk;
-    it.pitch = p->D == 2 ? batch_pitch2<T>(p, B->table) : p->spread_pitch;
+    it.pitch = p->spread_pitch;
+    it.pitch2 = p->D == 2 ? batch_pitch2<T>(p, B->table) : 0;
     it.grid = static_cast<T*>(p->grid);
     it.fsorted = static_cast<typename Cplx<T>::type*>(p->fsorted);
     const T* inv = static_cast<const T*>(p->inv);

@@ -560,8 +560,8 @@ extern "C" int nfft_dplan_create(nfft_dplan** out, int precision, int D, const i
   q->core->task_columns = q->ncols;
   if (q->tiled) {
     const int64_t per = q->ncols < 65535 ? q->ncols : 65535;
-    // (only the 3-D spreaders read the values in bin order)
-    if ((q->R == 3 && cudaMalloc(&q->sorted, 2 * rs * size_t(M) * size_t(per)) != cudaSuccess) ||
+    if ((spread_cols_sorted(q->core, q->ncols) &&
+         cudaMalloc(&q->sorted, 2 * rs * size_t(M) * size_t(per)) != cudaSuccess) ||
         (q->pre > 1 && cudaMalloc(&q->vals, 2 * rs * size_t(M) * size_t(q->ncols)) != cudaSuccess)) {
       nfft_dplan_destroy(q);
       set_error("cudaMalloc of the column node values failed");

@@ -265,8 +265,10 @@ int launch_interp_cols(const nfft_plan* p, const void* g, void* fhat, int ncols,
 // spread.cu
 int launch_spread(nfft_plan* p, const void* fhat, int fhat_real, void* g, int g_real);
 // ncols columns in one launch: values fhat + c fcol, contiguous grids g + c gcol (gcol = |Ntilde|),
-// bin-sorted values in `sorted` (M x ncols complex)
+// bin-sorted values in `sorted` (M x ncols complex; null where spread_cols_sorted is false)
 int launch_spread_cols(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fcol, int64_t gcol, void* sorted);
+// whether spreading ncols columns of the plan may need them
+bool spread_cols_sorted(const nfft_plan* p, int64_t ncols);
 // plan.cu: the grid FFT of a plan (pruned for D >= 2)
 int exec_fft_plan(nfft_plan* p, int dir);
 // fft.cu: fused pruned FFT with the deconvolution

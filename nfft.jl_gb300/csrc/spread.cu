@@ -59,9 +59,8 @@ int spread_line_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const
 template <int L, typename T, bool TABLE>
 int spread_warp2_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* fhat, T* g,
                         int ncols, int64_t fcol, int64_t gcol_t) {
-  using W = Warp2<L, T, TABLE>;
   const int pitch = warp2_plan_pitch<L, T, TABLE>(p);
-  const size_t smem = W::SPREAD_STAGE + 2 * sizeof(T) * size_t(pitch) * size_t(p->bs[1] + L - 1);
+  const size_t smem = warp2_spread_bytes<L, T, TABLE>(p);
   WinPoly<L, T, TABLE> wp{};
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
@@ -71,6 +70,22 @@ int spread_warp2_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, cons
                                                                             gcol_t, wp);
   NFFT_LAUNCH_CHECK();
   return NFFT_OK;
+}
+
+// Whether the uncompensated 2-D spreading of ncols columns runs two warps per
+// tile (spread_owned_kernel, on bin-sorted values) instead of one (warp2.cuh).
+// FP64, tiles that fit in shared memory with the staging of the former but not
+// with that of the latter, which is 2 to 5 KB larger (FP32: smaller).
+// FP64, single plans: from m = 5 on, for few nodes, and for m = 4
+// where the GPU is full anyway (a task's window values and taps keep one
+// warp's FP64 operations in a row too long).  Adjoint, us one warp / two warps per task, 60,000 uniform nodes on a
+// 300 x 263 image: m = 4 275 / 270, m = 5 307 / 297, m = 8 410 / 377; 3,000 radial
+// nodes, 64 x 56: m = 4 109 / 96, m = 8 232 / 159.
+template <int L, typename T> bool spread2_two_warps(const nfft_plan* p, int ncols) {
+  if (sizeof(T) == 4) return false;
+  const bool table = p->prm.precompute != NFFT_PRECOMPUTE_POLYNOMIAL;
+  if ((table ? warp2_spread_bytes<L, T, true>(p) : warp2_spread_bytes<L, T, false>(p)) > size_t(kSmemMost)) return true;
+  return ncols == 1 && (L >= 10 || p->M < 4096 || (L == 8 && p->M >= 32768));
 }
 
 // fHat in bin-sorted order (node4[i].w = input index), for coalesced staging.
@@ -209,12 +224,7 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
     auto kern = p->wtab ? spread_owned_kernel<D, L, T, true, true> : spread_owned_kernel<D, L, T, false, true>;
     int threads = OwnedCfg<D, L>::THREADS;
     if constexpr (D == 2) {
-      // FP64, single plans: two warps per tile from m = 5 on, for few nodes, and for m = 4
-      // where the GPU is full anyway (a task's window values and taps keep one
-      // warp's FP64 operations in a row too long).  Adjoint, us one warp / two warps per task, 60,000 uniform nodes on a
-      // 300 x 263 image: m = 4 275 / 270, m = 5 307 / 297, m = 8 410 / 377; 3,000 radial
-      // nodes, 64 x 56: m = 4 109 / 96, m = 8 232 / 159.
-      const bool two = sizeof(T) == 8 && ncols == 1 && (L >= 10 || p->M < 4096 || (L == 8 && p->M >= 32768));
+      const bool two = spread2_two_warps<L, T>(p, ncols);
       if (!comp && !two)
         return p->wtab ? spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
                        : spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
@@ -305,6 +315,21 @@ const float4* zero_tile_for(nfft_plan* p) {
     }
   }
   return p->spread_zero_copy ? static_cast<const float4*>(p->zero_tile) : nullptr;
+}
+
+bool spread_cols_sorted(const nfft_plan* p, int64_t ncols) {
+  if (p->D != 2) return p->D == 3;
+  if (p->precision == 32) return false;
+  const int n = ncols > 1 ? 2 : 1;
+  switch (p->m) {
+    case 2: return spread2_two_warps<4, double>(p, n);
+    case 3: return spread2_two_warps<6, double>(p, n);
+    case 4: return spread2_two_warps<8, double>(p, n);
+    case 5: return spread2_two_warps<10, double>(p, n);
+    case 6: return spread2_two_warps<12, double>(p, n);
+    case 7: return spread2_two_warps<14, double>(p, n);
+    default: return spread2_two_warps<16, double>(p, n);
+  }
 }
 
 // Row pitch (in accumulator elements) of the padded tile: the smallest pitch

@@ -91,6 +91,12 @@ template <int L, typename T, bool TABLE> int warp2_plan_pitch(const nfft_plan* p
   return warp2_pitch(apart ? 2 : L, apart ? 4 : 128 / int(2 * sizeof(T)), P0, room / (int64_t(2 * sizeof(T)) * P1));
 }
 
+// Shared memory of the spreader for a plan's tiles.
+template <int L, typename T, bool TABLE> size_t warp2_spread_bytes(const nfft_plan* p) {
+  return Warp2<L, T, TABLE>::SPREAD_STAGE +
+         2 * sizeof(T) * size_t(warp2_plan_pitch<L, T, TABLE>(p)) * size_t(p->bs[1] + L - 1);
+}
+
 // The polynomial window's coefficients passed by value (uniform reads hit
 // the constant bank); empty for table windows.
 template <int L, typename T, bool TABLE> struct WinPoly {
