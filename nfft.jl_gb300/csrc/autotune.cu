@@ -5,7 +5,9 @@
 // nodes for each candidate shape, times one gather + one spreading pass with
 // CUDA events on the plan's stream (median of three), keeps the fastest and
 // records it in a small text cache (file named by NFFT_GB300_TUNE_CACHE, if
-// set), keyed by (D, Ntilde, log2 M, m, precision, SM count, mode).
+// set), keyed by (D, Ntilde, log2 M, m, precision, SM count, mode) and a version that
+// changes with the kernels the shapes are timed with: entries of another version
+// are not used.
 #include "nfft_internal.cuh"
 
 #include <algorithm>
@@ -32,7 +34,7 @@ std::string cache_key(const nfft_plan* p) {
   int lm = 0;
   while ((int64_t(1) << (lm + 1)) <= p->M) ++lm;
   char buf[256];
-  snprintf(buf, sizeof(buf), "v2_D%d_N%lldx%lldx%lld_M2^%d_m%d_p%d_sm%d_pre%d_c%d", p->D, (long long)p->Nt[0],
+  snprintf(buf, sizeof(buf), "v3_D%d_N%lldx%lldx%lld_M2^%d_m%d_p%d_sm%d_pre%d_c%d", p->D, (long long)p->Nt[0],
            (long long)p->Nt[1], (long long)p->Nt[2], lm, p->m, p->precision, sms, p->prm.precompute,
            p->prm.compensated);
   return buf;
