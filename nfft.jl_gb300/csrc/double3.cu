@@ -51,9 +51,14 @@ template <int L, bool TABLE> int spread_launch(const nfft_plan* p, const double2
 // memory.  Forward transform, us tiled / direct, m = 5: 4096 tasks, 20,000 nodes
 // 486 / 332, 100,000 797 / 1014, 262,144 1.31 / 1.99 ms in the gather; 225 tasks, 20,000
 // nodes 248 / 225, 100,000 785 / 903.  m = 3: 4096 tasks, 20,000 nodes 278 / 232, 100,000
-// 332 / 468; 225 tasks, 4000 nodes 83 / 82, 100,000 262 / 359).
+// 332 / 468; 225 tasks, 4000 nodes 83 / 82, 100,000 262 / 359).  Compensated plans
+// (tasks_suit): 80,000 radial nodes, 32^3, m = 4 595 / 347, m = 5 1552 / 861, uniform 259 /
+// 327, 469 / 842; 300,000 radial m = 4 1210 / 1008, m = 5 1958 / 2167; 270,000 in 128 tiles
+// m = 4 1150 / 905.
 int launch_gather_double3(const nfft_plan* p, const void* g, void* fhat) {
   if (!p->tasks || p->n_tasks == 0 || p->M < 16 * p->n_tasks || p->M < 65536) return -1;
+  if (!tasks_suit(p, 4)) return -1;
+  if (p->m == 4 && p->prm.compensated && p->longest_task > 512 && p->M < (int64_t(1) << 19)) return -1;
 #define NFFT_D3_ARGS (p, static_cast<const double2*>(g), static_cast<double2*>(fhat))
 #define NFFT_D3_CASE8(CALL) case 4: return p->wtab ? CALL<8, true> NFFT_D3_ARGS : CALL<8, false> NFFT_D3_ARGS;
   NFFT_D3_DISPATCH(gather_launch);

@@ -189,6 +189,7 @@ int grad_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, 
   // (FP64, few nodes: as in the gather.  Training step, 3,000 radial nodes, m = 8: 0.90 times as fast
   // as with a warp per node; 16,384: 1.3 to 1.8 times)
   if (sizeof(T) == 8 && p->M < 4096) return -1;
+  if (!tasks_suit(p, sizeof(T) == 8 && L <= 6 ? 2 : 1)) return -1;
   const int64_t limit = (int64_t(227) * 1024 - int64_t(GradWarp2<L, T>::STAGE)) / (int64_t(2 * sizeof(T)) * P1);
   if (P0 > limit) return -1;
   const int pitch = warp2_pitch(L, 128 / int(2 * sizeof(T)), P0, limit);

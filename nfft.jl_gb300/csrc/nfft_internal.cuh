@@ -162,6 +162,7 @@ struct nfft_plan {
   int4* tasks = nullptr;
   int64_t wrap_nodes = 0;          // 3-D FP32 m = 4: nodes in tiles whose padded box wraps around the (centred) grid
   int task_chunk = 1024;           // most nodes of a task
+  int64_t longest_task = 0;        // nodes of the longest one
   int64_t task_columns = 1;        // columns that every launch over the tasks covers (directional plans)
   int spread_pitch = 0;            // shared-memory row pitch of the padded spreading tile
   int spread_layout = 1;           // D = 3 spreading kernel: 1 = 8 warps owning slices, 2 = 16 warps owning
@@ -200,7 +201,7 @@ struct nfft_plan {
          NB_KEY2, NB_VAL2, NB_TCOUNT, NB_SCR, NB_TCNT, NB_TOFF, NB_COUNT };
   void* nbuf[NB_COUNT] = {};
   size_t nbuf_cap[NB_COUNT] = {};
-  int* dflag = nullptr;            // device words: [0] node check, [1] an async copy wait that timed out, [2] task count, [3] wrap_nodes
+  int* dflag = nullptr;            // device words: [0] node check, [1] an async copy wait that timed out, [2] task count, [3] wrap_nodes, [4] longest_task
   size_t scratch_bytes = 0;
 
   // TimingStats: every forward/adjoint records 4 events into a ring slot; the
@@ -229,6 +230,7 @@ int launch_reduce_nodes(const nfft_plan* p, const void* k, int32_t* ti_u, void* 
 int launch_build_node_tables(const nfft_plan* p, const int32_t* perm, const int32_t* ti_u, const void* te_u);
 int launch_build_weight_table(const nfft_plan* p);
 int launch_deconv_factors(nfft_plan* p);
+// ntasks[0], ntasks[2]: the number of tasks, the nodes of the longest
 int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks);
 int launch_wrap_nodes(const nfft_plan* p, const int32_t* tcount, int* out);
 // autotune.cu
@@ -285,6 +287,21 @@ int launch_grad_nodes(const nfft_plan* p, const void* g, const void* w, void* dk
 // plain.cu (per-node kernels of the plain path, blocking = 0)
 int launch_plain_interp(const nfft_plan* p, const void* g, int g_real, void* fhat, int fhat_real);
 int launch_plain_spread(const nfft_plan* p, const void* fhat, int fhat_real, void* g, int g_real);
+
+// Whether a plan's tasks suit kernels that give each to one warp or CTA for the
+// length of its nodes.  Compensated plans keep tasks of up to 1024 nodes (fewer
+// roundings in the grid's sums), and one such task of a hot tile can outlast all the
+// others: the tasks have to be even and enough to fill the GPU, or so many
+// that the longest is a third of an SM's share (`share` times that for CTAs,
+// whose warps divide a task, and for FP64 kernels that gain more).  Forward transform, us one warp per task / per node,
+// 128^2: 64,000 radial nodes FP32 m = 3 73 / 32, m = 8 88 / 45, FP64 m = 5 731 / 171;
+// 250,000 74 / 56, 94 / 89, 757 / 528; 10^6 84 / 130, 144 / 236, 1479 / 1944; uniform nodes
+// 64,000 14 / 21, 19 / 34, 115 / 143; 250,000 26 / 42, 41 / 75, 337 / 498.
+inline bool tasks_suit(const nfft_plan* p, int share) {
+  if (!p->prm.compensated || p->longest_task <= 64) return true;
+  const bool even = p->n_tasks * p->longest_task <= 2 * p->M && 4 * p->n_tasks >= (p->D == 2 ? 12 : 3) * int64_t(p->sms);
+  return even || 3 * p->longest_task * p->sms <= share * p->M;
+}
 
 template <typename T> Geom<T> make_geom(const nfft_plan* p);
 // plan.cu: allocates p->cbuf

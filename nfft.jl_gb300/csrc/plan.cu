@@ -605,7 +605,7 @@ int nfft_plan_create(nfft_plan** out, int precision, int D, const int64_t* N, in
   const int64_t ninv = p->N[0] + (D > 1 ? p->N[1] : 0) + (D > 2 ? p->N[2] : 0) + 1;
   const int deg = 2 * p->m + 1, L = 2 * p->m;
   if (cudaMalloc(&p->inv, rs * ninv) != cudaSuccess || cudaMalloc(&p->coeffs, rs * deg * L) != cudaSuccess ||
-      cudaMalloc(&p->dflag, 4 * sizeof(int)) != cudaSuccess || cudaMemset(p->dflag, 0, 4 * sizeof(int)) != cudaSuccess) {
+      cudaMalloc(&p->dflag, 5 * sizeof(int)) != cudaSuccess || cudaMemset(p->dflag, 0, 5 * sizeof(int)) != cudaSuccess) {
     set_error("cudaMalloc of plan tables failed");
     return fail(NFFT_ERR_ALLOC);
   }
@@ -737,7 +737,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
   // (the node check runs with the reduction below: its verdict and the task
   // count are read back together, the only wait of this call)
   NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag, 0, sizeof(int), s));
-  NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag + 2, 0, 2 * sizeof(int), s));
+  NFFT_CUDA_TRY(cudaMemsetAsync(p->dflag + 2, 0, 3 * sizeof(int), s));
   int rc = NFFT_OK;
   int chunk = 0;
   if (p->prm.blocking) {
@@ -818,7 +818,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     if (!p->fsorted) return NFFT_ERR_ALLOC;
     p->scratch_bytes += 2 * rs * size_t(M);
   }
-  int words[4] = {0, 0, 0, 0};
+  int words[5] = {0, 0, 0, 0, 0};
   NFFT_CUDA_TRY(cudaMemcpyAsync(words, p->dflag, sizeof(words), cudaMemcpyDeviceToHost, s));
   NFFT_CUDA_TRY(cudaStreamSynchronize(s));
   NFFT_CUDA_TRY(cudaGetLastError());
@@ -829,6 +829,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
   }
   p->n_tasks = words[2];
   p->wrap_nodes = words[3];
+  p->longest_task = words[4];
   p->scratch_bytes += sizeof(int4) * size_t(p->n_tasks);
   p->has_nodes = true;
   p->nodes_version += 1;

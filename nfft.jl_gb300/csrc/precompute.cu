@@ -168,12 +168,17 @@ __global__ void fill_tasks_kernel(const int32_t* __restrict__ tstart, const int3
                                   int64_t ntiles, int chunk, TileOrder order, int4* __restrict__ tasks,
                                   int* __restrict__ ntasks) {
   int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (q >= ntiles) return;
-  if (q == 0) *ntasks = toff[ntiles];
-  const int t = order.tile(q);
-  const int s = tstart[t], e = tstart[t + 1];
-  int pos = toff[q];
-  for (int b = s; b < e; b += chunk) tasks[pos++] = make_int4(t, b, min(e, b + chunk), 0);
+  if (q == 0) ntasks[0] = toff[ntiles];
+  int longest = 0;
+  if (q < ntiles) {
+    const int t = order.tile(q);
+    const int s = tstart[t], e = tstart[t + 1];
+    longest = min(e - s, chunk);
+    int pos = toff[q];
+    for (int b = s; b < e; b += chunk) tasks[pos++] = make_int4(t, b, min(e, b + chunk), 0);
+  }
+  longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(ntasks + 2, longest);
 }
 
 // Small grids: the CSR of the tiles and the task list by one CTA, in place of
@@ -225,13 +230,20 @@ __global__ void __launch_bounds__(kListThreads) tile_lists_kernel(const int32_t*
   if (threadIdx.x == 0) tstart[ntiles] = total;
   if (chunk == 0) return;  // no task list (plain path)
   sum = 0;
-  for (int q = q0; q < q1; ++q) sum += (tcount[order.tile(q)] + chunk - 1) / chunk;
+  int longest = 0;
+  for (int q = q0; q < q1; ++q) {
+    const int c = tcount[order.tile(q)];
+    sum += (c + chunk - 1) / chunk;
+    longest = max(longest, min(c, chunk));
+  }
+  longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(ntasks + 2, longest);
   at = cta_exclusive_scan(sum, s_warp, &total);  // (its barriers also publish tstart to the CTA)
   for (int q = q0; q < q1; ++q) {
     const int t = order.tile(q), b0 = tstart[t], e = b0 + tcount[t];
     for (int b = b0; b < e; b += chunk) tasks[at++] = make_int4(t, b, min(e, b + chunk), 0);
   }
-  if (threadIdx.x == 0) *ntasks = total;
+  if (threadIdx.x == 0) ntasks[0] = total;
 }
 
 // Nodes in tiles whose box padded by `pad` points on each side wraps around the grid.
@@ -356,7 +368,8 @@ int launch_deconv_factors(nfft_plan* p) {
 // The CSR of the nodes per tile from their counts, and (chunk > 0) the
 // spreading tasks of at most `chunk` nodes of the non-empty tiles, in the
 // order above.  Allocates p->tasks for the most tasks these nodes can make;
-// the number made goes to `ntasks` (device): nothing waits for it here.
+// the number made and the nodes of the longest go to ntasks[0] and ntasks[2]
+// (device, zeroed by the caller): nothing waits for them here.
 int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks) {
   const int64_t nt = p->ntiles_total;
   const TileOrder order{int(p->ntiles[0]), int(p->ntiles[1]), int(p->ntiles[2])};
