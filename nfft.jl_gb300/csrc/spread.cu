@@ -40,6 +40,47 @@ __global__ void __launch_bounds__(32) spread_warp2_kernel(Geom<T> G, Nodes<T> Nd
                                  pitch, wp.c, smem_raw);
 }
 
+// 1-D: whether the sorting spreader (line1.cuh) is faster than the kernels of
+// spread_body.cuh, atomics or, compensated, one warp per task.
+//
+// Up to 1024 cells (the counts and their scan outgrow
+// the CTA) and from 3 nodes per 2 cells of the occupied tiles on: its sort
+// and scan cost the same for few nodes (forward + adjoint, us, against the
+// per-node kernels: 0.5 nodes per cell 173 / 162, 1.2 nodes 50 / 49, 2
+// nodes 1233 / 1540 compensated, 30 nodes 180 / 222, 1500 nodes 243 / 448).
+// Without compensation the atomics of short windows are cheaper than the sort,
+// and in FP64 the serial window values and taps of a CTA's nodes cost more
+// than atomics over all SMs until there are many CTAs.  Adjoint, times as fast as
+// the per-node kernels: 300,000 nodes on 4,000 points (75 per cell), m = 2, 4, 5, 6, 8: FP32
+// 0.77 0.90 1.20 1.09 1.14, compensated 1.15 1.19 1.31 1.34 1.47; FP64 1.17 1.24 0.95 0.83
+// 0.71, compensated 1.05 1.01 0.72 0.72 0.72; 2e6 nodes on 200,000 points: FP32 0.85 0.90
+// 1.32 1.40 1.16; FP64 0.93 1.02 1.46 1.26 0.94; 20,000 nodes 0.90 - 1.02.
+//
+// A tile of few cells keeps only as many of its CTA's lanes busy as it has
+// positions, for all of its nodes.  That is made up for while the tasks do not fill
+// the GPU anyway (300,000 nodes, grid of 256 points, 300 tasks: 1.2 to 1.5 times as
+// fast), not by short or many tasks.  Adjoint, times as fast, compensated, tiles of 8 cells,
+// grid of 8,000 points: 66,000 / 300,000 / 2e6 nodes m = 3 0.78 / 0.76 / 0.55, m = 5 0.82 / 0.87 /
+// 0.68; 256 points, 900,000 / 2e6: m = 3 0.68 / 0.56; tiles of 32 cells 66,000 / 130,000 / 300,000:
+// 0.96 / 1.04 / 1.18, FP64 m = 8, 2e6 0.72.  FP32 without compensation, m = 6, tiles of 8 or 32
+// cells, about 1000 tasks, 66,000 to 900,000 nodes 0.81 to 0.89, 2e6 (2000 tasks) 1.14 to
+// 1.23; m = 8 0.93 (64 nodes per task) to 1.2.  FP64, m = 4, tiles of 32 cells, 66,000 /
+// 130,000 / 300,000 / 900,000 0.79 / 0.89 / 0.93 / 1.15, m = 3 0.87 / 0.98 / 1.04 / 1.35; 256 points, 66 to
+// 130 tasks 0.79.
+template <int L, typename T> bool line_sort_pays(const nfft_plan* p) {
+  constexpr bool kDouble = sizeof(T) == 8;
+  const bool comp = p->prm.compensated != 0;
+  const int64_t bs = p->bs[0], M = p->M, tasks = p->n_tasks;
+  if (bs > kLineMaxTile || 2 * M < 3 * std::min(tasks, p->ntiles_total) * bs) return false;
+  if (M < (kDouble && L >= 10 ? int64_t(1) << 20 : 65536)) return false;
+  if (!comp && (kDouble ? L == 4 || L == 16 : L <= 8)) return false;
+  if (bs >= 64) return true;
+  if (tasks <= 4 * int64_t(p->sms)) return comp || !kDouble || 2 * tasks >= 3 * int64_t(p->sms);
+  if (comp) return bs >= 32 && M >= 96 * tasks && !(kDouble && L >= 12);
+  if (!kDouble) return L == 16 ? M >= 128 * tasks : 2 * tasks >= 17 * int64_t(p->sms);
+  return M >= (bs < 16 ? 96 : L == 8 ? 384 : 128) * tasks;
+}
+
 template <int L, typename T, bool TABLE, bool KAHAN>
 int spread_line_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* fhat, T* g,
                        int ncols, int64_t fcol, int64_t gcol_t) {
@@ -164,22 +205,7 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
     return NFFT_ERR_UNSUPPORTED;
   }
   if constexpr (D == 1) {
-    // the sorting spreader, up to 1024 cells (the counts and their scan outgrow
-    // the CTA) and from 3 nodes per 2 cells of the occupied tiles on: its sort
-    // and scan cost the same for few nodes (forward + adjoint, us, against the
-    // per-node kernels below: 0.5 nodes per cell 173 / 162, 1.2 nodes 50 / 49, 2
-    // nodes 1233 / 1540 compensated, 30 nodes 180 / 222, 1500 nodes 243 / 448).
-    // Without compensation the atomics of short windows are cheaper than the sort,
-    // and in FP64 the serial window values and taps of a CTA's nodes cost more
-    // than atomics over all SMs until there are many CTAs.  Adjoint, times as fast as
-    // the per-node kernels: 300,000 nodes on 4,000 points (75 per cell), m = 2, 4, 5, 6, 8: FP32
-    // 0.77 0.90 1.20 1.09 1.14, compensated 1.15 1.19 1.31 1.34 1.47; FP64 1.17 1.24 0.95 0.83
-    // 0.71, compensated 1.05 1.01 0.72 0.72 0.72; 2e6 nodes on 200,000 points: FP32 0.85 0.90
-    // 1.32 1.40 1.16; FP64 0.93 1.02 1.46 1.26 0.94; 20,000 nodes 0.90 - 1.02.
-    const int64_t occupied = std::min(p->n_tasks, p->ntiles_total) * p->bs[0];
-    const bool many = sizeof(T) == 8 && L >= 10 ? p->M >= (int64_t(1) << 20) : p->M >= 65536;
-    const bool atomics = !p->prm.compensated && (sizeof(T) == 4 ? L <= 8 : L == 4 || L == 16);
-    if (p->bs[0] <= kLineMaxTile && 2 * p->M >= 3 * occupied && many && !atomics) {
+    if (line_sort_pays<L, T>(p)) {
       // FP32 TENSOR plans: Horner (2m multiply-adds a value) gives the table's own
       // values for less than reading them; FP64 units are too few for that
       const bool table = p->wtab && !(sizeof(T) == 4 && G.mode == WIN_POLY);

@@ -1,0 +1,62 @@
+"""Which kernel a call takes on both sides of the rules of dispatch, and that its
+values agree with the oracle there: 1e-5 (FP32), 1e-11 (FP64; 1e-10 for polynomial
+windows with m >= 6, the conditioning of two fits of degree 2m).
+
+Each rule lies where the times of both kernels, beside it in the source, cross."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import nfftgb300 as nf  # noqa: E402
+from kernel_route import launched  # noqa: E402
+from oracle import oracle  # noqa: E402
+
+ALL = ("spread_line_kernel", "spread_line_kahan_kernel", "spread_pad1_kernel", "gather_line_kernel", "interp_kernel",
+       "gather_warp2_kernel", "gather_plane3_kernel", "gather_double3_kernel", "interp_tile3_kernel",
+       "spread_warp2_kernel", "spread_owned_kernel", "spread_plane3_kernel", "spread_double3_kernel",
+       "grad_nodes_kernel", "grad_warp2_kernel")
+F32, F64 = np.float32, np.float64
+
+# direction, N, M, m, precision, plan keywords, kernel
+ROWS = [
+    # 1-D spreading: tiles of 8 cells (grids of 512 and 8,000 points), 32 cells, 512 cells
+    ("adjoint", (256,), 70000, 3, F32, {"compensated": True}, "spread_line_kernel"),
+    ("adjoint", (4000,), 70000, 3, F32, {"compensated": True}, "spread_line_kahan_kernel"),
+    ("adjoint", (16384,), 70000, 5, F32, {"compensated": True}, "spread_line_kahan_kernel"),
+    ("adjoint", (16384,), 130000, 5, F32, {"compensated": True}, "spread_line_kernel"),
+    ("adjoint", (40000,), 130000, 5, F32, {"compensated": True, "blockSize": (512,)}, "spread_line_kernel"),
+    ("adjoint", (4000,), 130000, 4, F64, {"compensated": True}, "spread_line_kahan_kernel"),
+    ("adjoint", (256,), 70000, 6, F32, {}, "spread_line_kernel"),
+    ("adjoint", (4000,), 70000, 6, F32, {}, "spread_pad1_kernel"),
+    ("adjoint", (4000,), 140000, 8, F32, {}, "spread_line_kernel"),
+    ("adjoint", (128,), 70000, 3, F64, {}, "spread_pad1_kernel"),
+    ("adjoint", (4000,), 140000, 3, F64, {}, "spread_line_kernel"),
+    ("adjoint", (16384,), 130000, 4, F64, {}, "spread_pad1_kernel"),
+]
+
+
+@pytest.mark.parametrize("row", range(len(ROWS)))
+def test_route_and_values(row):
+    direction, N, M, m, dtype, kw, kernel = ROWS[row]
+    rng = np.random.default_rng(row)
+    k = (rng.random((len(N), M)) - 0.5).astype(dtype)
+    kw = dict(kw)
+    pre = kw.pop("precompute", oracle.TENSOR)
+    f = (rng.standard_normal(N) + 1j * rng.standard_normal(N)).astype(np.complex64)
+    v = (rng.standard_normal(M) + 1j * rng.standard_normal(M)).astype(np.complex64)
+    p = nf.plan_nfft(k, N, m=m, sigma=2.0, precompute=pre, **kw)
+    op = oracle.OraclePlan(k.astype(np.float64), N, m=m, sigma=2.0, precompute=pre)
+    tol = 1e-5 if dtype == F32 else (1e-10 if pre != oracle.FULL and m >= 6 else 1e-11)
+    fd, vd = nf.as_colmajor(f, N, p.cdtype), torch.as_tensor(v).to(device="cuda", dtype=p.cdtype)
+    if direction == "forward":
+        y = torch.empty_like(vd)
+        call, got, ref = (lambda: nf.mul_(y, p, fd)), y, op.forward(f.astype(np.complex128))
+    else:
+        x = nf.empty_image(N, p.cdtype)
+        call, got, ref = (lambda: nf.mul_(x, nf.adjoint(p), vd)), x, op.adjoint(v.astype(np.complex128))
+    call()
+    assert launched(call, *ALL) == {kernel}
+    call()
+    assert oracle.rel_l2(got.cpu().numpy().ravel(order="F"), ref.ravel(order="F")) < tol
