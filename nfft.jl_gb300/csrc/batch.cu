@@ -455,6 +455,13 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
       // through tiles when there are enough nodes per task on the whole (as for one
       // plan, interp.cu).  FP64 tiles that do not fit with the staging of
       // warp2.cuh, larger than the owned spreader's, run on the latter.
+      // FP64 tasks keep one warp long: the owned spreader's two take m = 8, and
+      // POLYNOMIAL windows (evaluated by a node's lane) from m = 5 on unless a batch is
+      // large, and a warp per node gathers few nodes in all, or few per task.  Times
+      // as fast so as through warp2.cuh, forward + adjoint: 3 plans, 8,500 nodes, m = 5 1.13, m = 8
+      // 1.47, TENSOR 1.01, 1.07; 8 plans, 24,000 nodes 1.14, 1.33; 24 plans of 3,700 nodes 1.15,
+      // 1.42; spreading alone, 8 plans, 66,000 nodes 1.02, 1.07, 24 plans, 970,000 nodes m = 5
+      // 1.01, m = 6 0.96, m = 8 1.03, TENSOR 1.04; gathering alone there 0.98 - 1.02, 0.77 - 0.85.
       using W = Warp2<L, T, TABLE>;
       size_t tile = 0;
       double points = 0;
@@ -463,12 +470,17 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
         tile = std::max(tile, 2 * sizeof(T) * size_t(warp2_plan_pitch<L, T, TABLE>(p)) * P1);
         points += double(p->n_tasks) * P0 * P1;
       }
-      B->owned = sizeof(T) == 8 && W::SPREAD_STAGE + tile > size_t(kSmemMost);
+      const int64_t nodes = B->total[B_NODES];
+      const bool long_poly = !TABLE && L >= 10;
+      B->owned = sizeof(T) == 8 &&
+                 (W::SPREAD_STAGE + tile > size_t(kSmemMost) || L == 16 ||
+                  (long_poly && (L == 10 || nodes < (int64_t(1) << 19))));
+      const bool per_node = sizeof(T) == 8 && ((L >= 8 && nodes < 12288) || (long_poly && nodes < 16 * B->total[B_TASKS]));
       if (!B->owned) {
         B->spread_smem = W::SPREAD_STAGE + tile;
         NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
       }
-      if (double(B->total[B_NODES]) * 256 >= points && W::GATHER_STAGE + tile <= size_t(kSmemMost)) {
+      if (double(nodes) * 256 >= points && !per_node && W::GATHER_STAGE + tile <= size_t(kSmemMost)) {
         B->gather_smem = W::GATHER_STAGE + tile;
         NFFT_CUDA_TRY(allow_smem(batch_gather_warp2_kernel<L, T, TABLE>, B->gather_smem));
       }

@@ -122,11 +122,20 @@ int spread_warp2_launch(nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, cons
 // warp's FP64 operations in a row too long).  Adjoint, us one warp / two warps per task, 60,000 uniform nodes on a
 // 300 x 263 image: m = 4 275 / 270, m = 5 307 / 297, m = 8 410 / 377; 3,000 radial
 // nodes, 64 x 56: m = 4 109 / 96, m = 8 232 / 159.
-template <int L, typename T> bool spread2_two_warps(const nfft_plan* p, int ncols) {
+// FP64, several columns: m = 8, and few node values in all, or, m >= 6, few nodes (times
+// as fast with two warps, forward + adjoint of a 40 x 30 / 128 x 118 stack: m = 8, 6,000 nodes,
+// 2 columns 1.16 / 1.12, 8 1.03 / 1.07, 64 1.03 / 1.08; m = 5, 2 columns of 12,000 1.08 /
+// 1.03, of 24,000 1.01, 8 of 3,000 1.04 / 1.03, of 6,000 1.00 / 1.03; m = 7, 64 of 3,000 1.00 / 1.05,
+// of 12,000 0.92 - 1.01; m = 4, 2 of 3,000 1.06).
+template <int L, typename T> bool spread2_two_warps(const nfft_plan* p, int64_t ncols) {
   if (sizeof(T) == 4) return false;
   const bool table = p->prm.precompute != NFFT_PRECOMPUTE_POLYNOMIAL;
   if ((table ? warp2_spread_bytes<L, T, true>(p) : warp2_spread_bytes<L, T, false>(p)) > size_t(kSmemMost)) return true;
-  return ncols == 1 && (L >= 10 || p->M < 4096 || (L == 8 && p->M >= 32768));
+  if (ncols > 1) {
+    const int64_t values = p->M * p->task_columns;
+    return L == 16 || (L >= 10 && values < 32768) || (L >= 12 && p->M < 4096) || (L == 8 && values < 8192);
+  }
+  return L >= 10 || p->M < 4096 || (L == 8 && p->M >= 32768);
 }
 
 // fHat in bin-sorted order (node4[i].w = input index), for coalesced staging.
@@ -346,15 +355,14 @@ const float4* zero_tile_for(nfft_plan* p) {
 bool spread_cols_sorted(const nfft_plan* p, int64_t ncols) {
   if (p->D != 2) return p->D == 3;
   if (p->precision == 32) return false;
-  const int n = ncols > 1 ? 2 : 1;
   switch (p->m) {
-    case 2: return spread2_two_warps<4, double>(p, n);
-    case 3: return spread2_two_warps<6, double>(p, n);
-    case 4: return spread2_two_warps<8, double>(p, n);
-    case 5: return spread2_two_warps<10, double>(p, n);
-    case 6: return spread2_two_warps<12, double>(p, n);
-    case 7: return spread2_two_warps<14, double>(p, n);
-    default: return spread2_two_warps<16, double>(p, n);
+    case 2: return spread2_two_warps<4, double>(p, ncols);
+    case 3: return spread2_two_warps<6, double>(p, ncols);
+    case 4: return spread2_two_warps<8, double>(p, ncols);
+    case 5: return spread2_two_warps<10, double>(p, ncols);
+    case 6: return spread2_two_warps<12, double>(p, ncols);
+    case 7: return spread2_two_warps<14, double>(p, ncols);
+    default: return spread2_two_warps<16, double>(p, ncols);
   }
 }
 

@@ -60,3 +60,43 @@ def test_route_and_values(row):
     assert launched(call, *ALL) == {kernel}
     call()
     assert oracle.rel_l2(got.cpu().numpy().ravel(order="F"), ref.ravel(order="F")) < tol
+
+
+@pytest.mark.parametrize("m,M,C,kernel", [(4, 900, 2, "spread_owned_kernel"), (4, 9000, 3, "spread_warp2_kernel"),
+                                          (5, 6000, 4, "spread_owned_kernel"), (5, 6000, 8, "spread_warp2_kernel"),
+                                          (7, 3000, 20, "spread_owned_kernel"), (7, 6000, 8, "spread_warp2_kernel"),
+                                          (8, 9000, 5, "spread_owned_kernel")])
+def test_fp64_stack(m, M, C, kernel):
+    """FP64 directional plans: one or two warps per tile; each column equals its single 2-D plan."""
+    N = (40, 36)
+    rng = np.random.default_rng(m)
+    k = rng.random((2, M)) - 0.5
+    v = nf.as_colmajor(rng.standard_normal((M, C)) + 1j * rng.standard_normal((M, C)), (M, C), torch.complex128)
+    p = nf.plan_nfft(k, N + (C,), dims=(1, 2), m=m, sigma=2.0)
+    x = nf.empty_image(N + (C,), torch.complex128)
+    nf.mul_(x, nf.adjoint(p), v)
+    assert launched(lambda: nf.mul_(x, nf.adjoint(p), v), *ALL) == {kernel}
+    nf.mul_(x, nf.adjoint(p), v)
+    one = nf.plan_nfft(k, N, m=m, sigma=2.0, precompute=nf.LINEAR)
+    for c in range(C):
+        assert oracle.rel_l2(x[:, :, c].cpu().numpy(), (nf.adjoint(one) * v[:, c].contiguous()).cpu().numpy()) < 1e-11
+
+
+@pytest.mark.parametrize("m", [3, 5, 7, 8])
+@pytest.mark.parametrize("pre", [nf.TENSOR, nf.POLYNOMIAL])
+@pytest.mark.parametrize("Ms", [(2500, 700, 1900), (30000, 9000, 4000, 0), (60000,) * 9])
+def test_fp64_batch(m, pre, Ms):
+    """FP64 batches of few, some and many nodes: every member equals its own transforms (1e-12, as in the batch tests)."""
+    rng = np.random.default_rng(len(Ms) + m)
+    shapes = [((64, 48), (33, 31), (96, 20), (40, 40))[i % 4] for i in range(len(Ms))]
+    plans = [nf.plan_nfft(rng.random((2, M)) - 0.5, N, m=m, sigma=2.0, precompute=pre) for N, M in zip(shapes, Ms)]
+    fs = [nf.as_colmajor(rng.standard_normal(N) + 1j * rng.standard_normal(N), N, torch.complex128) for N in shapes]
+    vs = [torch.as_tensor(rng.standard_normal(M) + 1j * rng.standard_normal(M)).cuda() for M in Ms]
+    y1 = [(p * f).cpu().numpy() for p, f in zip(plans, fs)]
+    x1 = [(nf.adjoint(p) * v).cpu().numpy() for p, v in zip(plans, vs)]
+    batch = nf.NFFTBatch(plans)
+    for _ in range(2):
+        for i, (y, x) in enumerate(zip(batch.forward(fs), batch.adjoint(vs))):
+            if Ms[i]:
+                assert oracle.rel_l2(y.cpu().numpy(), y1[i]) <= 1e-12
+            assert oracle.rel_l2(x.cpu().numpy(), x1[i]) <= 1e-12 if Ms[i] else bool((x == 0).all())
