@@ -186,9 +186,11 @@ int grad_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, 
   if (!p->tasks || p->n_tasks == 0) return -1;
   const int P0 = int(p->bs[0]) + L - 1, P1 = int(p->bs[1]) + L - 1;
   if (p->M * 256 < p->n_tasks * int64_t(P0) * P1) return -1;
-  // (FP64, few nodes: as in the gather.  Training step, 3,000 radial nodes, m = 8: 0.90 times as fast
-  // as with a warp per node; 16,384: 1.3 to 1.8 times)
-  if (sizeof(T) == 8 && p->M < 4096) return -1;
+  // (FP64, few nodes: as in the gather, and more so where a lane evaluates the window function
+  // itself.  Training step, times as fast as with a warp per node, 40^2 and 128^2 radial nodes, 4,200 /
+  // 8,000 / 16,000 / 32,000: polynomial m = 3 0.95 / 0.95 / 1.0 / 1.2, m = 8 0.77 / 0.79 / 0.94 / 1.1;
+  // FULL m = 3 0.86 / 0.9 / 1.1 / 1.4, m = 5 0.70 / 0.72 / 0.95 / 1.2, m = 8 0.55 / 0.6 / 0.8 / 1.0)
+  if (sizeof(T) == 8 && p->M < (G.mode != WIN_EXACT || L <= 6 ? 12288 : L <= 10 ? 16384 : 32768)) return -1;
   if (!tasks_suit(p, sizeof(T) == 8 && L <= 6 ? 2 : 1)) return -1;
   const int64_t limit = (int64_t(227) * 1024 - int64_t(GradWarp2<L, T>::STAGE)) / (int64_t(2 * sizeof(T)) * P1);
   if (P0 > limit) return -1;

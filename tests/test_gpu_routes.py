@@ -100,3 +100,32 @@ def test_fp64_batch(m, pre, Ms):
             if Ms[i]:
                 assert oracle.rel_l2(y.cpu().numpy(), y1[i]) <= 1e-12
             assert oracle.rel_l2(x.cpu().numpy(), x1[i]) <= 1e-12 if Ms[i] else bool((x == 0).all())
+
+
+@pytest.mark.parametrize("m,M,pre,dtype,kernel", [(4, 9000, nf.TENSOR, F64, "grad_nodes_kernel"),
+                                                  (4, 13000, nf.TENSOR, F64, "grad_warp2_kernel"),
+                                                  (8, 13000, nf.LINEAR, F64, "grad_warp2_kernel"),
+                                                  (5, 13000, nf.FULL, F64, "grad_nodes_kernel"),
+                                                  (5, 17000, nf.FULL, F64, "grad_warp2_kernel"),
+                                                  (8, 30000, nf.FULL, F64, "grad_nodes_kernel"),
+                                                  (8, 33000, nf.FULL, F64, "grad_warp2_kernel"),
+                                                  (8, 3000, nf.FULL, F32, "grad_warp2_kernel")])
+def test_node_gradient(m, M, pre, dtype, kernel):
+    """By tiles or a warp per node; against the plain path (5e-5 / 1e-11, as in the node gradient's tests)."""
+    N = (40, 27)
+    rng = np.random.default_rng(m)
+    k = (rng.random((2, M)) - 0.5).astype(dtype)
+    f = rng.standard_normal(N) + 1j * rng.standard_normal(N)
+    w = rng.standard_normal(M) + 1j * rng.standard_normal(M)
+    out = []
+    for kw in ({}, {"blocking": False}):
+        p = nf.plan_nfft(k, N, m=m, sigma=2.0, precompute=pre, **kw)
+        fd, wd = nf.as_colmajor(f, N, p.cdtype), torch.as_tensor(w).to(device="cuda", dtype=p.cdtype)
+        dk = torch.empty((M, 2), dtype=p.dtype, device="cuda")
+        call = lambda: p.grad_nodes_(dk.t(), fd, wd)  # noqa: E731
+        call()
+        if not kw:
+            assert launched(call, *ALL) == {kernel}
+            call()
+        out.append(dk.cpu().numpy())
+    assert oracle.rel_l2(out[0], out[1]) < (5e-5 if dtype == F32 else 1e-11)
