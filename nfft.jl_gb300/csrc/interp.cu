@@ -452,7 +452,7 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   // fast, m = 5 0.89, m = 8 0.77; 60,000 nodes, 300 x 263 (86 per task): m = 5 266 / 283,
   // m = 8 1.02; 900 x 788 (11 per task): m = 5 1932 / 1913)
   // (also with several columns: 8 and 64 of 3,000 nodes; 2 of 6,000 and 4 of 4,200, forward + adjoint 0.93 to 0.96 times as fast)
-  if (sizeof(T) == 8 && (p->M < 4096 || p->M * p->task_columns < 20480)) return -1;
+  if (sizeof(T) == 8 && (p->M < 4096 || (ncols > 1 && p->M * p->task_columns < 20480))) return -1;
   if (!tasks_suit(p, sizeof(T) == 8 && L <= 6 ? 2 : 1)) return -1;
   if (ncols == 1 && (p->M < 4096 || (sizeof(T) == 8 && (p->M < (L >= 10 ? 49152 : 16384) || p->M < 12 * p->n_tasks))))
     return -1;

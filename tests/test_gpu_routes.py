@@ -34,6 +34,11 @@ ROWS = [
     ("adjoint", (128,), 70000, 3, F64, {}, "spread_pad1_kernel"),
     ("adjoint", (4000,), 140000, 3, F64, {}, "spread_line_kernel"),
     ("adjoint", (16384,), 130000, 4, F64, {}, "spread_pad1_kernel"),
+    # 2-D FP64 gather of a single plan
+    ("forward", (128, 128), 16384, 4, F64, {}, "gather_warp2_kernel"),
+    ("forward", (128, 128), 16383, 4, F64, {}, "interp_kernel"),
+    ("forward", (128, 128), 49151, 5, F64, {}, "interp_kernel"),
+    ("forward", (128, 128), 49152, 5, F64, {}, "gather_warp2_kernel"),
 ]
 
 
