@@ -448,13 +448,19 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   // (few nodes: a warp per node spreads them over more SMs, which in FP64 is
   // what counts: the window values alone are 2 L (L + 1) operations of a unit with
   // two lanes per SM.  Forward, us tiled / direct, POLYNOMIAL: 3,000 radial nodes, 64 x 56,
-  // m = 5, FP64 145 / 65, FP32 36 / 35; FP64, 16,384 nodes, 64 x 56: m = 3 1.06 times as
+  // m = 5, FP64 145 / 65; FP64, 16,384 nodes, 64 x 56: m = 3 1.06 times as
   // fast, m = 5 0.89, m = 8 0.77; 60,000 nodes, 300 x 263 (86 per task): m = 5 266 / 283,
   // m = 8 1.02; 900 x 788 (11 per task): m = 5 1932 / 1913)
   // (also with several columns: 8 and 64 of 3,000 nodes; 2 of 6,000 and 4 of 4,200, forward + adjoint 0.93 to 0.96 times as fast)
   if (sizeof(T) == 8 && (p->M < 4096 || (ncols > 1 && p->M * p->task_columns < 20480))) return -1;
   if (!tasks_suit(p, sizeof(T) == 8 && L <= 6 ? 2 : 1)) return -1;
-  if (ncols == 1 && (p->M < 4096 || (sizeof(T) == 8 && (p->M < (L >= 10 ? 49152 : 16384) || p->M < 12 * p->n_tasks))))
+  // FP32, few nodes: a task's first loads (tile, records, window values) take longer than a
+  // warp per node needs for all of them.  Forward, device us tiled / direct: 4,200 nodes, 14^2
+  // m = 5 14.4 / 10.7, 400^2 radial m = 3 24.8 / 21.0; 8,000 nodes 14.5 / 12.0, 25.2 / 22.2; 16,000
+  // 14.8 / 13.7, 25.1 / 23.4, 128^2 uniform m = 5 11.7 / 12.4; m = 8, 44^2, 8,000 16.9 / 14.9, 16,000 16.9 /
+  // 17.9, 20,000 16.9 / 19.4.
+  if (ncols == 1 && (p->M < (sizeof(T) == 8 ? 4096 : L >= 14 ? 10240 : 14336) ||
+                     (sizeof(T) == 8 && (p->M < (L >= 10 ? 49152 : 16384) || p->M < 12 * p->n_tasks))))
     return -1;
   const int pitch = warp2_plan_pitch<L, T, TABLE>(p);
   const size_t smem = W::GATHER_STAGE + 2 * sizeof(T) * size_t(pitch) * P1;

@@ -34,7 +34,12 @@ ROWS = [
     ("adjoint", (128,), 70000, 3, F64, {}, "spread_pad1_kernel"),
     ("adjoint", (4000,), 140000, 3, F64, {}, "spread_line_kernel"),
     ("adjoint", (16384,), 130000, 4, F64, {}, "spread_pad1_kernel"),
-    # 2-D FP64 gather of a single plan
+    # 2-D gathers of a single plan
+    ("forward", (44, 44), 14335, 5, F32, {}, "interp_kernel"),
+    ("forward", (44, 44), 14336, 5, F32, {}, "gather_warp2_kernel"),
+    ("forward", (44, 44), 14337, 3, F32, {"precompute": oracle.POLYNOMIAL}, "gather_warp2_kernel"),
+    ("forward", (44, 44), 10239, 8, F32, {"precompute": oracle.FULL}, "interp_kernel"),
+    ("forward", (44, 44), 10240, 8, F32, {"precompute": oracle.FULL}, "gather_warp2_kernel"),
     ("forward", (128, 128), 16384, 4, F64, {}, "gather_warp2_kernel"),
     ("forward", (128, 128), 16383, 4, F64, {}, "interp_kernel"),
     ("forward", (128, 128), 49151, 5, F64, {}, "interp_kernel"),
