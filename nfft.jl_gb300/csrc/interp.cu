@@ -396,13 +396,17 @@ int interp_tile3_launch(const nfft_plan* p, const CUtensorMap* map, const Geom<f
 // inside the grid only (nodes of wrapping tiles gather from L1, on one CTA per
 // task), so it wants few nodes in wrapping tiles (counted by nodes!), fewer
 // still where gather3.cu has many nodes per task to pay for its own tiles; with
-// under 24 nodes per task the direct gather moves less.  Forward, us, here /
+// under 20 nodes per task, 13 where there are 25 tasks for every SM, the direct
+// gather is faster (forward, device us here / direct, uniform nodes: 64^3, 2048 tasks, 16 /
+// 20 / 23 nodes per task 32.4 / 30.9, 34.9 / 34.6, 37.4 / 37.9; 80^3, 4000 tasks, 12 / 16 / 23 68 /
+// 67, 72 / 73, 80 / 90; 100^3, 8125 tasks, 9 / 12 / 15 / 23 132 / 130, 135 / 143, 140 / 147, 153 /
+// 170; 128^3, 16,384 tasks, 8 / 12 / 16 / 23 162 / 144, 171 / 170, 180 / 192, 202 / 237).  Forward, us, here /
 // gather3.cu / direct: 128^3, 10^6 uniform nodes, 23 % in wrapping tiles 351 / 371 /
 // 477; 64^3, 43 %: 100,000 nodes 64 / 71 / 72, 10^6 351 / 212 / 382; 240 x 216 x 180 grid
 // (not centred), 10^6 radial nodes 495 / 331 / 495; 256^3 grid, 8192 tasks, 100,000
 // nodes 175 / - / 156, 300,000 207 / - / 220.
 bool tile3_pays(const nfft_plan* p) {
-  if (p->M < 24 * p->n_tasks) return false;
+  if (p->M < (p->n_tasks >= 25 * int64_t(p->sms) ? 13 : 20) * p->n_tasks) return false;
   if (p->bs[1] != 8 || p->bs[0] > 16) return true;  // tile shapes that gather3.cu does not have
   const int64_t w = p->wrap_nodes;
   return 4 * w <= p->M || (2 * w <= p->M && p->M < 96 * p->n_tasks);

@@ -34,6 +34,11 @@ ROWS = [
     ("adjoint", (128,), 70000, 3, F64, {}, "spread_pad1_kernel"),
     ("adjoint", (4000,), 140000, 3, F64, {}, "spread_line_kernel"),
     ("adjoint", (16384,), 130000, 4, F64, {}, "spread_pad1_kernel"),
+    # 3-D gather, m = 4: 2048 and 4000 tasks
+    ("forward", (64, 64, 64), 38000, 4, F32, {}, "interp_kernel"),
+    ("forward", (64, 64, 64), 43000, 4, F32, {}, "interp_tile3_kernel"),
+    ("forward", (80, 80, 80), 48000, 4, F32, {}, "interp_kernel"),
+    ("forward", (80, 80, 80), 56000, 4, F32, {}, "interp_tile3_kernel"),
     # 2-D gathers of a single plan
     ("forward", (44, 44), 14335, 5, F32, {}, "interp_kernel"),
     ("forward", (44, 44), 14336, 5, F32, {}, "gather_warp2_kernel"),
