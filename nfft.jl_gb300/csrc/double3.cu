@@ -34,18 +34,6 @@ template <int L, bool TABLE> int spread_launch(const nfft_plan* p, const double2
 
 }  // namespace
 
-#define NFFT_D3_DISPATCH(CALL)                                                  \
-  switch (p->m) {                                                               \
-    case 2: return p->wtab ? CALL<4, true> NFFT_D3_ARGS : CALL<4, false> NFFT_D3_ARGS;    \
-    case 3: return p->wtab ? CALL<6, true> NFFT_D3_ARGS : CALL<6, false> NFFT_D3_ARGS;    \
-    NFFT_D3_CASE8(CALL)                                                         \
-    case 5: return p->wtab ? CALL<10, true> NFFT_D3_ARGS : CALL<10, false> NFFT_D3_ARGS;  \
-    case 6: return p->wtab ? CALL<12, true> NFFT_D3_ARGS : CALL<12, false> NFFT_D3_ARGS;  \
-    case 7: return p->wtab ? CALL<14, true> NFFT_D3_ARGS : CALL<14, false> NFFT_D3_ARGS;  \
-    case 8: return p->wtab ? CALL<16, true> NFFT_D3_ARGS : CALL<16, false> NFFT_D3_ARGS;  \
-  }                                                                             \
-  return -1
-
 // -1: not applicable (no task list, a tile that does not fit, or too few
 // nodes per task, or in all, to pay for bringing their tile into shared
 // memory.  Forward transform, us tiled / direct, m = 5: 4096 tasks, 20,000 nodes
@@ -59,27 +47,43 @@ int launch_gather_double3(const nfft_plan* p, const void* g, void* fhat) {
   if (!p->tasks || p->n_tasks == 0 || p->M < 16 * p->n_tasks || p->M < 65536) return -1;
   if (!tasks_suit(p, 4)) return -1;
   if (p->m == 4 && p->prm.compensated && p->longest_task > 512 && p->M < (int64_t(1) << 19)) return -1;
-#define NFFT_D3_ARGS (p, static_cast<const double2*>(g), static_cast<double2*>(fhat))
-#define NFFT_D3_CASE8(CALL) case 4: return p->wtab ? CALL<8, true> NFFT_D3_ARGS : CALL<8, false> NFFT_D3_ARGS;
-  NFFT_D3_DISPATCH(gather_launch);
-#undef NFFT_D3_CASE8
-#undef NFFT_D3_ARGS
+#define NFFT_D3_GATHER(L)                                                                                \
+  case L / 2:                                                                                            \
+    return p->wtab ? gather_launch<L, true>(p, static_cast<const double2*>(g), static_cast<double2*>(fhat)) \
+                   : gather_launch<L, false>(p, static_cast<const double2*>(g), static_cast<double2*>(fhat))
+  switch (p->m) {
+    NFFT_D3_GATHER(4);
+    NFFT_D3_GATHER(6);
+    NFFT_D3_GATHER(8);
+    NFFT_D3_GATHER(10);
+    NFFT_D3_GATHER(12);
+    NFFT_D3_GATHER(14);
+    NFFT_D3_GATHER(16);
+  }
+#undef NFFT_D3_GATHER
+  return -1;
 }
 
-// Spreading into a zeroed grid (values in the caller's order); -1: m = 4 and 6
+// Spreading into a zeroed grid (values in the caller's order); -1: m = 4 and m >= 6
 // (spread_owned_kernel is as good or better there), fewer tasks than fill the
-// GPU (a task's latency counts, and eight warps have less of it), or the tile
-// and its staging do not fit in shared memory.  Adjoint, us here / there, 64^3, 4096
+// GPU (a task's latency counts, and eight warps have less of it), m = 5 with few nodes in small
+// tiles, or the tile and its staging do not fit in shared memory.  Adjoint, us here / there, 64^3, 4096
 // tasks: m = 3, 24,576 uniform nodes 297 / 337, 196,608 549 / 624; m = 5 505 / 574,
 // 1291 / 1540; m = 6 906 / 734, 2451 / 2402.  24^3, 150 tasks: m = 3, 3,600 radial
-// nodes 133 / 127, m = 5 234 / 223, uniform 125 / 123.
+// nodes 133 / 127, m = 5 234 / 223, uniform 125 / 123.  32^3, tiles of 8 x 8 x 4, times as fast as there:
+// m = 7, 2,000 / 20,000 / 150,000 uniform nodes 0.71 / 0.80 / 0.85; m = 5 0.89 / 1.0 / 1.09, 10,000 0.94.
 int launch_spread_double3(const nfft_plan* p, const void* fhat, void* g) {
-#define NFFT_D3_ARGS (p, static_cast<const double2*>(fhat), static_cast<double*>(g))
-#define NFFT_D3_CASE8(CALL)
-  if (p->n_tasks < 4 * int64_t(p->sms) || p->m == 6) return -1;
-  NFFT_D3_DISPATCH(spread_launch);
-#undef NFFT_D3_CASE8
-#undef NFFT_D3_ARGS
+  if (p->n_tasks < 4 * int64_t(p->sms)) return -1;
+  const auto* f = static_cast<const double2*>(fhat);
+  double* gd = static_cast<double*>(g);
+  switch (p->m) {
+    case 2: return p->wtab ? spread_launch<4, true>(p, f, gd) : spread_launch<4, false>(p, f, gd);
+    case 3: return p->wtab ? spread_launch<6, true>(p, f, gd) : spread_launch<6, false>(p, f, gd);
+    case 5:
+      if (p->bs[0] * p->bs[1] * p->bs[2] < 512 && p->M < 16 * p->n_tasks) return -1;
+      return p->wtab ? spread_launch<10, true>(p, f, gd) : spread_launch<10, false>(p, f, gd);
+  }
+  return -1;
 }
 
 }  // namespace nfft

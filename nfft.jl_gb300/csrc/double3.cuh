@@ -1,4 +1,5 @@
-// 3-D FP64 gather and spreading for any window width L = 2m.
+// 3-D FP64 gather and spreading for any window width L = 2m (the spreader is
+// launched for L = 4, 6, 10, double3.cu).
 //
 // GB300 has two FP64 lanes per SM and clock (a warp instruction occupies them
 // for 16 cycles), so both kernels are bound by the number of FP64 warp

@@ -39,6 +39,12 @@ ROWS = [
     ("forward", (64, 64, 64), 43000, 4, F32, {}, "interp_tile3_kernel"),
     ("forward", (80, 80, 80), 48000, 4, F32, {}, "interp_kernel"),
     ("forward", (80, 80, 80), 56000, 4, F32, {}, "interp_tile3_kernel"),
+    # 3-D FP64 spreading: tiles of 8 x 8 x 4 (1024 tasks) and 5 x 7 x 3
+    ("adjoint", (32, 32, 32), 14000, 5, F64, {}, "spread_owned_kernel"),
+    ("adjoint", (32, 32, 32), 17000, 5, F64, {}, "spread_double3_kernel"),
+    ("adjoint", (32, 32, 32), 14000, 3, F64, {}, "spread_double3_kernel"),
+    ("adjoint", (32, 32, 32), 17000, 7, F64, {}, "spread_owned_kernel"),
+    ("adjoint", (23, 17, 20), 4000, 6, F64, {"blockSize": (5, 7, 3), "precompute": oracle.FULL}, "spread_owned_kernel"),
     # 2-D gathers of a single plan
     ("forward", (44, 44), 14335, 5, F32, {}, "interp_kernel"),
     ("forward", (44, 44), 14336, 5, F32, {}, "gather_warp2_kernel"),

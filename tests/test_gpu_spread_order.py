@@ -28,8 +28,9 @@ CASES = [  # D, N, M, m, FP64, plan keywords, environment, kernel
     (3, (40, 36, 32), 6000, 4, False, {}, {"NFFT_GB300_SPREAD_REC": "0"}, "spread_tile3_kernel"),
     (3, (40, 36, 32), 6000, 5, False, {}, {"NFFT_GB300_SPREAD_REC": "0"}, "spread_owned_kernel"),
     (3, (23, 17, 20), 9000, 3, True, {"blockSize": (5, 7, 3)}, {}, "spread_double3_kernel"),
-    (3, (23, 17, 20), 9000, 5, True, {"blockSize": (5, 7, 3)}, {}, "spread_double3_kernel"),
+    (3, (23, 17, 20), 9000, 5, True, {"blockSize": (5, 7, 3)}, {}, "spread_owned_kernel"),  # few nodes per tile
     (3, (23, 17, 20), 9000, 4, True, {"blockSize": (5, 7, 3)}, {}, "spread_owned_kernel"),
+    (3, (23, 17, 20), 13000, 5, True, {"blockSize": (5, 7, 3)}, {}, "spread_double3_kernel"),
 ]
 KERNELS = ("spread_warp2_kernel", "spread_owned_kernel", "spread_plane3_kernel", "spread_tile3_kernel",
            "spread_double3_kernel")
