@@ -480,7 +480,7 @@ int gather_warp2_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd
   return NFFT_OK;
 }
 
-// D = 1 (line1.cuh).  A tile row of 1024 points is 8 KB: with fewer than 16 nodes per
+// D = 1 (line1.cuh).  A tile row of 1024 points is 8 KB: with fewer than 32 nodes per
 // task the nodes read the grid themselves.
 template <int L, typename T, bool TABLE>
 int gather_line_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd, const typename Cplx<T>::type* g,
@@ -488,11 +488,22 @@ int gather_line_launch(const nfft_plan* p, const Geom<T>& G, const Nodes<T>& Nd,
   LinePoly<L, T, TABLE> wp{};
   if constexpr (!TABLE)
     for (int q = 0; q < L * (L + 1); ++q) wp.c[q] = T(p->coeffs_host[q]);
+  // forward, device us, a thread / a lane per tap: 1,000 nodes, 256 points m = 5 22.8 / 20.6, m = 8 28.8 /
+  // 21.5, 400,000 points 131.9 / 124.6; 4,000 nodes m = 5 23.0 / 22.2, m = 8 28.8 / 23.8; 10,000 no difference
+  if constexpr (sizeof(T) == 8 && !TABLE && L >= 10)
+    if (ncols == 1 && p->M < 6144) {
+      const int64_t per = kLineWarps * Lanes<1, L>::NPW;
+      gather_lanes_kernel<L, T><<<unsigned((p->M + per - 1) / per), kLineThreads, 0, p->stream>>>(G, Nd, g, fhat);
+      NFFT_LAUNCH_CHECK();
+      return NFFT_OK;
+    }
   const size_t smem = 2 * sizeof(T) * size_t(p->bs[0] + L - 1);
   // (and with few tasks per SM the nodes spread better without them: FP64, m = 8,
-  // 20,000 nodes 1.1 times as fast)
-  if (p->tasks && p->n_tasks > 0 && p->M >= 16 * p->n_tasks && p->M >= (sizeof(T) == 8 ? 131072 : 16384) &&
-      smem <= 227 * 1024) {
+  // 20,000 nodes 1.1 times as fast.  Forward, device us with tiles / without, FP32: 32,000 nodes in
+  // about 40 tasks, m = 3 7.1 / 5.9, m = 8 10.3 / 6.3; 64,000 in 64 7.4 / 5.9, 10.4 / 6.7; 1024 tasks of
+  // 31 nodes 12.8 / 12.0, 15.3 / 12.5)
+  if (p->tasks && p->n_tasks > 0 && p->M >= 32 * p->n_tasks && p->M >= (sizeof(T) == 8 ? 131072 : 16384) &&
+      3 * p->n_tasks >= 2 * int64_t(p->sms) && smem <= 227 * 1024) {
     auto kern = gather_line_kernel<L, T, TABLE, true>;
     NFFT_CUDA_TRY(allow_smem(kern, smem));
     // phases of the scattered stores: about 32 MB of output each from 64 MB on

@@ -5,7 +5,7 @@
 // neighbours there (about 2 wavefronts a node with random conflicts) and
 // evaluates or reads its window values itself, so nothing is shuffled or
 // summed across lanes.  Task lists with few nodes per tile read the grid
-// directly.  Node values go back to the caller's order, 8 or 16 bytes at a time:
+// directly, FP64 POLYNOMIAL plans of few nodes with a lane per tap.  Node values go back to the caller's order, 8 or 16 bytes at a time:
 // when they exceed a part of L2, a task's nodes (in input order) are taken in
 // phases, all tasks' first shares first, so that the stores of a phase fall
 // into a window of the output that stays in L2 until its sectors are full.
@@ -25,6 +25,7 @@
 #pragma once
 
 #include "spread_body.cuh"
+#include "warpnode.cuh"
 
 namespace nfft {
 namespace {
@@ -120,6 +121,45 @@ __global__ void __launch_bounds__(kLineThreads) gather_line_kernel(Geom<T> G, No
     }
     fhat[nd.w] = s;
   }
+}
+
+// The same gather with a node's taps on neighbouring lanes (32 / G1 nodes per warp, G1 the
+// power of two >= L), each lane evaluating its own column: FP64 POLYNOMIAL plans of few nodes,
+// where the L (L + 1) operations of a thread's window values in a row are the whole time.
+template <int L, typename T>
+__global__ void __launch_bounds__(kLineThreads) gather_lanes_kernel(Geom<T> G, Nodes<T> Nd,
+                                                                     const typename Cplx<T>::type* __restrict__ g,
+                                                                     typename Cplx<T>::type* __restrict__ fhat) {
+  using C = typename Cplx<T>::type;
+  using LN = Lanes<1, L>;
+  const int lane = threadIdx.x & 31, slot = lane / LN::G1, ix = lane % LN::G1;
+  const bool act = ix < L;
+  T c[L + 1];
+#pragma unroll
+  for (int q = 0; q <= L; ++q) c[q] = act ? __ldg(G.coeffs + ix * (L + 1) + q) : T(0);
+  const int64_t i = (int64_t(blockIdx.x) * kLineWarps + (threadIdx.x >> 5)) * LN::NPW + slot;
+  const bool ok = slot < LN::NPW && i < Nd.M;
+  int4 nd = make_int4(0, 0, 0, 0);
+  C s;
+  s.x = s.y = T(0);
+  if (ok) {
+    nd = __ldg(Nd.node4 + i);
+    if (act) {
+      const T t = __ldg(Nd.frac4 + 4 * i) - T(0.5);
+      T w = c[L];
+#pragma unroll
+      for (int q = L - 1; q >= 0; --q) w = fma(w, t, c[q]);
+      const C v = __ldg(g + wrap_any(nd.x + G.sh[0] - G.m + 1 + ix, G.Nt[0]));
+      s.x = w * v.x;
+      s.y = w * v.y;
+    }
+  }
+#pragma unroll
+  for (int o = LN::G1 / 2; o > 0; o >>= 1) {
+    s.x += __shfl_xor_sync(0xFFFFFFFFu, s.x, o);
+    s.y += __shfl_xor_sync(0xFFFFFFFFu, s.y, o);
+  }
+  if (ok && ix == 0) fhat[nd.w] = s;
 }
 
 // A sorted node: value and tile cell.

@@ -13,7 +13,8 @@ import nfftgb300 as nf  # noqa: E402
 from kernel_route import launched  # noqa: E402
 from oracle import oracle  # noqa: E402
 
-ALL = ("spread_line_kernel", "spread_line_kahan_kernel", "spread_pad1_kernel", "gather_line_kernel", "interp_kernel",
+ALL = ("spread_line_kernel", "spread_line_kahan_kernel", "spread_pad1_kernel", "gather_line_kernel", "gather_lanes_kernel",
+       "interp_kernel",
        "gather_warp2_kernel", "gather_plane3_kernel", "gather_double3_kernel", "interp_tile3_kernel",
        "spread_warp2_kernel", "spread_owned_kernel", "spread_plane3_kernel", "spread_double3_kernel",
        "grad_nodes_kernel", "grad_warp2_kernel")
@@ -39,6 +40,15 @@ ROWS = [
     ("forward", (64, 64, 64), 43000, 4, F32, {}, "interp_tile3_kernel"),
     ("forward", (80, 80, 80), 48000, 4, F32, {}, "interp_kernel"),
     ("forward", (80, 80, 80), 56000, 4, F32, {}, "interp_tile3_kernel"),
+    # 1-D gather
+    ("forward", (128,), 1000, 8, F64, {"precompute": oracle.POLYNOMIAL}, "gather_lanes_kernel"),
+    ("forward", (20000,), 6143, 5, F64, {"precompute": oracle.POLYNOMIAL}, "gather_lanes_kernel"),
+    ("forward", (3,), 33, 7, F64, {"precompute": oracle.POLYNOMIAL}, "gather_lanes_kernel"),
+    ("forward", (500,), 1, 6, F64, {"precompute": oracle.POLYNOMIAL, "compensated": True}, "gather_lanes_kernel"),
+    ("forward", (20000,), 6144, 5, F64, {"precompute": oracle.POLYNOMIAL}, "gather_line_kernel"),
+    ("forward", (128,), 1000, 8, F64, {}, "gather_line_kernel"),
+    ("forward", (128,), 1000, 4, F64, {"precompute": oracle.POLYNOMIAL}, "gather_line_kernel"),
+    ("forward", (128,), 32000, 8, F32, {}, "gather_line_kernel"),
     # 3-D FP64 spreading: tiles of 8 x 8 x 4 (1024 tasks) and 5 x 7 x 3
     ("adjoint", (32, 32, 32), 14000, 5, F64, {}, "spread_owned_kernel"),
     ("adjoint", (32, 32, 32), 17000, 5, F64, {}, "spread_double3_kernel"),
