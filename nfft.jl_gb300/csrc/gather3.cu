@@ -151,9 +151,10 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
   if (!bulk) asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's part of the tile
   __syncthreads();
   if (bulk) ok = mbar_wait_bounded(mbar_s, 0);
-  if (!ok) {
-    asm volatile("cp.async.wait_all;" ::: "memory");  // no copy into shared memory outlives the CTA
+  if (!ok) {  // no copy into shared memory outlives the CTA, as far as another bounded wait can tell
     if (lane == 0) atomicOr(status, 1);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    mbar_wait_bounded(mbar_s, 0);
     return;
   }
   int buf = 0;

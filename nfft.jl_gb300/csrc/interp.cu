@@ -283,11 +283,10 @@ __global__ void __launch_bounds__(kInterpThreads, 4) interp_tile3_kernel(const _
                      : "memory");
     }
   }
-  bool done = false;
-  for (int it = 0; it < (1 << 22) && !done; ++it) done = mbar_try_wait(mbar_s, 0);
-  if (!done) {
-    asm volatile("cp.async.wait_all;" ::: "memory");  // no copy into shared memory outlives the CTA
-    if (threadIdx.x == 0) atomicOr(status, 1);
+  if (!mbar_wait_bounded(mbar_s, 0)) {  // no copy into shared memory outlives the CTA, as far as another bounded wait can tell
+    if (lane == 0) atomicOr(status, 1);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    mbar_wait_bounded(mbar_s, 0);
     return;
   }
   int buf = 0;
