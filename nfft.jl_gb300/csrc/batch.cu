@@ -379,6 +379,8 @@ int forked_ffts(nfft_batch* B, int dir) {
 }
 
 template <int D, int L, typename T, bool TABLE> struct Launch {
+  // D = 2: whether some batch spreads with one warp per task (setup)
+  static constexpr bool kOneWarp = sizeof(T) == 4 || (L < 16 && (TABLE || L != 10));
   static int forward(nfft_batch* B) {
     const auto* items = static_cast<const BatchItem<T>*>(B->d_items);
     const int64_t* base = B->d_base;
@@ -407,7 +409,7 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
     batch_zero_kernel<T><<<grid_for_items(B->total[B_GRID], 256), 256, 0, B->stream>>>(
         items, base + B_GRID * (B->n + 1), B->n, B->total[B_GRID]);
     NFFT_LAUNCH_CHECK();
-    if constexpr (D == 2) {
+    if constexpr (D == 2 && kOneWarp) {
       if (!B->owned && B->n_tasks > 0) {
         batch_spread_warp2_kernel<L, T, TABLE><<<unsigned(B->n_tasks), 32, B->spread_smem, B->stream>>>(
             items, B->d_tasks, B->d_ptrs);
@@ -472,14 +474,14 @@ template <int D, int L, typename T, bool TABLE> struct Launch {
       }
       const int64_t nodes = B->total[B_NODES];
       const bool long_poly = !TABLE && L >= 10;
-      B->owned = sizeof(T) == 8 &&
-                 (W::SPREAD_STAGE + tile > size_t(kSmemMost) || L == 16 ||
-                  (long_poly && (L == 10 || nodes < (int64_t(1) << 19))));
+      B->owned = sizeof(T) == 8 && (!kOneWarp || W::SPREAD_STAGE + tile > size_t(kSmemMost) ||
+                                    (long_poly && nodes < (int64_t(1) << 19)));
       const bool per_node = sizeof(T) == 8 && ((L >= 8 && nodes < 12288) || (long_poly && nodes < 16 * B->total[B_TASKS]));
-      if (!B->owned) {
-        B->spread_smem = W::SPREAD_STAGE + tile;
-        NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
-      }
+      if constexpr (kOneWarp)
+        if (!B->owned) {
+          B->spread_smem = W::SPREAD_STAGE + tile;
+          NFFT_CUDA_TRY(allow_smem(batch_spread_warp2_kernel<L, T, TABLE>, B->spread_smem));
+        }
       if (double(nodes) * 256 >= points && !per_node && W::GATHER_STAGE + tile <= size_t(kSmemMost)) {
         B->gather_smem = W::GATHER_STAGE + tile;
         NFFT_CUDA_TRY(allow_smem(batch_gather_warp2_kernel<L, T, TABLE>, B->gather_smem));

@@ -260,9 +260,14 @@ int spread_launch(nfft_plan* p, const void* fhat, void* g, int ncols, int64_t fc
     int threads = OwnedCfg<D, L>::THREADS;
     if constexpr (D == 2) {
       const bool two = spread2_two_warps<L, T>(p, ncols);
-      if (!comp && !two)
-        return p->wtab ? spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t)
-                       : spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+      // (FP64: m = 8, and from m = 5 on POLYNOMIAL windows, which no stack has, always run two)
+      constexpr bool kTable = sizeof(T) == 4 || L < 16, kPoly = sizeof(T) == 4 || L <= 8;
+      if (!comp && !two) {
+        if constexpr (kTable)
+          if (p->wtab) return spread_warp2_launch<L, T, true>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+        if constexpr (kPoly)
+          if (!p->wtab) return spread_warp2_launch<L, T, false>(p, G, Nd, fp, gp, ncols, fcol, gcol_t);
+      }
       if constexpr (sizeof(T) == 8)
         if (!comp) kern = p->wtab ? spread_owned_kernel<D, L, T, true, false> : spread_owned_kernel<D, L, T, false, false>;
     }
