@@ -2,6 +2,7 @@
 graph's own description is searched for kernel names.  For calls that can be
 captured (no allocation by the library, no wait)."""
 import os
+import re
 import tempfile
 import warnings
 
@@ -9,7 +10,8 @@ import torch
 
 
 def launched(fn, *names):
-    """The subset of `names` (kernel names) among the kernels that fn() launches."""
+    """The subset of `names` among the kernels that fn() launches: kernel names, with the
+    first template arguments in their mangled form (I..) where these matter."""
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     graph.enable_debug_mode()
@@ -20,5 +22,5 @@ def launched(fn, *names):
         path = os.path.join(d, "graph.dot")
         graph.debug_dump(path)
         text = open(path).read()
-    # mangled names: length, then the identifier
-    return {n for n in names if f"{len(n)}{n}" in text}
+    # mangled names: length of the identifier, then the identifier
+    return {n for n in names if f"{len(re.match('[a-z0-9_]+', n)[0])}{n}" in text}
