@@ -274,13 +274,14 @@ template <int L> int gather3_shape(nfft_plan* p, const float2* g, float2* fhat) 
 // Compensated plans (tasks_suit): 65,536 radial nodes, 64^3, m = 3 49 / 42, m = 5 94 / 79;
 // 300,000 86 / 125, 178 / 272; m = 4, any number of them, no slower than before.
 // 27^3, 360 tasks (one or two CTAs per SM): m = 3, 34,560 nodes 46 / 44, m = 5, 17,280
-// 52 / 50, 34,560 60 / 68.  m = 4, 2048 tasks: 100,000 uniform / radial nodes 71, 83 /
-// 72, 300,000 102, 113 / 138.
+// 52 / 50, 34,560 60 / 68.  m = 4, device times as fast as direct, uniform (radial) nodes: 30^3
+// 66,000 0.97 (0.95), 80,000 1.18 (1.11), 150,000 1.25 (1.20), 300,000 1.45 (1.37); 60 x 54 x 45 0.88
+// (0.91), 1.02 (1.03), 1.12 (1.11), 1.32 (1.27).
 int launch_gather_plane3(const nfft_plan* cp, const void* g, void* fhat) {
   nfft_plan* p = const_cast<nfft_plan*>(cp);  // the tensor-map cache only
   if (!p->gather_tma || !p->tasks || p->n_tasks == 0 || p->D != 3 || p->precision != 32 || p->bs[2] != 8) return -1;
   const int per_task = p->m == 2 ? 64 : p->m <= 4 ? 48 : p->m == 5 ? 32 : 24;
-  if (p->M < per_task * p->n_tasks || p->M < (p->m >= 5 ? 32768 : 65536)) return -1;
+  if (p->M < per_task * p->n_tasks || p->M < (p->m >= 5 ? 32768 : p->m == 4 ? 73728 : 65536)) return -1;
   if (p->m != 4 && !tasks_suit(p, 6)) return -1;
   const float2* gp = static_cast<const float2*>(g);
   float2* f = static_cast<float2*>(fhat);
