@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
     ix[q] = tt - iy[q] * L;
     lofs[q] = iy[q] * PITCH + ix[q] + TC::LEAD;
   }
+  const unsigned origin = unsigned(o0) + unsigned(o1) * PITCH + unsigned(o2) * PLANE;
   bool ok = true;
   if (!bulk) asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's part of the tile
   __syncthreads();
@@ -189,8 +190,8 @@ __global__ void __launch_bounds__(kG3Threads, (Gather3<BX, BY, BZ, L, TABLE>::PE
       const int s = min(2 * k + half, n - 1);  // (nodes past the end repeat the last one and are dropped)
       const int4 nd = rec[s];
       const float* wn = win + s * GC::WROW;
-      // (the tile's origin first: PLANE times a grid index need not fit in 32 bits)
-      const float2* p = tile + ((nd.z - o2) * PLANE + (nd.y - o1) * PITCH + (nd.x - o0));
+      // (unsigned: PLANE times a grid index need not fit in 32 bits, its difference to the origin's does)
+      const float2* p = tile + int(unsigned(nd.z) * PLANE + unsigned(nd.y) * PITCH + unsigned(nd.x) - origin);
       float sr[NSTEP], si[NSTEP];
 #pragma unroll
       for (int q = 0; q < NSTEP; ++q) sr[q] = si[q] = 0.f;
