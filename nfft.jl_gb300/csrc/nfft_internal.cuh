@@ -162,7 +162,7 @@ struct nfft_plan {
   int4* tasks = nullptr;
   int64_t wrap_nodes = 0;          // 3-D FP32 m = 4: nodes in tiles whose padded box wraps around the (centred) grid
   int task_chunk = 1024;           // most nodes of a task
-  int64_t longest_task = 0;        // nodes of the longest one
+  int64_t longest_task = 0;        // compensated plans: nodes of the longest one
   int64_t task_columns = 1;        // columns that every launch over the tasks covers (directional plans)
   int spread_pitch = 0;            // shared-memory row pitch of the padded spreading tile
   int spread_layout = 1;           // D = 3 spreading kernel: 1 = 8 warps owning slices, 2 = 16 warps owning
@@ -230,8 +230,8 @@ int launch_reduce_nodes(const nfft_plan* p, const void* k, int32_t* ti_u, void* 
 int launch_build_node_tables(const nfft_plan* p, const int32_t* perm, const int32_t* ti_u, const void* te_u);
 int launch_build_weight_table(const nfft_plan* p);
 int launch_deconv_factors(nfft_plan* p);
-// ntasks[0], ntasks[2]: the number of tasks, the nodes of the longest
-int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks);
+int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks,
+                      int* longest);
 int launch_wrap_nodes(const nfft_plan* p, const int32_t* tcount, int* out);
 // autotune.cu
 int apply_block_size(nfft_plan* p, const int64_t* bs, const void* k, int ny);

@@ -796,7 +796,7 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     NFFT_CUDA_TRY(cudaMemsetAsync(tcount, 0, sizeof(int32_t) * size_t(nt + 1), s));
     rc = launch_reduce_nodes(p, p->k, ti_u, te_u, key, val, tcount, p->dflag);
     if (rc) return rc;
-    rc = launch_tile_lists(p, tcount, chunk, scr, sb, p->dflag + 2);
+    rc = launch_tile_lists(p, tcount, chunk, scr, sb, p->dflag + 2, p->prm.compensated ? p->dflag + 4 : nullptr);
     if (rc) return rc;
     if (D == 3 && p->m == 4 && p->precision == 32 && (rc = launch_wrap_nodes(p, tcount, p->dflag + 3))) return rc;
     uint32_t* ko = nullptr;

@@ -166,9 +166,9 @@ __global__ void task_counts_kernel(const int32_t* __restrict__ tstart, int64_t n
 
 __global__ void fill_tasks_kernel(const int32_t* __restrict__ tstart, const int32_t* __restrict__ toff,
                                   int64_t ntiles, int chunk, TileOrder order, int4* __restrict__ tasks,
-                                  int* __restrict__ ntasks) {
+                                  int* __restrict__ ntasks, int* __restrict__ longest_out) {
   int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (q == 0) ntasks[0] = toff[ntiles];
+  if (q == 0) *ntasks = toff[ntiles];
   int longest = 0;
   if (q < ntiles) {
     const int t = order.tile(q);
@@ -177,8 +177,10 @@ __global__ void fill_tasks_kernel(const int32_t* __restrict__ tstart, const int3
     int pos = toff[q];
     for (int b = s; b < e; b += chunk) tasks[pos++] = make_int4(t, b, min(e, b + chunk), 0);
   }
-  longest = __reduce_max_sync(0xFFFFFFFFu, longest);
-  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(ntasks + 2, longest);
+  if (longest_out) {
+    longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(longest_out, longest);
+  }
 }
 
 // Small grids: the CSR of the tiles and the task list by one CTA, in place of
@@ -215,7 +217,8 @@ __device__ __forceinline__ int cta_exclusive_scan(int v, int* s_warp, int* total
 
 __global__ void __launch_bounds__(kListThreads) tile_lists_kernel(const int32_t* __restrict__ tcount, int ntiles,
                                                                   int chunk, TileOrder order, int32_t* tstart,
-                                                                  int4* __restrict__ tasks, int* __restrict__ ntasks) {
+                                                                  int4* __restrict__ tasks, int* __restrict__ ntasks,
+                                                                  int* __restrict__ longest_out) {
   static_assert(kListThreads == 32 * 32, "one warp sum per lane");
   __shared__ int s_warp[32];
   const int cpt = (ntiles + kListThreads - 1) / kListThreads;
@@ -236,14 +239,16 @@ __global__ void __launch_bounds__(kListThreads) tile_lists_kernel(const int32_t*
     sum += (c + chunk - 1) / chunk;
     longest = max(longest, min(c, chunk));
   }
-  longest = __reduce_max_sync(0xFFFFFFFFu, longest);
-  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(ntasks + 2, longest);
+  if (longest_out) {
+    longest = __reduce_max_sync(0xFFFFFFFFu, longest);
+    if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(longest_out, longest);
+  }
   at = cta_exclusive_scan(sum, s_warp, &total);  // (its barriers also publish tstart to the CTA)
   for (int q = q0; q < q1; ++q) {
     const int t = order.tile(q), b0 = tstart[t], e = b0 + tcount[t];
     for (int b = b0; b < e; b += chunk) tasks[at++] = make_int4(t, b, min(e, b + chunk), 0);
   }
-  if (threadIdx.x == 0) ntasks[0] = total;
+  if (threadIdx.x == 0) *ntasks = total;
 }
 
 // Nodes in tiles whose box padded by `pad` points on each side wraps around the grid.
@@ -368,9 +373,10 @@ int launch_deconv_factors(nfft_plan* p) {
 // The CSR of the nodes per tile from their counts, and (chunk > 0) the
 // spreading tasks of at most `chunk` nodes of the non-empty tiles, in the
 // order above.  Allocates p->tasks for the most tasks these nodes can make;
-// the number made and the nodes of the longest go to ntasks[0] and ntasks[2]
-// (device, zeroed by the caller): nothing waits for them here.
-int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks) {
+// the number made and (longest not null) the nodes of the longest go to `ntasks`
+// and `longest` (device, zeroed by the caller): nothing waits for them here.
+int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr, size_t scr_bytes, int* ntasks,
+                      int* longest) {
   const int64_t nt = p->ntiles_total;
   const TileOrder order{int(p->ntiles[0]), int(p->ntiles[1]), int(p->ntiles[2])};
   if (chunk > 0) {
@@ -380,7 +386,7 @@ int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr,
   }
   if (nt <= kListTiles) {
     tile_lists_kernel<<<1, kListThreads, 0, p->stream>>>(tcount, int(nt), chunk, order, p->tile_start, p->tasks,
-                                                         ntasks);
+                                                         ntasks, longest);
     NFFT_LAUNCH_CHECK();
     return NFFT_OK;
   }
@@ -395,7 +401,7 @@ int launch_tile_lists(nfft_plan* p, const int32_t* tcount, int chunk, void* scr,
   rc = exclusive_scan_i32(tcnt, toff, nt + 1, scr, scr_bytes, p->stream);
   if (rc) return rc;
   fill_tasks_kernel<<<unsigned((nt + 255) / 256), 256, 0, p->stream>>>(p->tile_start, toff, nt, chunk, order,
-                                                                        p->tasks, ntasks);
+                                                                        p->tasks, ntasks, longest);
   NFFT_LAUNCH_CHECK();
   return NFFT_OK;
 }
