@@ -9,7 +9,8 @@
 //             tasks of all plans from one atomic counter), the plans' FFTs,
 //             crop+apodize;
 //   D = 2:    gather and spreading run one warp per task over the plans'
-//             concatenated task lists (warp2.cuh), without the value sort.
+//             concatenated task lists (warp2.cuh), without the value sort; in
+//             FP64 some batches keep the two warps and the gather of above (setup).
 // The plans' FFTs run concurrently on forked streams: the fused pruned FFT
 // (with its own pad / crop, reading the image pointer from the per-call
 // table) for power-of-two grids, cuFFT for the others.

@@ -56,7 +56,7 @@ struct nfft_dplan {
   bool tiled = false;
   bool fused = false;              // the pruned line FFTs instead of pad / crop and cuFFT
   int64_t ncols = 1;               // pre x post
-  void* sorted = nullptr;          // tiled: bin-sorted node values of a launch's columns (M x <= 65535 complex)
+  void* sorted = nullptr;          // tiled, where spread_cols_sorted: bin-sorted node values of a launch's columns (M x <= 65535 complex)
   void* vals = nullptr;            // tiled, pre > 1: node values in column order (M x ncols complex)
 };
 

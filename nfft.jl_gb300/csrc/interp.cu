@@ -2,7 +2,8 @@
 // of prod_d phi_d * g[tap], src/convolution.jl:229-344 (blocked) and :56-99.
 //
 // D = 1: one thread per node (line1.cuh); D = 2: one warp per task from
-// tiles in shared memory (warp2.cuh); D = 3, FP32: tiled (below, gather3.cu).
+// tiles in shared memory (warp2.cuh); D = 3: tiled (below, gather3.cu, double3.cuh); each
+// where its rule finds enough nodes and tasks.
 // Otherwise a warp per node, nodes visited in bin-sorted order; each CTA takes
 // a contiguous chunk of the sorted nodes, so the nodes an SM visits close in time read overlapping grid
 // neighbourhoods through L1, and a warp issues all of a node's grid loads

@@ -19,8 +19,9 @@
 // No atomics, and a fixed order of additions (cell, then input order).
 // 2^24 nodes on 2^23 points, L = 10, compensated: 1019 -> 668 us against one warp
 // per tile whose lanes own the positions mod 32 (10 of 32 lanes on a tap); the
-// instruction issue bounds it (25 warp instructions a node: taps 14, window
-// values 4, sort and scan 5).  Measured slower: batches of 768 nodes with four
+// instruction issue and the sort's latency bound it (31 warp instructions a node, of
+// which the taps are 14; 64 % of the issue slots; 6.1 shared-memory wavefronts a node, a third
+// of them bank conflicts).  Measured slower: batches of 768 nodes with four
 // lanes owning eight positions (748 us).
 #pragma once
 

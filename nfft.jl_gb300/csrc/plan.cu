@@ -759,8 +759,9 @@ int nfft_set_nodes(nfft_plan* p, const void* k, int k_on_device) {
     // 117 / 128 / 255; adjoint, m = 4, 300,000 nodes 143 / 145 / 199; uniform, 34 x 32
     // x 17, 300,000 nodes forward 133 / 117 / 129; FP64 forward 100,000 nodes 471 / 533 /
     // 841; FP64 adjoint, 56^3, 500,000 uniform nodes, m = 4 1552 with 128, 1488 with 256).
-    // The 256 of few 2-D nodes keeps FP32 sums of a hot tile in one place; FP64 has no
-    // need of it, and its tasks take longer.
+    // Fewer than 4096 nodes keep the longer tasks in FP32 (2-D 256, 3-D 1024): with 64 they
+    // would be 2 us faster and a hot tile's plain sums rounded less than the earlier kernels
+    // rounded them, which is what compensated sums are compared with.
     chunk = D == 1 && M >= (int64_t(1) << 21) ? 2048 : 1024;
     if (D == 3 && !p->prm.compensated && M >= 4096) {
       if (M < (int64_t(1) << 19)) chunk = M < (int64_t(p->precision == 64 ? 3 : 1) << 17) ? 128 : 256;

@@ -18,6 +18,9 @@
 //   * D = 1 (spread_pad1_kernel): 32/G nodes per warp, shared-memory atomics;
 //     compensated (spread_line_kahan_kernel): one warp per task, lane l owns
 //     the padded positions x = l mod 32, Kahan read-modify-writes;
+//   * where they are faster (rules below, spread3.cu, double3.cu): D = 1 nodes sorted
+//     by cell (line1.cuh), D = 2 one warp per task (warp2.cuh), D = 3 plane owners
+//     (spread_plane3.cuh, double3.cuh);
 //   * the padded tile is added to the zeroed grid with vector global atomics
 //     (red.global.add.v2), wrapping periodically; all-zero points are skipped.
 // The lock of the reference becomes the L2 atomics of the flush.

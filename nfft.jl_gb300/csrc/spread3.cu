@@ -35,7 +35,7 @@ int plane3_table(nfft_plan* p, const Geom<float>& G, const Nodes<float>& Nd, con
 }
 
 // Two or four warps per tile.  Two read a node's weights half as often, four
-// hide more latency where a tile has few nodes; L = 12's 68 KB tiles leave two CTAs per
+// hide more latency where a tile has few nodes; L = 12's 79 KB tiles leave two CTAs per
 // SM and want four.  Adjoint, us with two / four warps, uniform (radial) nodes:
 //   m = 2: 64^3: 5,000 nodes 45 / 45 (40 / 42), 10^6 133 / 166 (124 / 160)
 //   m = 3: 64^3: 50,000 67 / 63 (57 / 60), 200,000 97 / 102 (90 / 100), 4e6 875 / 1024;

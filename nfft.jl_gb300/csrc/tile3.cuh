@@ -1,6 +1,6 @@
 // Fixed 3-D tile shapes shared by the shape-specialised spreading
 // (spread_tile3.cuh, spread_plane3.cuh) and gather (interp.cu,
-// gather_plane3.cuh) kernels: the tile padded by the window, laid out in
+// gather3.cu) kernels: the tile padded by the window, laid out in
 // shared memory as a TMA box of the grid, and the host side that encodes the
 // grid's tensor map.
 //

@@ -66,7 +66,7 @@ template <int L, typename T, bool TABLE> struct Warp2 {
   static constexpr int NBUF = TABLE ? 2 : 1;
   // L = 8, 16: a lane's taps of two successive steps lie in successive rows, so
   // that their y window values are one 8-byte read.  L = 8 (FP32) then has
-  // rows two apart in one wavefront: pitch = 4 (mod 8) keeps those on
+  // rows two apart in one wavefront: pitch = 2 (mod 4) keeps those on
   // distinct banks.
   static constexpr bool PAIR = L == 8 || L == 16;
   // FP64 spreading: c times the y window values per node (the FP64 units
